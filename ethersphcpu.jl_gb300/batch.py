@@ -67,12 +67,12 @@ def bytes_per(dim: int, thermal: bool, precision: int) -> tuple[int, int, int]:
     """Device bytes per particle, per cell and per wall particle of a batch handle."""
     vec = 16 if dim == 2 else 32
     scal = 7 + (3 if thermal else 0)
-    per_sorted = 2 * vec + 8 * scal + 8
+    per_sorted = 2 * vec + 8 * scal + 8 + 16 + 4 + 8
     if precision == _abi.PRECISION_FP32_COMPENSATED:
-        per_sorted += 3 * 16 + 4 + 4 + 8
+        per_sorted += 2 * 16 + 4
     particle = 2 * per_sorted + 2 * vec + 8 + (8 if thermal else 0) + 12
     cell = 4 * 3 + 1
-    wall = 3 * vec + 3 * 8 + 4 + (48 if precision == _abi.PRECISION_FP32_COMPENSATED else 0)
+    wall = 3 * vec + 3 * 8 + 4 + (48 if precision == _abi.PRECISION_FP32_COMPENSATED else 16)
     return particle, cell, wall
 
 

@@ -182,6 +182,23 @@ bool build_scene(const SphParams& p, SceneDev& S, std::string& err) {
     S.reinit_interval = p.density_reinitialized_interval;
     S.check_interval = p.check_interval;
 
+    S.inv_h = 1.0 / p.h;
+    S.inv_hh = 1.0 / (p.h * p.h);
+    S.kg_h = S.kg_a / p.h;
+    S.nu4 = 4.0 * p.nu_0;
+    double q2 = rc * rc * S.inv_hh;
+    if (p.kernel == SPH_KERNEL_GAUSSIAN) q2 = std::min(q2, 9.0);  // the Gaussian is cut at q = 3
+    auto upper = [](double v) {
+        int64_t bits;
+        std::memcpy(&bits, &v, 8);
+        return (int32_t)(bits >> 32);
+    };
+    S.q2_in_hi = upper(q2 * (1.0 - 1e-6));
+    S.d2_in_hi = upper(rc * rc * (1.0 - 1e-6));
+    S.q2_max = rc * rc * S.inv_hh * (1.0 + 1e-9);
+    for (int a = 0; a < 3; ++a) S.sel_e[a] = (float)(S.cell_d[a] / rc);
+    S.sel_inv_ex = (float)(rc / S.cell_d[0]);
+
     for (int a = 0; a < 3; ++a) S.cell_f[a] = (float)S.cell_d[a];
     S.inv_cell_fx = 1.0f / S.cell_f[0];
     S.h_f = (float)p.h;
@@ -200,6 +217,27 @@ bool build_scene(const SphParams& p, SceneDev& S, std::string& err) {
     S.inv_rho0 = 1.0 / p.rho_0;
     S.inv_rho0_f = (float)(1.0 / p.rho_0);
     return true;
+}
+
+// W(r) (see kernel_w in sph_physics.cuh).
+double host_kernel_w(int kernel, const SceneDev& S, double r) {
+    const double q = r / S.h, t = 2.0 - q;
+    switch (kernel) {
+        case SPH_KERNEL_CUBIC_SPLINE:
+            return q < 1.0 ? S.kw_a * (3.0 * (q * q) * (q - 2.0) + 4.0) : (q < 2.0 ? S.kw_a * (t * t * t) : 0.0);
+        case SPH_KERNEL_GAUSSIAN: return q < 3.0 ? S.kw_a * std::exp(-(q * q)) : 0.0;
+        case SPH_KERNEL_WENDLAND_C2: return q < 2.0 ? S.kw_a * host_powi(t, 4) * (1.0 + 2.0 * q) * 0.0625 : 0.0;
+        default:
+            return q < 2.0 ? S.kw_a * host_powi(t, 6) * (35.0 * (q * q) + 36.0 * q + 12.0) / 768.0 : 0.0;
+    }
+}
+
+// Every particle a fluid one meets has spacing gap0 (or not): the tensile term's W(gap) is
+// then a constant of the scene.
+void set_uniform_gap(int kernel, SceneDev& S, bool uniform, double gap0) {
+    S.wg = uniform ? host_kernel_w(kernel, S, gap0) : 0.0;
+    S.uniform_gap = S.wg > 0.0 ? 1 : 0;
+    S.inv_wg = S.uniform_gap ? 1.0 / S.wg : 0.0;
 }
 
 int32_t host_cell_key(const SceneDev& S, int dim, const double* x) {
@@ -407,13 +445,13 @@ cudaError_t alloc_sorted(SphHandle* h, SortedState& s) {
     }
     if ((e = dalloc(h, &s.id, n)) != cudaSuccess) return e;
     if ((e = dalloc(h, &s.scene, n)) != cudaSuccess) return e;
+    if ((e = dalloc(h, &s.fa, n)) != cudaSuccess) return e;
+    if ((e = dalloc(h, &s.cell, n)) != cudaSuccess) return e;
+    if ((e = dalloc(h, &s.vol, n)) != cudaSuccess) return e;
     if (h->precision == SPH_PRECISION_FP32_COMPENSATED) {  // FP32 shadows of the gathers
-        if ((e = dalloc(h, &s.fa, n)) != cudaSuccess) return e;
         if ((e = dalloc(h, &s.fb, n)) != cudaSuccess) return e;
         if ((e = dalloc(h, &s.fc, n)) != cudaSuccess) return e;
         if ((e = dalloc(h, &s.fd, n)) != cudaSuccess) return e;
-        if ((e = dalloc(h, &s.cell, n)) != cudaSuccess) return e;
-        if ((e = dalloc(h, &s.vol, n)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -696,8 +734,8 @@ int32_t write_scene_walls(SphHandle* h, int s) {
     std::vector<int32_t> bkind(nw);
     std::vector<float4> fa, fb, fc;
     const bool shadow = h->precision == SPH_PRECISION_FP32_COMPENSATED;
+    fa.resize(nw);
     if (shadow) {
-        fa.resize(nw);
         fb.resize(nw);
         fc.resize(nw);
     }
@@ -712,9 +750,16 @@ int32_t write_scene_walls(SphHandle* h, int s) {
         bT[q] = R.wT[w];
         bk[q] = R.wkappa[w];
         bkind[q] = R.wkind[w];
-        if (shadow) {  // position relative to the origin of the wall's cell
-            const int32_t k = key[w] - S.cell_off;
-            const int32_t cc[3] = {k % S.n[0], (k / S.n[0]) % S.n[1], k / (S.n[0] * S.n[1])};
+        const int32_t k = key[w] - S.cell_off;
+        const int32_t cc[3] = {k % S.n[0], (k / S.n[0]) % S.n[1], k / (S.n[0] * S.n[1])};
+        if (!shadow) {  // selection position (select_pos in sph_coop.cuh)
+            float u[3] = {0.f, 0.f, 0.f};
+            for (int a = 0; a < dim; ++a) {
+                const double d = (R.wx[w * dim + a] - S.lo[a]) * S.inv_cell[a] - (double)cc[a];
+                u[a] = (float)std::fmin(std::fmax(d, -1e6), 1e6);
+            }
+            fa[q] = make_float4(u[0], u[1], u[2], (float)cc[0]);
+        } else {  // position relative to the origin of the wall's cell
             float xr[3] = {0.f, 0.f, 0.f}, nr[3] = {0.f, 0.f, 0.f}, vr[3] = {0.f, 0.f, 0.f};
             for (int a = 0; a < dim; ++a) {
                 xr[a] = (float)(R.wx[w * dim + a] - (S.lo[a] + (double)cc[a] * S.cell_d[a]));
@@ -744,8 +789,8 @@ int32_t write_scene_walls(SphHandle* h, int s) {
         SPH_CUDA(h, cudaMemcpyAsync(h->W.T + o, bT.data(), nw * 8, cudaMemcpyHostToDevice, st));
         SPH_CUDA(h, cudaMemcpyAsync(h->W.kappa + o, bk.data(), nw * 8, cudaMemcpyHostToDevice, st));
         SPH_CUDA(h, cudaMemcpyAsync(h->W.kind + o, bkind.data(), nw * 4, cudaMemcpyHostToDevice, st));
+        SPH_CUDA(h, cudaMemcpyAsync(h->W.fa + o, fa.data(), nw * sizeof(float4), cudaMemcpyHostToDevice, st));
         if (shadow) {
-            SPH_CUDA(h, cudaMemcpyAsync(h->W.fa + o, fa.data(), nw * sizeof(float4), cudaMemcpyHostToDevice, st));
             SPH_CUDA(h, cudaMemcpyAsync(h->W.fb + o, fb.data(), nw * sizeof(float4), cudaMemcpyHostToDevice, st));
             SPH_CUDA(h, cudaMemcpyAsync(h->W.fc + o, fc.data(), nw * sizeof(float4), cudaMemcpyHostToDevice, st));
         }
@@ -1035,8 +1080,8 @@ int32_t allocate_handle(SphHandle* h, int64_t cells) {
     if ((e = dalloc(h, &h->W.gap, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
     if ((e = dalloc(h, &h->W.T, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
     if ((e = dalloc(h, &h->W.kappa, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
+    if ((e = dalloc(h, &h->W.fa, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
     if (h->precision == SPH_PRECISION_FP32_COMPENSATED) {
-        if ((e = dalloc(h, &h->W.fa, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
         if ((e = dalloc(h, &h->W.fb, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
         if ((e = dalloc(h, &h->W.fc, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
     }
@@ -1236,7 +1281,7 @@ int32_t sph_upload_fluid(SphHandle* h, int64_t n, const double* x, const double*
     for (int64_t i = 1; i < n; ++i) uniform &= gap[i] == gap[0];
     R.gap0 = n > 0 ? gap[0] : 0.0;
     R.uniform_fluid = uniform;
-    R.dev.uniform_gap = uniform && (!h->has_buffers || h->buffer_gap_uniform(R.gap0)) ? 1 : 0;
+    set_uniform_gap(h->kernel, R.dev, uniform && (!h->has_buffers || h->buffer_gap_uniform(R.gap0)), R.gap0);
     int32_t rc = upload_scene_const(h, 0);
     if (rc != SPH_OK) return rc;
     rc = append_fluid(h, 0, 0, n, x, v, rho, p, c, mass, gap, t, kappa, cp);  // replaces the state
@@ -1401,7 +1446,7 @@ int32_t sph_batch_add_scene(SphHandle* h, const SphParams* params, int64_t first
                             wall_v ? wall_v + w * dim : nullptr);
     bool uniform = true;
     for (int64_t i = 1; i < n; ++i) uniform &= gap[i] == gap[0];
-    R.dev.uniform_gap = uniform ? 1 : 0;
+    set_uniform_gap(h->kernel, R.dev, uniform, n > 0 ? gap[0] : 0.0);
     if (rc == SPH_OK) rc = upload_scene_const(h, s);
     if (rc == SPH_OK) rc = write_scene_walls(h, s);
     if (rc == SPH_OK) rc = append_fluid(h, s, n_before, n, x, v, rho, p, c, mass, gap, t, kappa, cp);
@@ -2050,8 +2095,8 @@ int32_t sph_upload_buffers(SphHandle* h, const SphBufferRules* rules, int64_t ca
     // fluid made from the inlet (or a buffer with another gap) breaks the uniform-gap shortcut
     SceneRec& Rw = h->scenes[0];
     const bool uniform = Rw.uniform_fluid && h->buffer_gap_uniform(Rw.gap0);
-    if ((Rw.dev.uniform_gap != 0) != uniform) {
-        Rw.dev.uniform_gap = uniform ? 1 : 0;
+    if ((Rw.dev.uniform_gap != 0) != (uniform && Rw.gap0 > 0.0)) {
+        set_uniform_gap(h->kernel, Rw.dev, uniform, Rw.gap0);
         int32_t rc = upload_scene_const(h, 0);
         if (rc != SPH_OK) return rc;
     }

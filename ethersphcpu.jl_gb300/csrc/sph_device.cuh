@@ -81,6 +81,17 @@ struct SceneDev {
     double check_hi[3];
     double inv_rho0;  // 1 / rho0 (FP32-compensated form's equation of state)
 
+    // plain FP64 form: constants taken out of the pair sums, and the bounds of the support
+    double inv_h, inv_hh;  // 1 / h, 1 / h^2
+    double kg_h;           // kg_a / h
+    double nu4;            // 4 nu0
+    double wg, inv_wg;     // W(gap) of the tensile term and 1 / W(gap), when uniform_gap
+    double q2_max;         // (r_cut / h)^2, a little more
+    int32_t q2_in_hi;      // pairs with a smaller upper word of q^2 (of d^2) are inside r_cut
+    int32_t d2_in_hi;
+    float sel_e[3];    // cell edges / r_cut
+    float sel_inv_ex;  // 1 / sel_e[0]
+
     // FP32-compensated form
     float cell_f[3];   // cell edge per axis (float)
     float h_f, rc2_f, hh001_f, nu0_f, P_bg_f;
@@ -119,12 +130,13 @@ struct SortedState {
     int32_t* id;
     int32_t* scene;
     // FP32 shadows (allocated only for the compensated form)
+    // (the FP64 form keeps fa = select_pos, see sph_coop.cuh, cell and vol as well)
     float4* fa;   // 2D: (xr, yr, vx, vy)      3D: (xr, yr, zr, m)
     float4* fb;   // 2D: (m, rho, P, gap)      3D: (vx, vy, vz, rho)
     float4* fc;   // 2D: (T, kappa, cp, -)     3D: (P, gap, T, kappa)
     float* fd;    // 3D: cp
     int32_t* cell;  // cell key of the particle (global)
-    double* vol;    // m / rho after continuity (FP32 form: FP64 Shepard weights)
+    double* vol;    // m / rho after continuity
 };
 
 struct NextState {
@@ -144,7 +156,7 @@ struct WallState {
     int32_t* kind;
     int32_t* start;  // global cells + 1
     uint8_t* near;   // global cells: 1 where a wall particle lies within +-reach cells
-    float4* fa;      // FP32: 2D (xr, yr, nx, ny)    3D (xr, yr, zr, gap)
+    float4* fa;      // FP32: 2D (xr, yr, nx, ny)    3D (xr, yr, zr, gap); FP64: select_pos
     float4* fb;      // FP32: 2D (vx, vy, gap, T)    3D (nx, ny, nz, T)
     float4* fc;      // FP32: 2D (kappa, kind, -, -) 3D (vx, vy, vz, kappa)
     int32_t* cell;
@@ -278,6 +290,13 @@ __device__ __forceinline__ int32_t cell_coord(double x, const SceneDev& S, int a
 __device__ __forceinline__ bool outside_grid(double x, const SceneDev& S, int a) {
     const double u = (x - S.lo[a]) * S.inv_cell[a];
     return !(u >= 0.0) || u >= (double)S.n[a];
+}
+
+__device__ __forceinline__ void decode_cell(int32_t key, const SceneDev& S, int32_t c[3]) {
+    const int32_t k = key - S.cell_off;
+    c[0] = k % S.n[0];
+    c[1] = (k / S.n[0]) % S.n[1];
+    c[2] = k / (S.n[0] * S.n[1]);
 }
 
 // ---------------------------------------------------------------- Julia numerics

@@ -454,13 +454,6 @@ struct Cand3S {
     double vol, m;
 };
 
-__device__ __forceinline__ void decode_cell(int32_t key, const SceneDev& S, int32_t c[3]) {
-    const int32_t k = key - S.cell_off;
-    c[0] = k % S.n[0];
-    c[1] = (k / S.n[0]) % S.n[1];
-    c[2] = k / (S.n[0] * S.n[1]);
-}
-
 // -------------------------------------------------------------------- K4 (FP32)
 // LIST (one lane per particle): also records the neighbours within r_cut in nl.
 template <int DIM, int KK, int TPP, bool PF, bool LIST>

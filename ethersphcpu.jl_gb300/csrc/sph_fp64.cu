@@ -1,4 +1,6 @@
-// sph_fp64.cu — plain FP64 gather kernels of the WCSPH step (compiled -fmad=false).
+// sph_fp64.cu — plain FP64 gather kernels of the WCSPH step (compiled -fmad=false: the
+// per-particle updates keep the reference's unfused operations; the pair terms write their
+// fused multiply-adds out).
 //
 // K4 continuity + updateDensity! + updatePressure!   (Continuity.jl:8-17,
 //    UpdateDensity.jl:8-12, UpdatePressure.jl:8-16)
@@ -7,88 +9,132 @@
 //    cell hash of the next step's sort   (PressureForce.jl, ViscosityForce.jl,
 //    WallForce.jl, ThermalConduction.jl, SelfAction/*.jl, FluidWallSolve.jl:37-81)
 // On a re-initialisation step K5 also forms the Shepard sums of reconstructScalar!
-//    (ReconstructValue.jl:22-57) over the same fluid neighbours, in the same order, at
-//    the same start-of-step positions, and writes the re-initialised density: the update
-//    and the re-initialisation are one kernel (FluidWallSolve.jl:64-72).
+//    (ReconstructValue.jl:22-57) over the same fluid neighbours at the same start-of-step
+//    positions, and writes the re-initialised density: the update and the
+//    re-initialisation are one kernel (FluidWallSolve.jl:64-72).
 //
-// One thread per fluid particle in sorted (cell, id) order; each thread sums its own
-// full neighbour list in a fixed order (cells z, y, x; particles by id), so there are
-// no atomics on the physics and results are deterministic.  Walls are visited after
-// fluid neighbours.  The reference scatters each unordered pair to both particles
-// with atomics; every pair term here is the bitwise same number the reference adds
-// (the pair formulas are antisymmetric under exact negation), only the order of the
-// additions differs.
-#include "sph_physics.cuh"
-#include "sph_kernels.h"
+// Eight lanes share one fluid particle (sph_coop.cuh): FP32 selection of its neighbours
+// into shared memory, FP64 pair terms over that list, and one thread that updates the
+// particle.  No atomics on the physics, a fixed order of every sum: results are
+// deterministic and do not depend on the batch or the block size.
+//
+// What bounds them: FP64 instructions (2 lanes a SM and cycle).
+//   * K4 and the viscosity and heat terms of K5 are factored so that a pair divides once or
+//     not at all: r by one Householder step on rsqrt, dW/r as the kernel's own polynomial
+//     (no normalisation of r_vec), constants outside the sums, m/rho formed once a particle,
+//     one reciprocal for the quotients of viscosity and heat.
+//   * pressure and wall forces cancel to a 1e-9 th of themselves in a fluid at rest, so their
+//     terms keep the reference's operations, rounding and order of addition; what changes
+//     is their cost: root and reciprocal share one iteration, division by h and W(gap) is a
+//     multiplication with a residual step, and rejected candidates cost no FP64 at all.
+#include "sph_coop.cuh"
 
 namespace sph {
 
 // Solve variants: which wall terms and which body force.
 enum { kModeFluidWall = 0, kModeWallPressure = 1, kModeThermal = 2, kModeBuffers = 3 };
 
+// Sum of a particle's partial sums (one per lane) in a fixed tree order.
+__device__ __forceinline__ double lane_sum(const double* part) {
+    const double a = (part[0] + part[kCoopStride]) + (part[2 * kCoopStride] + part[3 * kCoopStride]);
+    const double b = (part[4 * kCoopStride] + part[5 * kCoopStride]) + (part[6 * kCoopStride] + part[7 * kCoopStride]);
+    return a + b;
+}
+
+// Geometry of the pair (i, j): r_vec and q^2 = |r_vec|^2 / h^2.
+template <int DIM, typename V>
+__device__ __forceinline__ double pair_q2(const V& xi, const V& xj, const SceneDev& S, double rv[DIM]) {
+    make_rvec<DIM>(xi, xj, S, rv);
+    double d2 = fma(rv[0], rv[0], rv[1] * rv[1]);
+    if (DIM == 3) d2 = fma(rv[DIM - 1], rv[DIM - 1], d2);
+    return d2 * S.inv_hh;
+}
+
+template <int DIM, typename V>
+__device__ __forceinline__ void vec_diff(const V& a, const V& b, double d[DIM]) {
+    d[0] = a.x - b.x;
+    d[1] = a.y - b.y;
+    if (DIM == 3) d[DIM - 1] = comp(a, DIM - 1) - comp(b, DIM - 1);
+}
+
+template <int DIM>
+__device__ __forceinline__ double dot_fma(const double a[DIM], const double b[DIM]) {
+    double s = fma(a[0], b[0], a[1] * b[1]);
+    if (DIM == 3) s = fma(a[DIM - 1], b[DIM - 1], s);
+    return s;
+}
+
+// d^2 <= r_cut^2 in FP64, for the selection of particles far outside the grid.
+template <int DIM, typename V>
+__device__ __forceinline__ bool within_cut(const V& xi, const V& xj, const SceneDev& S) {
+    double rv[DIM];
+    make_rvec<DIM>(xi, xj, S, rv);
+    return norm_sq<DIM>(rv) <= S.rc2;
+}
+
 template <int DIM, int KK>
-__global__ void __launch_bounds__(128) k_continuity_fp64(const SceneDev* __restrict__ scenes, SortedState st,
-                                                         SortScratch sc, int32_t cap, BufferState bf) {
+__global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
+    k_continuity_fp64(const SceneDev* __restrict__ scenes, SortedState st, SortScratch sc, int32_t cap, BufferState bf) {
+    pdl_wait();
     using V = typename VecT<DIM>::T;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cap || i >= *sc.n_live) return;
-    const int32_t s = st.scene[i];
-    const SceneDev& S = scenes[s];
-    if (!scene_runs(S, sc.scene_step[s])) return;
-    const int32_t* __restrict__ start = sc.start;
+    __shared__ int32_t lists[kCoopMaxParticles * kCoopList<DIM>];
+    __shared__ double part[kCoopLanes * kCoopStride];
+    const int g = threadIdx.x / kCoopLanes, lane = threadIdx.x % kCoopLanes;
+    const int i0 = blockIdx.x * (blockDim.x / kCoopLanes);
+    const int n = min(cap, *sc.n_live);
+    if (i0 >= n) return;  // the whole block
     const V* __restrict__ x = (const V*)st.x;
     const V* __restrict__ v = (const V*)st.v;
-    const V xi = x[i];
-    const V vi = v[i];
-    int32_t c[3];
-    cell_of<DIM>(xi, S, c);
-    float xd[3];
-    cell_units<DIM>(xi, S, c, xd);
-    double drho = 0.0;
-    walk_cells_pruned<DIM>(S, start, c, xd, [&](int jb, int je) {
-        for (int j = jb; j < je; ++j) {
-            if (j == i) continue;
-            const V xj = x[j];
-            double rv[DIM];
-            make_rvec<DIM>(xi, xj, S, rv);
-            const double d2 = norm_sq<DIM>(rv);
-            if (!(d2 <= S.rc2)) continue;
-            const double r = sqrt(d2);
-            double W, dW;
-            kernel_wdw<KK>(r, S, W, dW);
-            double g[DIM];
-            grad_vec<DIM>(dW, r, rv, g);
-            const V vj = v[j];
-            double vv[DIM];
-            vv[0] = vi.x - vj.x;
-            vv[1] = vi.y - vj.y;
-            if (DIM == 3) vv[DIM - 1] = comp(vi, DIM - 1) - comp(vj, DIM - 1);
-            drho += dotd<DIM>(vv, g) * st.m[j];
+    const double* __restrict__ m = st.m;
+    {
+        const int i = min(i0 + g, n - 1);
+        const SceneDev& S = scenes[st.scene[i]];
+        const bool on = i0 + g < n && scene_runs(S, sc.scene_step[st.scene[i]]);
+        const V xi = x[i];
+        const V vi = v[i];
+        int32_t c[3];
+        decode_cell(st.cell[i], S, c);
+        int32_t* list = lists + g * kCoopList<DIM>;
+        double drho = 0.0;
+        coop_select<DIM>(
+            S, sc.start, st.fa, c, st.fa[i], i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
+            [&](int first, int cnt) {
+                for (int k = (lane - first) & (kCoopLanes - 1); k < cnt; k += kCoopLanes) {
+                    const int j = list[k];
+                    const V xj = x[j];
+                    const V vj = v[j];
+                    const double m_j = m[j];
+                    double rv[DIM], vv[DIM];
+                    const double q2 = pair_q2<DIM>(xi, xj, S, rv);
+                    if (!inside_cut<DIM, KK>(rv, q2, S)) continue;
+                    vec_diff<DIM>(vi, vj, vv);
+                    drho = fma(m_j * kernel_f<KK>(q2), dot_fma<DIM>(rv, vv), drho);
+                }
+            });
+        drho *= S.kg_h;
+        if (on && bf.n) {  // inlet/outlet buffer neighbours (FluidInletOutletWallSolve.jl:59-72)
+            const V* __restrict__ bx = (const V*)bf.x;
+            const V* __restrict__ bv = (const V*)bf.v;
+            walk_cells<DIM>(S, bf.start, c, [&](int jb, int je) {
+                for (int b = jb + lane; b < je; b += kCoopLanes) {
+                    double rv[DIM], vv[DIM];
+                    const double q2 = pair_q2<DIM>(xi, bx[b], S, rv);
+                    if (!(q2 <= S.q2_max) || !inside_cut<DIM, KK>(rv, q2, S)) continue;
+                    vec_diff<DIM>(vi, bv[b], vv);
+                    drho = fma(bf.m[b] * kernel_f<KK>(q2) * S.kg_h, dot_fma<DIM>(rv, vv), drho);
+                }
+            });
         }
-    });
-    if (bf.n) {  // inlet/outlet buffer neighbours (FluidInletOutletWallSolve.jl:59-72)
-        const V* __restrict__ bx = (const V*)bf.x;
-        const V* __restrict__ bv = (const V*)bf.v;
-        walk_cells<DIM>(S, bf.start, c, [&](int jb, int je) {
-            for (int b = jb; b < je; ++b) {
-                double rv[DIM];
-                make_rvec<DIM>(xi, bx[b], S, rv);
-                const double d2 = norm_sq<DIM>(rv);
-                if (!(d2 <= S.rc2)) continue;
-                const double r = sqrt(d2);
-                double W, dW;
-                kernel_wdw<KK>(r, S, W, dW);
-                double g[DIM];
-                grad_vec<DIM>(dW, r, rv, g);
-                const V vb = bv[b];
-                double vv[DIM];
-                vv[0] = vi.x - vb.x;
-                vv[1] = vi.y - vb.y;
-                if (DIM == 3) vv[DIM - 1] = comp(vi, DIM - 1) - comp(vb, DIM - 1);
-                drho += dotd<DIM>(vv, g) * bf.m[b];
-            }
-        });
+        part[lane * kCoopStride + g] = drho;
     }
+    __syncthreads();
+    // the update, one thread a particle
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= blockDim.x / kCoopLanes || i >= n) return;
+    const SceneDev& S = scenes[st.scene[i]];
+    if (!scene_runs(S, sc.scene_step[st.scene[i]])) return;
+    const double drho = lane_sum(part + threadIdx.x);
+    const double m_i = m[i];
     double rho = st.rho[i];
     rho += drho * S.dt;  // written to rhoc, so the kernel can be re-run on the same input
     const double rr = rho / S.rho0;
@@ -98,6 +144,7 @@ __global__ void __launch_bounds__(128) k_continuity_fp64(const SceneDev* __restr
     st.p[i] = p;
     st.c[i] = cs;
     st.P[i] = p / (rho * rho);
+    st.vol[i] = m_i / rho;
 }
 
 // SHEP: the momentum gather of density re-initialisation steps, for the particles of the
@@ -105,205 +152,282 @@ __global__ void __launch_bounds__(128) k_continuity_fp64(const SceneDev* __restr
 // `sel` set leaves those particles to the SHEP launch of the same step (a batch whose
 // scenes re-initialise at different steps runs both).
 template <int DIM, int KK, int MODE, bool SHEP>
-__global__ void __launch_bounds__(128) k_momentum_fp64(const SceneDev* __restrict__ scenes, SortedState st,
-                                                       NextState nx, WallState wl, SortScratch sc,
-                                                       int32_t cap, BufferState bf, BufferScratch bs,
-                                                       BufferRules br, int sel) {
+__global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
+    k_momentum_fp64(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl, SortScratch sc,
+                    int32_t cap, BufferState bf, BufferScratch bs, BufferRules br, int sel) {
+    pdl_wait();
     using V = typename VecT<DIM>::T;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cap || i >= *sc.n_live) return;
-    const int32_t s = st.scene[i];
-    const SceneDev& S = scenes[s];
-    const int64_t step = sc.scene_step[s];
-    const bool runs = scene_runs(S, step);
-    const bool reinit_scene = runs && is_step(step, S.reinit_interval);
-    if (SHEP ? !(runs && (sel || reinit_scene)) : (sel && reinit_scene)) return;
-    if (!runs) {
-        carry_frozen<DIM>(i, S, st, nx, sc);
-        return;
-    }
+    constexpr bool HEAT = MODE == kModeThermal;
+    constexpr int kSums = (HEAT ? 2 : 0) + (SHEP ? 2 : 0);  // sums taken by lane
+    __shared__ int32_t lists[kCoopMaxParticles * kCoopList<DIM>];
+    __shared__ double terms_all[kCoopMaxParticles * kCoopLanes / 32 * 3 * DIM * kTermStride];
+    __shared__ double part[(kSums ? kSums : 1) * kCoopLanes * kCoopStride];
+    __shared__ double dv_all[DIM * kCoopMaxParticles];
+    const int g = threadIdx.x / kCoopLanes, lane = threadIdx.x % kCoopLanes;
+    const int i0 = blockIdx.x * (blockDim.x / kCoopLanes);
+    const int n = min(cap, *sc.n_live);
+    if (i0 >= n) return;  // the whole block
     const V* __restrict__ x = (const V*)st.x;
     const V* __restrict__ v = (const V*)st.v;
+    auto takes = [&](const SceneDev& S, int64_t step) {  // the particle's sums are formed by this launch
+        const bool runs = scene_runs(S, step);
+        if (SHEP) return runs && (sel || is_step(step, S.reinit_interval));
+        return runs && !(sel && is_step(step, S.reinit_interval));
+    };
+    {
+        const int i = min(i0 + g, n - 1);
+        const SceneDev& S = scenes[st.scene[i]];
+        const bool on = i0 + g < n && takes(S, sc.scene_step[st.scene[i]]);
+        const int shift = (threadIdx.x & 31) & ~(kCoopLanes - 1);
+        double* terms = terms_all + threadIdx.x / 32 * (3 * DIM * kTermStride);
+        double* mine = terms + (threadIdx.x & 31);  // this lane's place in a row of terms
+        const V xi = x[i];
+        const V vi = v[i];
+        const double rho_i = st.rhoc[i];
+        const double P_i = st.P[i];
+        const double gap_i = st.gap[i];
+        // W((gap_i + gap_j)/2) of the tensile term: with uniform gaps a constant of the scene
+        const bool uniform = S.uniform_gap != 0;
+        double T_i = 0.0, kap_i = 0.0;
+        if (HEAT) {
+            T_i = st.T[i];
+            kap_i = st.kappa[i];
+        }
+        int32_t c[3];
+        decode_cell(st.cell[i], S, c);
+        const float4 me = st.fa[i];
+        int32_t* list = lists + g * kCoopList<DIM>;
+        double dv = 0.0;  // lane d < DIM: component d of the acceleration
+        double aT = 0.0, wT = 0.0, sw = 0.0, sws = 0.0;
+
+        // rounds of a list pass: the entries' places are those of the whole list (first + k),
+        // so a lane's entries do not depend on where the passes are cut
+        auto rounds = [&](int first, int cnt, auto&& body) {
+            const int r0 = first / kCoopLanes, r1 = (first + cnt + kCoopLanes - 1) / kCoopLanes;
+            const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)(r1 - r0));
+            for (int r = 0; r < most; ++r) {
+                const int at = (r0 + r) * kCoopLanes - first;  // entry of lane 0
+                body(at + lane, max(0, -at), min(kCoopLanes, cnt - at));
+            }
+        };
+
+        // ---- fluid neighbours: pressureForce! + viscosityForce! (+ thermalConduction!),
+        // PressureForce.jl:14-19, ViscosityForce.jl:15-23, ThermalConduction.jl:15-21.  With
+        // mu = nu0 rho the viscosity factor is 4 nu0 m_j r dW / ((rho_i + rho_j) (r^2 + 0.01 h^2));
+        // heat is taken as aT = sum m_j/rho_j kappa_j r dW / ((kappa_i + kappa_j) (r^2 + 0.01 h^2)) T_ij
+        coop_select<DIM>(
+            S, sc.start, st.fa, c, me, i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
+            [&](int first, int cnt) {
+                rounds(first, cnt, [&](int k, int e0, int e1) {
+                    double tp[DIM], tv[DIM];
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) tp[d] = tv[d] = 0.0;
+                    if (k >= 0 && k < cnt) {
+                        const int j = list[k];
+                        const V xj = x[j];
+                        const V vj = v[j];
+                        const double m_j = st.m[j], rho_j = st.rhoc[j], P_j = st.P[j];
+                        double vol_j = 0.0, kap_j = 0.0, T_j = 0.0;
+                        if (HEAT || SHEP) vol_j = st.vol[j];
+                        if (HEAT) {
+                            kap_j = st.kappa[j];
+                            T_j = st.T[j];
+                        }
+                        double rv[DIM];
+                        make_rvec<DIM>(xi, xj, S, rv);
+                        const double d2 = norm_sq<DIM>(rv);
+                        if (inside_cut<KK>(d2, S)) {
+                            double r, W, dW, grad[DIM], vv[DIM];
+                            pair_kernel<DIM, KK>(rv, d2, S, r, W, dW, grad);
+                            if (SHEP) {
+                                sw = fma(W, vol_j, sw);
+                                sws = fma(W, m_j, sws);
+                            }
+                            double prho2 = P_i + P_j;
+                            const double tens = fabs(prho2) * 0.01 * W;
+                            prho2 += uniform ? div_rn(tens, S.wg, S.inv_wg)
+                                             : tens / kernel_w<KK>((gap_i + st.gap[j]) / 2.0, S);
+                            const double fp = -m_j * prho2;
+                            vec_diff<DIM>(vi, vj, vv);
+                            const double sum_rho = rho_i + rho_j;
+                            const double rdW = r * dW;
+                            const double den = sum_rho * (d2 + S.hh001);
+                            double fv;
+                            if (HEAT) {
+                                const double sum_kap = kap_i + kap_j;
+                                const double R = rcp3(den * sum_kap);
+                                fv = m_j * (S.nu4 * rdW) * (R * sum_kap);
+                                aT = fma(rdW * vol_j * (R * sum_rho * kap_j), T_i - T_j, aT);
+                            } else {
+                                fv = m_j * (S.nu4 * rdW) * rcp3(den);
+                            }
+#pragma unroll
+                            for (int d = 0; d < DIM; ++d) {
+                                tp[d] = fp * grad[d];
+                                tv[d] = fv * vv[d];
+                            }
+                        }
+                    }
+#pragma unroll
+                    for (int d = 0; d < DIM; ++d) {
+                        mine[d * kTermStride] = tp[d];
+                        mine[(DIM + d) * kTermStride] = tv[d];
+                    }
+                    __syncwarp();
+                    add_terms<DIM, 2>(terms, lane, shift, e0, e1, dv);
+                    __syncwarp();
+                });
+            });
+
+        // ---- inlet/outlet buffer neighbours: pressureForce! + viscosityForce! with the
+        // buffer particle's frozen density and pressure (FluidInletOutletWallSolve.jl:125-158)
+        if (MODE == kModeBuffers) {
+            const V* __restrict__ bx = (const V*)bf.x;
+            const V* __restrict__ bv = (const V*)bf.v;
+            double db[DIM];  // every lane of the particle continues the whole sum (few particles do)
+#pragma unroll
+            for (int d = 0; d < DIM; ++d) db[d] = __shfl_sync(0xffffffffu, dv, d, kCoopLanes);
+            if (on && bf.n) {
+                walk_cells<DIM>(S, bf.start, c, [&](int jb, int je) {
+                    for (int b = jb; b < je; ++b) {
+                        double rv[DIM], vv[DIM];
+                        make_rvec<DIM>(xi, bx[b], S, rv);
+                        const double d2 = norm_sq<DIM>(rv);
+                        if (!(d2 <= S.rc2)) continue;
+                        double r, W, dW, grad[DIM];
+                        pair_kernel<DIM, KK>(rv, d2, S, r, W, dW, grad);
+                        vec_diff<DIM>(vi, bv[b], vv);
+                        const double rho_b = bf.rho[b], m_b = bf.m[b], gap_b = bf.gap[b];
+                        double prho2 = P_i + bf.p[b] / (rho_b * rho_b);
+                        prho2 += fabs(prho2) * 0.01 * W / kernel_w<KK>(gap_b == gap_i ? gap_i : (gap_i + gap_b) / 2.0, S);
+                        const double fv = S.nu4 * (r * dW) / ((rho_i + rho_b) * (d2 + S.hh001));
+#pragma unroll
+                        for (int k = 0; k < DIM; ++k) db[k] += -m_b * prho2 * grad[k];
+#pragma unroll
+                        for (int k = 0; k < DIM; ++k) db[k] += m_b * fv * vv[k];
+                    }
+                });
+            }
+#pragma unroll
+            for (int d = 0; d < DIM; ++d)
+                if (lane == d) dv = db[d];
+        }
+
+        // ---- walls: wallForce! (+ background pressureForce!) + viscosityForce! (+ heat),
+        // only where a wall cell is within reach of the particle's cell
+        const bool walls = on && wl.n > 0 && wl.near[st.cell[i]];
+        if (__any_sync(0xffffffffu, walls)) {
+            const V* __restrict__ wx = (const V*)wl.x;
+            const V* __restrict__ wn = (const V*)wl.nrm;
+            const V* __restrict__ wv = (const V*)wl.v;
+            const double c_i = st.c[i];
+            const double m_i = st.m[i];
+            const double Pw = P_i + S.P_bg;
+            const double Wg_i = uniform ? S.wg : kernel_w<KK>(gap_i, S);
+            const double nu_rho = 2.0 * S.nu0 / rho_i;  // 8 mu_i / (2 rho_i)^2
+            coop_select<DIM>(
+                S, wl.start, wl.fa, c, me, -1, walls, list, [&](int j) { return within_cut<DIM>(xi, wx[j], S); },
+                [&](int first, int cnt) {
+                    rounds(first, cnt, [&](int k, int e0, int e1) {
+                        double tw[DIM], tp[DIM], tv[DIM];
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) tw[d] = tp[d] = tv[d] = 0.0;
+                        if (k >= 0 && k < cnt) {
+                            const int j = list[k];
+                            const V nw = wn[j];
+                            double rv[DIM];
+                            make_rvec<DIM>(xi, wx[j], S, rv);
+                            const double d2 = norm_sq<DIM>(rv);
+                            if (inside_cut<KK>(d2, S)) {
+                                double r, W, dW, grad[DIM], vv[DIM], nn[DIM];
+                                pair_kernel<DIM, KK>(rv, d2, S, r, W, dW, grad);
+                                vec_diff<DIM>(vi, wv[j], vv);
+                                nn[0] = nw.x;
+                                nn[1] = nw.y;
+                                if (DIM == 3) nn[DIM - 1] = comp(nw, DIM - 1);
+                                const double vert = dotd<DIM>(vv, nn);
+                                {  // WallForce.jl:15-28 (Rogers & Dalrymple 2008)
+                                    const double gw = wl.gap[j];
+                                    const double psi = fabs(dotd<DIM>(rv, nn));
+                                    double t = r * r - psi * psi;
+                                    t = t < 0.0 ? 0.0 : t;  // NaN stays
+                                    const double far = gw * (1.0 + 1e-9);
+                                    if (!(psi > far || t > far * far)) {
+                                        const double xi_ = sqrt(t);
+                                        const double q = psi / gw;
+                                        if (!(q > 1.0 || xi_ > gw)) {
+                                            const double pxi = fabs((1.0 + cos(CUDART_PI * xi_ / gw)) / 2.0);
+                                            const double beta = vert > 0.0 ? 0.0 : 1.0;
+                                            const double rpsi = (0.01 * (c_i * c_i) + beta * c_i * fabs(vert)) / S.h *
+                                                                fabs(1.0 - q) / sqrt(q);
+                                            const double wf = rpsi * pxi;
+#pragma unroll
+                                            for (int d = 0; d < DIM; ++d) tw[d] = wf * nn[d];
+                                        }
+                                    }
+                                }
+                                if (MODE == kModeWallPressure || HEAT) {  // PressureForce.jl:29-33
+                                    const double tens = fabs(Pw) * 0.01 * W;
+                                    const double prho2 = Pw + (uniform ? div_rn(tens, S.wg, S.inv_wg) : tens / Wg_i);
+#pragma unroll
+                                    for (int d = 0; d < DIM; ++d) tp[d] = -m_i * prho2 * grad[d];
+                                }
+                                // ViscosityForce.jl:34-44
+                                const double rdW = r * dW * rcp3(d2 + S.hh001);
+                                const double fv = m_i * (nu_rho * rdW);
+#pragma unroll
+                                for (int d = 0; d < DIM; ++d) tv[d] = fv * fma(-vert, nn[d], vv[d]);
+                                if (HEAT && wl.kind[j] == SPH_WALL_THERMOSTATIC)  // ThermalConduction.jl:31-35
+                                    wT = fma((kap_i + wl.kappa[j]) * rdW, T_i - wl.T[j], wT);
+                            }
+                        }
+#pragma unroll
+                        for (int d = 0; d < DIM; ++d) {
+                            mine[d * kTermStride] = tw[d];
+                            mine[(DIM + d) * kTermStride] = tp[d];
+                            mine[(2 * DIM + d) * kTermStride] = tv[d];
+                        }
+                        __syncwarp();
+                        add_terms<DIM, 3>(terms, lane, shift, e0, e1, dv);
+                        __syncwarp();
+                    });
+                });
+        }
+        if (lane < DIM) dv_all[lane * kCoopMaxParticles + g] = dv;
+        double* sums = part + lane * kCoopStride + g;
+        if (HEAT) {
+            sums[0] = aT;
+            sums[kCoopLanes * kCoopStride] = wT;
+        }
+        if (SHEP) {
+            sums[(kSums - 2) * kCoopLanes * kCoopStride] = sw;
+            sums[(kSums - 1) * kCoopLanes * kCoopStride] = sws;
+        }
+    }
+    __syncthreads();
+
+    // ---- the update, one thread a particle
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= blockDim.x / kCoopLanes || i >= n) return;
+    const SceneDev& S = scenes[st.scene[i]];
+    const int64_t step = sc.scene_step[st.scene[i]];
+    if (!takes(S, step)) {
+        if (!SHEP && !scene_runs(S, step)) carry_frozen<DIM>(i, S, st, nx, sc);
+        return;
+    }
     const V xi = x[i];
     const V vi = v[i];
     const double rho_i = st.rhoc[i];
-    const double P_i = st.P[i];
     const double m_i = st.m[i];
-    const double gap_i = st.gap[i];
-    const double c_i = st.c[i];
-    const double mu_i = S.nu0 * rho_i;
-    double T_i = 0.0, kap_i = 0.0, cp_i = 1.0;
-    if (MODE == kModeThermal) {
-        T_i = st.T[i];
-        kap_i = st.kappa[i];
-        cp_i = st.cp[i];
-    }
-    // W((gap_i + gap_j)/2) of the tensile term; with uniform gaps it is W(gap_i).
-    const double Wg_i = kernel_w<KK>(gap_i, S);
-    int32_t c[3];
-    cell_of<DIM>(xi, S, c);
-    float xd[3];
-    cell_units<DIM>(xi, S, c, xd);
+    const double* sums = part + threadIdx.x;
     double dv[DIM];
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) dv[k] = 0.0;
-    double dT = 0.0;
-    // Shepard sums (ReconstructValue.jl:28-50): sum W m_j/rho_j and sum W m_j/rho_j rho_j
-    // over the fluid neighbours, with the post-continuity densities
-    double sw = 0.0, sws = 0.0;
-
-    // ---- fluid neighbours: pressureForce! + viscosityForce! (+ thermalConduction!)
-    walk_cells_pruned<DIM>(S, sc.start, c, xd, [&](int jb, int je) {
-        for (int j = jb; j < je; ++j) {
-            if (j == i) continue;
-            const V xj = x[j];
-            double rv[DIM];
-            make_rvec<DIM>(xi, xj, S, rv);
-            const double d2 = norm_sq<DIM>(rv);
-            if (!(d2 <= S.rc2)) continue;
-            const double r = sqrt(d2);
-            double W, dW;
-            kernel_wdw<KK>(r, S, W, dW);
-            double g[DIM];
-            grad_vec<DIM>(dW, r, rv, g);
-            const V vj = v[j];
-            double vv[DIM];
-            vv[0] = vi.x - vj.x;
-            vv[1] = vi.y - vj.y;
-            if (DIM == 3) vv[DIM - 1] = comp(vi, DIM - 1) - comp(vj, DIM - 1);
-            const double rho_j = st.rhoc[j];
-            const double m_j = st.m[j];
-            if (SHEP) {
-                sw += W * m_j / rho_j;
-                sws += W * m_j / rho_j * rho_j;
-            }
-            // PressureForce.jl:14-19
-            double prho2 = P_i + st.P[j];
-            const double Wg = S.uniform_gap ? Wg_i : kernel_w<KK>((gap_i + st.gap[j]) / 2.0, S);
-            prho2 += fabs(prho2) * 0.01 * W / Wg;
-#pragma unroll
-            for (int k = 0; k < DIM; ++k) dv[k] += -m_j * prho2 * g[k];
-            // ViscosityForce.jl:15-23
-            const double sum_rho = rho_i + rho_j;
-            const double mu_j = S.nu0 * rho_j;
-            const double f = 4.0 * (mu_i + mu_j) * r * dW / (sum_rho * sum_rho) / (r * r + S.hh001);
-#pragma unroll
-            for (int k = 0; k < DIM; ++k) dv[k] += m_j * f * vv[k];
-            if (MODE == kModeThermal) {  // ThermalConduction.jl:15-21
-                const double kap_j = st.kappa[j];
-                const double keq = 2.0 * kap_i * kap_j / (kap_i + kap_j);
-                const double dq = 2.0 * keq * r * dW / rho_i / rho_j / (r * r + S.hh001) * (T_i - st.T[j]);
-                dT += dq * m_j / cp_i;
-            }
-        }
-    });
-
-    // ---- inlet/outlet buffer neighbours: pressureForce! + viscosityForce! with the
-    // buffer particle's frozen density and pressure (FluidInletOutletWallSolve.jl:125-158)
-    if (MODE == kModeBuffers && bf.n) {
-        const V* __restrict__ bx = (const V*)bf.x;
-        const V* __restrict__ bv = (const V*)bf.v;
-        walk_cells<DIM>(S, bf.start, c, [&](int jb, int je) {
-            for (int b = jb; b < je; ++b) {
-                double rv[DIM];
-                make_rvec<DIM>(xi, bx[b], S, rv);
-                const double d2 = norm_sq<DIM>(rv);
-                if (!(d2 <= S.rc2)) continue;
-                const double r = sqrt(d2);
-                double W, dW;
-                kernel_wdw<KK>(r, S, W, dW);
-                double g[DIM];
-                grad_vec<DIM>(dW, r, rv, g);
-                const V vb = bv[b];
-                double vv[DIM];
-                vv[0] = vi.x - vb.x;
-                vv[1] = vi.y - vb.y;
-                if (DIM == 3) vv[DIM - 1] = comp(vi, DIM - 1) - comp(vb, DIM - 1);
-                const double rho_b = bf.rho[b];
-                const double m_b = bf.m[b];
-                const double gap_b = bf.gap[b];
-                double prho2 = P_i + bf.p[b] / (rho_b * rho_b);
-                const double Wg = gap_b == gap_i ? Wg_i : kernel_w<KK>((gap_i + gap_b) / 2.0, S);
-                prho2 += fabs(prho2) * 0.01 * W / Wg;
-#pragma unroll
-                for (int k = 0; k < DIM; ++k) dv[k] += -m_b * prho2 * g[k];
-                const double sum_rho = rho_i + rho_b;
-                const double mu_b = S.nu0 * rho_b;
-                const double f = 4.0 * (mu_i + mu_b) * r * dW / (sum_rho * sum_rho) / (r * r + S.hh001);
-#pragma unroll
-                for (int k = 0; k < DIM; ++k) dv[k] += m_b * f * vv[k];
-            }
-        });
-    }
-
-    // ---- walls: wallForce! (+ background pressureForce!) + viscosityForce! (+ heat)
-    if (wl.n > 0) {
-        const V* __restrict__ wx = (const V*)wl.x;
-        const V* __restrict__ wn = (const V*)wl.nrm;
-        const V* __restrict__ wv = (const V*)wl.v;
-        const double Wgap_bg = Wg_i;  // kernelValue(p_i.gap_) of PressureForce.jl:30
-        walk_cells_pruned<DIM>(S, wl.start, c, xd, [&](int jb, int je) {
-            for (int w = jb; w < je; ++w) {
-                const V xw = wx[w];
-                double rv[DIM];
-                make_rvec<DIM>(xi, xw, S, rv);
-                const double d2 = norm_sq<DIM>(rv);
-                if (!(d2 <= S.rc2)) continue;
-                const double r = sqrt(d2);
-                double W, dW;
-                kernel_wdw<KK>(r, S, W, dW);
-                double g[DIM];
-                grad_vec<DIM>(dW, r, rv, g);
-                const V vw = wv[w];
-                const V nw = wn[w];
-                double vv[DIM], n[DIM];
-                vv[0] = vi.x - vw.x;
-                vv[1] = vi.y - vw.y;
-                n[0] = nw.x;
-                n[1] = nw.y;
-                if (DIM == 3) {
-                    vv[DIM - 1] = comp(vi, DIM - 1) - comp(vw, DIM - 1);
-                    n[DIM - 1] = comp(nw, DIM - 1);
-                }
-                const double gw = wl.gap[w];
-                // WallForce.jl:15-28 (Rogers & Dalrymple 2008)
-                {
-                    const double psi = fabs(dotd<DIM>(rv, n));
-                    double t = r * r - psi * psi;
-                    t = isnan(t) ? t : (t > 0.0 ? t : 0.0);
-                    const double xi_ = sqrt(t);
-                    const double q = psi / gw;
-                    if (!(q > 1.0 || xi_ > gw)) {
-                        const double pxi = fabs((1.0 + cos(CUDART_PI * xi_ / gw)) / 2.0);
-                        const double vert = dotd<DIM>(vv, n);
-                        const double beta = vert > 0.0 ? 0.0 : 1.0;
-                        const double rpsi =
-                            (0.01 * (c_i * c_i) + beta * c_i * fabs(vert)) / S.h * fabs(1.0 - q) / sqrt(q);
-                        const double wf = rpsi * pxi;
-#pragma unroll
-                        for (int k = 0; k < DIM; ++k) dv[k] += wf * n[k];
-                    }
-                }
-                if (MODE == kModeWallPressure || MODE == kModeThermal) {  // PressureForce.jl:29-33
-                    double prho2 = P_i + S.P_bg;
-                    prho2 += fabs(prho2) * 0.01 * W / Wgap_bg;
-#pragma unroll
-                    for (int k = 0; k < DIM; ++k) dv[k] += -m_i * prho2 * g[k];
-                }
-                {  // ViscosityForce.jl:34-44
-                    const double sum_rho = 2.0 * rho_i;
-                    const double f = 8.0 * mu_i * r * dW / (sum_rho * sum_rho) / (r * r + S.hh001);
-                    const double vert = dotd<DIM>(vv, n);
-#pragma unroll
-                    for (int k = 0; k < DIM; ++k) dv[k] += m_i * f * (vv[k] - vert * n[k]);
-                }
-                if (MODE == kModeThermal && wl.kind[w] == SPH_WALL_THERMOSTATIC) {  // ThermalConduction.jl:31-35
-                    const double dq = S.inv_cp_d * (kap_i + wl.kappa[w]) * r * dW / rho_i / S.rho0 /
-                                      (r * r + S.hh001) * (T_i - wl.T[w]);
-                    dT += dq * m_i;
-                }
-            }
-        });
+    for (int k = 0; k < DIM; ++k) dv[k] = dv_all[k * kCoopMaxParticles + threadIdx.x];
+    double T_i = 0.0, dT = 0.0;
+    if (HEAT) {
+        T_i = st.T[i];
+        const double fluid = lane_sum(sums), wall = lane_sum(sums + kCoopLanes * kCoopStride);
+        dT = (4.0 * st.kappa[i] / st.cp[i] * fluid + m_i * S.inv_cp_d / S.rho0 * wall) / rho_i;
     }
 
     // ---- updateTemperature!, updateVelocity!, updatePosition!
@@ -352,8 +476,8 @@ __global__ void __launch_bounds__(128) k_momentum_fp64(const SceneDev* __restric
     ((V*)nx.x)[i] = xo;
     ((V*)nx.v)[i] = vo;
     if (SHEP) {  // the particle's own W(0) term, then the Shepard quotient
-        sw += S.k0 * m_i / rho_i;
-        sws += S.k0 * m_i / rho_i * rho_i;
+        const double sw = lane_sum(sums + (kSums - 2) * kCoopLanes * kCoopStride) + S.k0 * m_i / rho_i;
+        const double sws = lane_sum(sums + (kSums - 1) * kCoopLanes * kCoopStride) + S.k0 * m_i;
         nx.rho[i] = sws / sw;
     } else {
         nx.rho[i] = rho_i;
@@ -386,18 +510,20 @@ __global__ void __launch_bounds__(128) k_momentum_fp64(const SceneDev* __restric
 namespace {
 template <int DIM, int KK>
 void launch_k4(const LaunchCtx& L) {
-    const int grid = (L.cap + 127) / 128;
-    k_continuity_fp64<DIM, KK><<<grid, 128, 0, L.stream>>>(L.scenes, L.st, L.sc, L.cap, L.bf);
+    const int np = coop_particles(L.cap);
+    launch_dep(k_continuity_fp64<DIM, KK>, (L.cap + np - 1) / np, np * kCoopLanes, L.stream, L.scenes, L.st, L.sc, L.cap,
+               L.bf);
 }
 template <int DIM, int KK, int MODE>
 void launch_k5(const LaunchCtx& L) {
-    const int grid = (L.cap + 127) / 128;
+    const int np = coop_particles(L.cap);
+    const int grid = (L.cap + np - 1) / np;
     if (L.shepard)
-        k_momentum_fp64<DIM, KK, MODE, true><<<grid, 128, 0, L.stream>>>(L.scenes, L.st, L.nx, L.wl, L.sc, L.cap,
-                                                                          L.bf, L.bs, L.br, L.force_reinit);
+        launch_dep(k_momentum_fp64<DIM, KK, MODE, true>, grid, np * kCoopLanes, L.stream, L.scenes, L.st, L.nx, L.wl,
+                   L.sc, L.cap, L.bf, L.bs, L.br, L.force_reinit);
     else
-        k_momentum_fp64<DIM, KK, MODE, false><<<grid, 128, 0, L.stream>>>(L.scenes, L.st, L.nx, L.wl, L.sc, L.cap,
-                                                                           L.bf, L.bs, L.br, L.skip_reinit);
+        launch_dep(k_momentum_fp64<DIM, KK, MODE, false>, grid, np * kCoopLanes, L.stream, L.scenes, L.st, L.nx, L.wl,
+                   L.sc, L.cap, L.bf, L.bs, L.br, L.skip_reinit);
 }
 
 template <int DIM>

@@ -12,8 +12,7 @@
 //   4. place: rank = #ids in the cell smaller than mine -> destination start[key]+rank,
 //      copy every field there (deterministic: the order is (cell, id) whatever the
 //      arrival order was)
-#include "sph_physics.cuh"
-#include "sph_kernels.h"
+#include "sph_coop.cuh"
 
 namespace sph {
 
@@ -309,6 +308,13 @@ __global__ void k_place(const SceneDev* __restrict__ scenes, SortedState src, Ne
         dst.T[d] = T;
         dst.kappa[d] = kap;
         dst.cp[d] = cpv;
+    }
+    if (!SHADOW) {  // the FP64 gathers' cell and selection position
+        const SceneDev& S = scenes[scn];
+        int32_t c[3];
+        decode_cell(key, S, c);
+        dst.cell[d] = key;
+        dst.fa[d] = select_pos<DIM>(x, S, c);
     }
     if (SHADOW) {  // FP32 shadows: position relative to the origin of the particle's cell
         const SceneDev& S = scenes[scn];
