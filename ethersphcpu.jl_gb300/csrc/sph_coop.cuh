@@ -8,12 +8,19 @@
 //     coop_select), packing them into a list in shared memory; then each lane takes every
 //     kCoopLanes-th entry of the list, so the FP64 pair terms run on full warps and no
 //     rejected candidate costs an FP64 instruction.
-//   * a particle's sums do not depend on the batch, the block size or the other particles
-//     of its warp: where a scene at rest cancels large terms (pressure and wall forces) the
+//   * each of an SM's four schedulers has its own FP64 unit, which one warp can keep busy:
+//     the work has to be even over 608 of them.  The grid is what the SMs hold at once, and
+//     its warps draw the scene's particles from a queue, four at a time; after eight draws a
+//     warp updates its 32 particles, one a lane.  (Warps with a fixed share of 32 particles
+//     left the FP64 units idle for a third of the time, shares of 8 ran the update on a
+//     quarter of a warp.)  No warp waits for another.
+//   * a particle's sums do not depend on the batch, the warp or its other particles: where a scene at rest cancels large terms (pressure and wall forces) the
 //     terms are rounded and added in the reference's own order (pair_kernel, add_terms);
 //     the other sums are taken by lane, lane t entries t, t + 8, ..., and the lanes' sums
 //     added in one fixed order.
 #pragma once
+
+#include <algorithm>
 
 #include "sph_physics.cuh"
 #include "sph_kernels.h"
@@ -21,13 +28,11 @@
 namespace sph {
 
 constexpr int kCoopLanes = 8;        // lanes per particle (the 2 m + 1 <= 7 rows of a plane fit them)
-constexpr int kCoopMaxParticles = 32;  // particles of the largest block (256 threads)
+constexpr int kCoopGroups = 32 / kCoopLanes;  // particles a warp works on at a time
 // Entries of a particle's list: r_cut = 3 dx has about 28 (2D) / 112 (3D) neighbours; a
 // particle with more runs its pair terms in several passes (coop_select).
 template <int DIM> constexpr int kCoopList = DIM == 2 ? 64 : 144;
-// Row lengths in shared memory, in 8-byte words: partial sums (a particle's lanes fall on
-// different banks) and pair terms (one a lane).
-constexpr int kCoopStride = kCoopMaxParticles + 4;
+// Row length of the pair terms in shared memory (8-byte words; one term a lane).
 constexpr int kTermStride = 33;
 
 // ---------------------------------------------------------------- FP64 building blocks
@@ -82,6 +87,16 @@ __device__ __forceinline__ double sqrt_rn(double a, double& inv) {
 __device__ __forceinline__ bool sqrt_rn_range(double a) {
     return ((unsigned)__double2hiint(a) >> 20) - 123u < 1800u;
 }
+// |a| in [2^-300, 2^300] (a^2 and quotients of ordinary values by it stay normal numbers)
+__device__ __forceinline__ bool rcp_rn_range(double a) {
+    return ((unsigned)__double2hiint(a) >> 20 & 0x7ffu) - 723u < 600u;
+}
+
+// 1 / a rounded to nearest, for |a| in [2^-900, 2^900].
+__device__ __forceinline__ double rcp_rn(double a) {
+    const double y = rcp3(a);
+    return fma(fma(-a, y, 1.0), y, y);
+}
 
 // a / b rounded to nearest, y = 1 / b rounded to nearest (the same residual correction).
 __device__ __forceinline__ double div_rn(double a, double b, double y) {
@@ -92,7 +107,7 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
 // max(a, 0) on the sign bit (integer work)
 __device__ __forceinline__ double relu(double a) { return __double2hiint(a) < 0 ? 0.0 : a; }
 
-// x^4, x^5, x^6 as jl_powi rounds them (finite x).
+// x^4 .. x^7 as jl_powi rounds them (finite x).
 template <int N>
 __device__ __forceinline__ double powi_fixed(double x) {
     const double h = x * x, l = fma(x, x, -h);
@@ -100,7 +115,9 @@ __device__ __forceinline__ double powi_fixed(double x) {
     const double ll = fma(h, h, -hh) + h * 2.0 * l;
     if (N == 4) return hh + ll;
     if (N == 5) return fma(hh, x, x * ll);
-    return fma(hh, h, fma(h, ll, hh * l));
+    if (N == 6) return fma(hh, h, fma(h, ll, hh * l));
+    const double c = h * x, cl = fma(h, x, -c) + x * l;  // x^3
+    return fma(hh, c, fma(c, ll, hh * cl));
 }
 
 // ---------------------------------------------------------------- kernels
@@ -283,38 +300,49 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const int32_t* __
         const bool wraps = __any_sync(full, l2 != 0);
         const int most = (int)__reduce_max_sync(full, (unsigned)total);
         const int rounds = dz == planes ? max(most, 1) : most;  // the last round runs the pairs
-        for (int t0 = 0; t0 < rounds; t0 += kCoopLanes) {
-            const int t = t0 + lane;
-            int r = 0;
+        // two rounds at a time: both candidates' positions are loaded before the first is tested
+        for (int t0 = 0; t0 < rounds; t0 += 2 * kCoopLanes) {
+            int j[2];
+            float dyf[2];
+            float4 p[2];
 #pragma unroll
-            for (int k = 0; k < 6; ++k) r += t >= ends[k];
-            int j = t - __shfl_sync(full, first, r, kCoopLanes);  // place in the row
-            const int jb = __shfl_sync(full, b, r, kCoopLanes);
-            if (wraps) {
-                const int n1 = __shfl_sync(full, l1, r, kCoopLanes), jb2 = __shfl_sync(full, b2, r, kCoopLanes);
-                j = j < n1 ? jb + j : jb2 + (j - n1);
-            } else {
-                j += jb;
+            for (int h = 0; h < 2; ++h) {
+                const int t = t0 + h * kCoopLanes + lane;
+                int r = 0;
+#pragma unroll
+                for (int k = 0; k < 6; ++k) r += t >= ends[k];
+                int q = t - __shfl_sync(full, first, r, kCoopLanes);  // place in the row
+                const int jb = __shfl_sync(full, b, r, kCoopLanes);
+                if (wraps) {
+                    const int n1 = __shfl_sync(full, l1, r, kCoopLanes), jb2 = __shfl_sync(full, b2, r, kCoopLanes);
+                    q = q < n1 ? jb + q : jb2 + (q - n1);
+                } else {
+                    q += jb;
+                }
+                dyf[h] = (float)(r - 3);
+                j[h] = t < total ? q : -1;
+                p[h] = me;
+                if (t < total) p[h] = __ldg(pos + q);
             }
-            bool take = t < total;
-            if (take) {
-                const float4 p = __ldg(pos + j);
-                float cx = p.w - me.w;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                float cx = p[h].w - me.w;
                 if (S.periodic_x) cx = cx > 0.5f * nx ? cx - nx : (cx < -0.5f * nx ? cx + nx : cx);
-                const float rx = (cx + (p.x - me.x)) * ex;
-                const float ry = ((float)(r - 3) + (p.y - me.y)) * ey;
+                const float rx = (cx + (p[h].x - me.x)) * ex;
+                const float ry = (dyf[h] + (p[h].y - me.y)) * ey;
                 float d2 = rx * rx + ry * ry;
                 if (DIM == 3) {
-                    const float rz = ((float)dz + (p.z - me.z)) * ez;
+                    const float rz = ((float)dz + (p[h].z - me.z)) * ez;
                     d2 += rz * rz;
                 }
-                take = j != self && (wide ? within(j) : d2 <= r2);
+                bool take = j[h] >= 0 && j[h] != self;
+                if (take) take = wide ? within(j[h]) : d2 <= r2;
+                const unsigned hit = (__ballot_sync(full, take) >> shift) & 0xffu;
+                if (take) list[cnt + __popc(hit & below)] = j[h];
+                cnt += __popc(hit);
             }
-            const unsigned hit = (__ballot_sync(full, take) >> shift) & 0xffu;
-            if (take) list[cnt + __popc(hit & below)] = j;
-            cnt += __popc(hit);
-            const bool last = dz == planes && t0 + kCoopLanes >= rounds;
-            if (last || __any_sync(full, cnt > CAP - kCoopLanes)) {
+            const bool last = dz == planes && t0 + 2 * kCoopLanes >= rounds;
+            if (last || __any_sync(full, cnt > CAP - 2 * kCoopLanes)) {
                 __syncwarp(full);
                 pairs(first_entry, cnt);
                 __syncwarp(full);
@@ -336,14 +364,66 @@ __device__ __forceinline__ void add_terms(const double* terms, int lane, int shi
             for (int s = 0; s < kTerms; ++s) sum += terms[(s * DIM + lane) * kTermStride + shift + e];
 }
 
-// Particles of a block (blockDim.x / kCoopLanes) for n particles.  Large blocks run the
-// per-particle epilogue (about 70 FP64 instructions) on full warps; small ones spread a
-// small scene over the SMs.
-inline int coop_particles(int64_t n) {
-    const int64_t sms = 152;
-    if (n >= 6 * sms * 32) return 32;
-    if (n >= 4 * sms * 16) return 16;
-    return 8;
+// Sum of v over the lanes of a particle, the same tree and bits in every lane.
+__device__ __forceinline__ double coop_sum(double v) {
+#pragma unroll
+    for (int o = 1; o < kCoopLanes; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+// The grid: two blocks of eight warps on each of the 152 SMs, where a scene has 16 fours or
+// more for each of those warps or no more than one; in between one block of six to eight
+// warps an SM (a warp with two or three draws would run its update on few lanes, and the
+// 16 warps' second draws would be uneven).  A lid-driven cavity of 10,201 particles: K4 36
+// us with 16 warps an SM, 27 us with 6; K5 98 and 86 us.
+constexpr int kCoopThreads = 256;
+constexpr int kCoopBlocks = 2;
+struct CoopShape {
+    int grid, threads;
+};
+inline CoopShape coop_shape(int64_t n) {
+    const int64_t sms = 152, fours = std::max<int64_t>(1, (n + kCoopGroups - 1) / kCoopGroups);
+    if (fours <= sms * 16 || n >= sms * 8 * 32)
+        return {(int)std::min(kCoopBlocks * sms, fours), kCoopThreads};
+    return {(int)sms, (int)(32 * std::max<int64_t>(6, n / (32 * sms)))};
+}
+
+// A warp's part of n particles: body(i, p, on) for its group's particle i (clamped to a
+// valid one with on = false past the end), p its place among the warp's next 32; update(i)
+// one lane a particle after each 32 and at the end.  queue[0]: draws beyond every warp's
+// first, queue[1]: blocks that are done (the last one leaves both at 0 for the next launch).
+template <typename Body, typename Update>
+__device__ __forceinline__ void coop_turns(int n, int32_t* queue, Body&& body, Update&& update) {
+    const unsigned full = 0xffffffffu;
+    const int fours = (n + kCoopGroups - 1) / kCoopGroups;
+    const int W = gridDim.x * (blockDim.x / 32);
+    const int lane = threadIdx.x & 31, g = lane / kCoopLanes;
+    int next = threadIdx.x / 32 * gridDim.x + blockIdx.x;  // the first draw
+    while (next < fours) {
+        int mine = fours;  // lane k: the k-th four of this set
+        int k = 0;
+#pragma unroll 1
+        for (; k < kCoopLanes && next < fours; ++k) {
+            if (lane == k) mine = next;
+            const int i = next * kCoopGroups + g;
+            int drawn = 0;
+            if (lane == 0) drawn = atomicAdd(queue, 1);
+            body(min(i, n - 1), k * kCoopGroups + g, i < n);
+            next = W + __shfl_sync(full, drawn, 0);
+        }
+        __syncwarp();
+        const int i = __shfl_sync(full, mine, lane / kCoopGroups) * kCoopGroups + lane % kCoopGroups;
+        if (i < n) update(i);
+        __syncwarp();
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        if (atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
+            queue[0] = 0;
+            queue[1] = 0;
+        }
+    }
 }
 
 }  // namespace sph

@@ -192,6 +192,7 @@ struct SortScratch {
     int32_t* block_sums;
     int32_t* n_live;    // device scalar: live particles after the last sort
     int32_t* status;    // device scalar: status bits
+    int32_t* queue;     // draws and finished blocks of a cooperative gather (coop_turns), both 0 between launches
     int64_t* scene_step;  // per scene: number of the step being run
     // non-null in a step whose scan runs over 1,024-cell tiles: the momentum epilogue adds
     // each particle's arrival to its tile's sum here (the scan then skips its tile pass)

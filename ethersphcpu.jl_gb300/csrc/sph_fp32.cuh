@@ -87,11 +87,6 @@ __device__ __forceinline__ void group_combine(Kahan& k, unsigned mask) {
     }
 }
 
-// Non-finite test on the exponent bits (integer work instead of FP64 compares).
-__device__ __forceinline__ bool bits_finite(double x) {
-    return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
-}
-
 template <int TPP>
 __device__ __forceinline__ double group_sum(double v, unsigned mask) {
 #pragma unroll

@@ -14,9 +14,9 @@
 //    re-initialisation are one kernel (FluidWallSolve.jl:64-72).
 //
 // Eight lanes share one fluid particle (sph_coop.cuh): FP32 selection of its neighbours
-// into shared memory, FP64 pair terms over that list, and one thread that updates the
+// into shared memory, FP64 pair terms over that list, and one lane that updates the
 // particle.  No atomics on the physics, a fixed order of every sum: results are
-// deterministic and do not depend on the batch or the block size.
+// deterministic and do not depend on the batch.
 //
 // What bounds them: FP64 instructions (2 lanes a SM and cycle).
 //   * K4 and the viscosity and heat terms of K5 are factored so that a pair divides once or
@@ -33,13 +33,6 @@ namespace sph {
 
 // Solve variants: which wall terms and which body force.
 enum { kModeFluidWall = 0, kModeWallPressure = 1, kModeThermal = 2, kModeBuffers = 3 };
-
-// Sum of a particle's partial sums (one per lane) in a fixed tree order.
-__device__ __forceinline__ double lane_sum(const double* part) {
-    const double a = (part[0] + part[kCoopStride]) + (part[2 * kCoopStride] + part[3 * kCoopStride]);
-    const double b = (part[4 * kCoopStride] + part[5 * kCoopStride]) + (part[6 * kCoopStride] + part[7 * kCoopStride]);
-    return a + b;
-}
 
 // Geometry of the pair (i, j): r_vec and q^2 = |r_vec|^2 / h^2.
 template <int DIM, typename V>
@@ -73,37 +66,44 @@ __device__ __forceinline__ bool within_cut(const V& xi, const V& xj, const Scene
 }
 
 template <int DIM, int KK>
-__global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
+__global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
     k_continuity_fp64(const SceneDev* __restrict__ scenes, SortedState st, SortScratch sc, int32_t cap, BufferState bf) {
     pdl_wait();
     using V = typename VecT<DIM>::T;
-    __shared__ int32_t lists[kCoopMaxParticles * kCoopList<DIM>];
-    __shared__ double part[kCoopLanes * kCoopStride];
-    const int g = threadIdx.x / kCoopLanes, lane = threadIdx.x % kCoopLanes;
-    const int i0 = blockIdx.x * (blockDim.x / kCoopLanes);
-    const int n = min(cap, *sc.n_live);
-    if (i0 >= n) return;  // the whole block
+    constexpr int kWarps = kCoopThreads / 32;
+    __shared__ int32_t lists[kWarps * kCoopGroups * kCoopList<DIM>];
+    __shared__ double drho_all[kCoopThreads];
+    const int lane = threadIdx.x % kCoopLanes;
     const V* __restrict__ x = (const V*)st.x;
     const V* __restrict__ v = (const V*)st.v;
     const double* __restrict__ m = st.m;
-    {
-        const int i = min(i0 + g, n - 1);
+    int32_t* list = lists + threadIdx.x / kCoopLanes * kCoopList<DIM>;
+    double* drhos = drho_all + (threadIdx.x & ~31);
+    auto gather = [&](int i, int place, bool valid) {
         const SceneDev& S = scenes[st.scene[i]];
-        const bool on = i0 + g < n && scene_runs(S, sc.scene_step[st.scene[i]]);
+        const bool on = valid && scene_runs(S, sc.scene_step[st.scene[i]]);
         const V xi = x[i];
         const V vi = v[i];
         int32_t c[3];
         decode_cell(st.cell[i], S, c);
-        int32_t* list = lists + g * kCoopList<DIM>;
         double drho = 0.0;
         coop_select<DIM>(
             S, sc.start, st.fa, c, st.fa[i], i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
             [&](int first, int cnt) {
-                for (int k = (lane - first) & (kCoopLanes - 1); k < cnt; k += kCoopLanes) {
-                    const int j = list[k];
-                    const V xj = x[j];
-                    const V vj = v[j];
-                    const double m_j = m[j];
+                int k = (lane - first) & (kCoopLanes - 1);
+                if (k >= cnt) return;
+                V xn = x[list[k]], vn = v[list[k]];
+                double mn = m[list[k]];
+                for (; k < cnt; k += kCoopLanes) {
+                    const V xj = xn;
+                    const V vj = vn;
+                    const double m_j = mn;
+                    if (k + kCoopLanes < cnt) {  // the next pair's data
+                        const int j = list[k + kCoopLanes];
+                        xn = x[j];
+                        vn = v[j];
+                        mn = m[j];
+                    }
                     double rv[DIM], vv[DIM];
                     const double q2 = pair_q2<DIM>(xi, xj, S, rv);
                     if (!inside_cut<DIM, KK>(rv, q2, S)) continue;
@@ -125,26 +125,42 @@ __global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
                 }
             });
         }
-        part[lane * kCoopStride + g] = drho;
-    }
-    __syncthreads();
-    // the update, one thread a particle
-    const int i = i0 + threadIdx.x;
-    if (threadIdx.x >= blockDim.x / kCoopLanes || i >= n) return;
-    const SceneDev& S = scenes[st.scene[i]];
-    if (!scene_runs(S, sc.scene_step[st.scene[i]])) return;
-    const double drho = lane_sum(part + threadIdx.x);
-    const double m_i = m[i];
-    double rho = st.rho[i];
-    rho += drho * S.dt;  // written to rhoc, so the kernel can be re-run on the same input
-    const double rr = rho / S.rho0;
-    const double p = S.b * (jl_powi(rr, S.gamma) - 1.0) + S.p0;
-    const double cs = S.c0 * sqrt(jl_powi(rr, S.gamma - 1));
-    st.rhoc[i] = rho;
-    st.p[i] = p;
-    st.c[i] = cs;
-    st.P[i] = p / (rho * rho);
-    st.vol[i] = m_i / rho;
+        drho = coop_sum(drho);
+        if (lane == 0) drhos[place] = drho;
+    };
+    auto update = [&](int i) {
+        const SceneDev& S = scenes[st.scene[i]];
+        if (!scene_runs(S, sc.scene_step[st.scene[i]])) return;
+        const double drho = drhos[threadIdx.x & 31];
+        const double m_i = m[i];
+        double rho = st.rho[i];
+        rho += drho * S.dt;  // written to rhoc, so the kernel can be re-run on the same input
+        // updatePressure! (UpdatePressure.jl:8-16), every operation rounded as written there
+        const bool ordinary = rcp_rn_range(rho) && rho > 0.0;
+        const double rr = ordinary ? div_rn(rho, S.rho0, S.inv_rho0) : rho / S.rho0;
+        double pw, cw;  // rr^gamma, rr^(gamma - 1)
+        if (S.gamma == 7 && ordinary) {
+            pw = powi_fixed<7>(rr);
+            cw = powi_fixed<6>(rr);
+        } else {
+            pw = jl_powi(rr, S.gamma);
+            cw = jl_powi(rr, S.gamma - 1);
+        }
+        double inv;
+        const double p = S.b * (pw - 1.0) + S.p0;
+        st.rhoc[i] = rho;
+        st.p[i] = p;
+        st.c[i] = S.c0 * (sqrt_rn_range(cw) ? sqrt_rn(cw, inv) : sqrt(cw));
+        if (ordinary) {
+            const double r2 = rho * rho;
+            st.P[i] = div_rn(p, r2, rcp_rn(r2));
+            st.vol[i] = div_rn(m_i, rho, rcp_rn(rho));
+        } else {
+            st.P[i] = p / (rho * rho);
+            st.vol[i] = m_i / rho;
+        }
+    };
+    coop_turns(min(cap, *sc.n_live), sc.queue, gather, update);
 }
 
 // SHEP: the momentum gather of density re-initialisation steps, for the particles of the
@@ -152,21 +168,21 @@ __global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
 // `sel` set leaves those particles to the SHEP launch of the same step (a batch whose
 // scenes re-initialise at different steps runs both).
 template <int DIM, int KK, int MODE, bool SHEP>
-__global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
+__global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
     k_momentum_fp64(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl, SortScratch sc,
                     int32_t cap, BufferState bf, BufferScratch bs, BufferRules br, int sel) {
     pdl_wait();
     using V = typename VecT<DIM>::T;
     constexpr bool HEAT = MODE == kModeThermal;
     constexpr int kSums = (HEAT ? 2 : 0) + (SHEP ? 2 : 0);  // sums taken by lane
-    __shared__ int32_t lists[kCoopMaxParticles * kCoopList<DIM>];
-    __shared__ double terms_all[kCoopMaxParticles * kCoopLanes / 32 * 3 * DIM * kTermStride];
-    __shared__ double part[(kSums ? kSums : 1) * kCoopLanes * kCoopStride];
-    __shared__ double dv_all[DIM * kCoopMaxParticles];
-    const int g = threadIdx.x / kCoopLanes, lane = threadIdx.x % kCoopLanes;
-    const int i0 = blockIdx.x * (blockDim.x / kCoopLanes);
-    const int n = min(cap, *sc.n_live);
-    if (i0 >= n) return;  // the whole block
+    constexpr int kWarps = kCoopThreads / 32;
+    __shared__ int32_t lists[kWarps * kCoopGroups * kCoopList<DIM>];
+    __shared__ double terms_all[kWarps * 3 * DIM * kTermStride];
+    __shared__ double vecs_all[kWarps * DIM * 32], sums_all[kWarps * (kSums ? kSums : 1) * 32];
+    const int warp = threadIdx.x / 32, lane = threadIdx.x % kCoopLanes;
+    double* terms = terms_all + warp * 3 * DIM * kTermStride;
+    double* vecs = vecs_all + warp * DIM * 32;
+    double* sums = sums_all + warp * (kSums ? kSums : 1) * 32;
     const V* __restrict__ x = (const V*)st.x;
     const V* __restrict__ v = (const V*)st.v;
     auto takes = [&](const SceneDev& S, int64_t step) {  // the particle's sums are formed by this launch
@@ -174,13 +190,12 @@ __global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
         if (SHEP) return runs && (sel || is_step(step, S.reinit_interval));
         return runs && !(sel && is_step(step, S.reinit_interval));
     };
-    {
-        const int i = min(i0 + g, n - 1);
+    const int shift = (threadIdx.x & 31) - lane;
+    double* mine = terms + (threadIdx.x & 31);  // this lane's place in a row of terms
+    int32_t* list = lists + threadIdx.x / kCoopLanes * kCoopList<DIM>;
+    auto gather = [&](int i, int place, bool valid) {
         const SceneDev& S = scenes[st.scene[i]];
-        const bool on = i0 + g < n && takes(S, sc.scene_step[st.scene[i]]);
-        const int shift = (threadIdx.x & 31) & ~(kCoopLanes - 1);
-        double* terms = terms_all + threadIdx.x / 32 * (3 * DIM * kTermStride);
-        double* mine = terms + (threadIdx.x & 31);  // this lane's place in a row of terms
+        const bool on = valid && takes(S, sc.scene_step[st.scene[i]]);
         const V xi = x[i];
         const V vi = v[i];
         const double rho_i = st.rhoc[i];
@@ -196,7 +211,6 @@ __global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
         int32_t c[3];
         decode_cell(st.cell[i], S, c);
         const float4 me = st.fa[i];
-        int32_t* list = lists + g * kCoopList<DIM>;
         double dv = 0.0;  // lane d < DIM: component d of the acceleration
         double aT = 0.0, wT = 0.0, sw = 0.0, sws = 0.0;
 
@@ -316,7 +330,8 @@ __global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
         // ---- walls: wallForce! (+ background pressureForce!) + viscosityForce! (+ heat),
         // only where a wall cell is within reach of the particle's cell
         const bool walls = on && wl.n > 0 && wl.near[st.cell[i]];
-        if (__any_sync(0xffffffffu, walls)) {
+        const bool near = __any_sync(0xffffffffu, walls);
+        if (near) {
             const V* __restrict__ wx = (const V*)wl.x;
             const V* __restrict__ wn = (const V*)wl.nrm;
             const V* __restrict__ wv = (const V*)wl.v;
@@ -393,136 +408,143 @@ __global__ void __launch_bounds__(kCoopLanes * kCoopMaxParticles)
                     });
                 });
         }
-        if (lane < DIM) dv_all[lane * kCoopMaxParticles + g] = dv;
-        double* sums = part + lane * kCoopStride + g;
+        if (lane < DIM) vecs[lane * 32 + place] = dv;
         if (HEAT) {
-            sums[0] = aT;
-            sums[kCoopLanes * kCoopStride] = wT;
+            aT = coop_sum(aT);
+            if (near) wT = coop_sum(wT);
         }
         if (SHEP) {
-            sums[(kSums - 2) * kCoopLanes * kCoopStride] = sw;
-            sums[(kSums - 1) * kCoopLanes * kCoopStride] = sws;
+            sw = coop_sum(sw);
+            sws = coop_sum(sws);
         }
-    }
-    __syncthreads();
+        if (lane == 0) {
+            if (HEAT) {
+                sums[place] = aT;
+                sums[32 + place] = wT;
+            }
+            if constexpr (SHEP) {
+                sums[(kSums - 2) * 32 + place] = sw;
+                sums[(kSums - 1) * 32 + place] = sws;
+            }
+        }
+    };
 
-    // ---- the update, one thread a particle
-    const int i = i0 + threadIdx.x;
-    if (threadIdx.x >= blockDim.x / kCoopLanes || i >= n) return;
-    const SceneDev& S = scenes[st.scene[i]];
-    const int64_t step = sc.scene_step[st.scene[i]];
-    if (!takes(S, step)) {
-        if (!SHEP && !scene_runs(S, step)) carry_frozen<DIM>(i, S, st, nx, sc);
-        return;
-    }
-    const V xi = x[i];
-    const V vi = v[i];
-    const double rho_i = st.rhoc[i];
-    const double m_i = st.m[i];
-    const double* sums = part + threadIdx.x;
-    double dv[DIM];
+    // ---- the update, one lane a particle
+    auto update = [&](int i) {
+        const SceneDev& S = scenes[st.scene[i]];
+        const int64_t step = sc.scene_step[st.scene[i]];
+        if (!takes(S, step)) {
+            if (!SHEP && !scene_runs(S, step)) carry_frozen<DIM>(i, S, st, nx, sc);
+            return;
+        }
+        const V xi = x[i];
+        const V vi = v[i];
+        const double rho_i = st.rhoc[i];
+        const double m_i = st.m[i];
+        double dv[DIM];
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) dv[k] = dv_all[k * kCoopMaxParticles + threadIdx.x];
-    double T_i = 0.0, dT = 0.0;
-    if (HEAT) {
-        T_i = st.T[i];
-        const double fluid = lane_sum(sums), wall = lane_sum(sums + kCoopLanes * kCoopStride);
-        dT = (4.0 * st.kappa[i] / st.cp[i] * fluid + m_i * S.inv_cp_d / S.rho0 * wall) / rho_i;
-    }
+        for (int k = 0; k < DIM; ++k) dv[k] = vecs[k * 32 + (threadIdx.x & 31)];
+        double T_i = 0.0, dT = 0.0;
+        if (HEAT) {
+            T_i = st.T[i];
+            const double fluid = sums[threadIdx.x & 31], wall = sums[32 + (threadIdx.x & 31)];
+            const double cp_i = st.cp[i];
+        dT = (4.0 * st.kappa[i] * fluid + S.inv_cp_d * S.inv_rho0 * m_i * cp_i * wall) / (cp_i * rho_i);
+        }
 
-    // ---- updateTemperature!, updateVelocity!, updatePosition!
-    const double dt = S.dt;
-    double body[DIM];
-    if (MODE == kModeThermal) {
-        T_i += dt * dT;
+        // ---- updateTemperature!, updateVelocity!, updatePosition!
+        const double dt = S.dt;
+        double body[DIM];
+        if (MODE == kModeThermal) {
+            T_i += dt * dT;
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) body[k] = S.bous[k] * (T_i - S.t0);
-        nx.T[i] = T_i;
-    } else {
-        if (nx.T) nx.T[i] = st.T[i];  // thermal particles in a solve without heat terms
+            for (int k = 0; k < DIM; ++k) body[k] = S.bous[k] * (T_i - S.t0);
+            nx.T[i] = T_i;
+        } else {
+            if (nx.T) nx.T[i] = st.T[i];  // thermal particles in a solve without heat terms
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) body[k] = S.g[k];
-    }
-    double vn[DIM], xn[DIM];
-    vn[0] = vi.x;
-    vn[1] = vi.y;
-    xn[0] = xi.x;
-    xn[1] = xi.y;
-    if (DIM == 3) {
-        vn[DIM - 1] = comp(vi, DIM - 1);
-        xn[DIM - 1] = comp(xi, DIM - 1);
-    }
+            for (int k = 0; k < DIM; ++k) body[k] = S.g[k];
+        }
+        double vn[DIM], xn[DIM];
+        vn[0] = vi.x;
+        vn[1] = vi.y;
+        xn[0] = xi.x;
+        xn[1] = xi.y;
+        if (DIM == 3) {
+            vn[DIM - 1] = comp(vi, DIM - 1);
+            xn[DIM - 1] = comp(xi, DIM - 1);
+        }
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) vn[k] += body[k] * dt;
+        for (int k = 0; k < DIM; ++k) vn[k] += body[k] * dt;
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) vn[k] += dv[k] * dt;
+        for (int k = 0; k < DIM; ++k) vn[k] += dv[k] * dt;
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) xn[k] += vn[k] * dt - dv[k] * S.dtdt / 2.0;
-    if (S.periodic_x) {
-        if (xn[0] >= S.wrap_hi) xn[0] -= S.period;
-        else if (xn[0] < S.lo[0]) xn[0] += S.period;
-    }
-    V xo, vo;
-    xo.x = xn[0];
-    xo.y = xn[1];
-    vo.x = vn[0];
-    vo.y = vn[1];
-    if constexpr (DIM == 3) {
-        xo.z = xn[2];
-        xo.w = 0.0;
-        vo.z = vn[2];
-        vo.w = 0.0;
-    }
-    ((V*)nx.x)[i] = xo;
-    ((V*)nx.v)[i] = vo;
-    if (SHEP) {  // the particle's own W(0) term, then the Shepard quotient
-        const double sw = lane_sum(sums + (kSums - 2) * kCoopLanes * kCoopStride) + S.k0 * m_i / rho_i;
-        const double sws = lane_sum(sums + (kSums - 1) * kCoopLanes * kCoopStride) + S.k0 * m_i;
-        nx.rho[i] = sws / sw;
-    } else {
-        nx.rho[i] = rho_i;
-    }
+        for (int k = 0; k < DIM; ++k) xn[k] += vn[k] * dt - dv[k] * S.dtdt / 2.0;
+        if (S.periodic_x) {
+            if (xn[0] >= S.wrap_hi) xn[0] -= S.period;
+            else if (xn[0] < S.lo[0]) xn[0] += S.period;
+        }
+        V xo, vo;
+        xo.x = xn[0];
+        xo.y = xn[1];
+        vo.x = vn[0];
+        vo.y = vn[1];
+        if constexpr (DIM == 3) {
+            xo.z = xn[2];
+            xo.w = 0.0;
+            vo.z = vn[2];
+            vo.w = 0.0;
+        }
+        ((V*)nx.x)[i] = xo;
+        ((V*)nx.v)[i] = vo;
+        if constexpr (SHEP) {  // the particle's own W(0) term, then the Shepard quotient
+            const double sw = sums[(kSums - 2) * 32 + (threadIdx.x & 31)] + S.k0 * m_i / rho_i;
+            const double sws = sums[(kSums - 1) * 32 + (threadIdx.x & 31)] + S.k0 * m_i;
+            nx.rho[i] = sws / sw;
+        } else {
+            nx.rho[i] = rho_i;
+        }
 
-    // ---- non-finite state, out-of-domain check, next step's cell hash
-    bool finite = isfinite(rho_i);
+        // ---- non-finite state, out-of-domain check, next step's cell hash
+        bool finite = bits_finite(rho_i);
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) finite &= isfinite(xn[k]) & isfinite(vn[k]);
-    if (!finite && S.nan_check) atomicOr(sc.status, kStatusNonFinite);
-    bool dead = false;
-    if (S.check_enabled && is_step(step, S.check_interval)) {
+        for (int k = 0; k < DIM; ++k) finite &= bits_finite(xn[k]) & bits_finite(vn[k]);
+        if (!finite && S.nan_check) atomicOr(sc.status, kStatusNonFinite);
+        bool dead = false;
+        if (S.check_enabled && is_step(step, S.check_interval)) {
 #pragma unroll
-        for (int k = 0; k < DIM; ++k) dead |= (xn[k] > S.check_hi[k]) | (xn[k] < S.check_lo[k]);
-    }
-    if (dead) {
-        sc.key[i] = kDeadKey;
-    } else if (MODE == kModeBuffers && bs.npend && beyond_plane<DIM>(br.out_n, br.out_d, xn)) {
-        // outlet_out_calculation_domain_check: leaves the fluid, joins the outlet
-        sc.key[i] = kDeadKey;
-        const int32_t k = atomicAdd(bs.npend, 1);
-        if (k < bs.cap) bs.pend[k] = i;
-        else atomicOr(sc.status, kStatusBufferOverflow);
-    } else {
-        cell_arrival(sc, i, cell_key<DIM>(xo, S));
-    }
+            for (int k = 0; k < DIM; ++k) dead |= (xn[k] > S.check_hi[k]) | (xn[k] < S.check_lo[k]);
+        }
+        if (dead) {
+            sc.key[i] = kDeadKey;
+        } else if (MODE == kModeBuffers && bs.npend && beyond_plane<DIM>(br.out_n, br.out_d, xn)) {
+            // outlet_out_calculation_domain_check: leaves the fluid, joins the outlet
+            sc.key[i] = kDeadKey;
+            const int32_t k = atomicAdd(bs.npend, 1);
+            if (k < bs.cap) bs.pend[k] = i;
+            else atomicOr(sc.status, kStatusBufferOverflow);
+        } else {
+            cell_arrival(sc, i, cell_key<DIM>(xo, S));
+        }
+    };
+    coop_turns(min(cap, *sc.n_live), sc.queue, gather, update);
 }
 
 // ---------------------------------------------------------------- launchers
 namespace {
 template <int DIM, int KK>
 void launch_k4(const LaunchCtx& L) {
-    const int np = coop_particles(L.cap);
-    launch_dep(k_continuity_fp64<DIM, KK>, (L.cap + np - 1) / np, np * kCoopLanes, L.stream, L.scenes, L.st, L.sc, L.cap,
-               L.bf);
+    const CoopShape shape = coop_shape(L.cap);
+    launch_dep(k_continuity_fp64<DIM, KK>, shape.grid, shape.threads, L.stream, L.scenes, L.st, L.sc, L.cap, L.bf);
 }
 template <int DIM, int KK, int MODE>
 void launch_k5(const LaunchCtx& L) {
-    const int np = coop_particles(L.cap);
-    const int grid = (L.cap + np - 1) / np;
+    const CoopShape shape = coop_shape(L.cap);
     if (L.shepard)
-        launch_dep(k_momentum_fp64<DIM, KK, MODE, true>, grid, np * kCoopLanes, L.stream, L.scenes, L.st, L.nx, L.wl,
+        launch_dep(k_momentum_fp64<DIM, KK, MODE, true>, shape.grid, shape.threads, L.stream, L.scenes, L.st, L.nx, L.wl,
                    L.sc, L.cap, L.bf, L.bs, L.br, L.force_reinit);
     else
-        launch_dep(k_momentum_fp64<DIM, KK, MODE, false>, grid, np * kCoopLanes, L.stream, L.scenes, L.st, L.nx, L.wl,
+        launch_dep(k_momentum_fp64<DIM, KK, MODE, false>, shape.grid, shape.threads, L.stream, L.scenes, L.st, L.nx, L.wl,
                    L.sc, L.cap, L.bf, L.bs, L.br, L.skip_reinit);
 }
 

@@ -283,6 +283,11 @@ __device__ __forceinline__ int32_t cell_key(const V& x, const SceneDev& S) {
     return S.cell_off + (c[2] * S.n[1] + c[1]) * S.n[0] + c[0];
 }
 
+// Non-finite test on the exponent bits (integer work instead of FP64 compares).
+__device__ __forceinline__ bool bits_finite(double x) {
+    return (__double2hiint(x) & 0x7ff00000) != 0x7ff00000;
+}
+
 __device__ __forceinline__ bool is_step(int64_t step, int64_t interval) {
     return interval > 0 && step % interval == 0;
 }
