@@ -69,10 +69,11 @@ def bytes_per(dim: int, thermal: bool, precision: int) -> tuple[int, int, int]:
     scal = 7 + (3 if thermal else 0)
     per_sorted = 2 * vec + 8 * scal + 8 + 16 + 4 + 8
     if precision == _abi.PRECISION_FP32_COMPENSATED:
-        per_sorted += 2 * 16 + 4
-    particle = 2 * per_sorted + 2 * vec + 8 + (8 if thermal else 0) + 12
+        per_sorted += 2 * 16
+    sums = 2 * (dim + (1 if thermal else 0)) + 2 if precision == _abi.PRECISION_FP32_COMPENSATED else 0
+    particle = 2 * per_sorted + 2 * vec + 8 + (8 if thermal else 0) + 12 + 8 * sums + (4 if sums else 0)
     cell = 4 * 3 + 1
-    wall = 3 * vec + 3 * 8 + 4 + (48 if precision == _abi.PRECISION_FP32_COMPENSATED else 16)
+    wall = 3 * vec + 3 * 8 + 4 + (52 if precision == _abi.PRECISION_FP32_COMPENSATED else 16)
     return particle, cell, wall
 
 

@@ -200,19 +200,17 @@ bool build_scene(const SphParams& p, SceneDev& S, std::string& err) {
     S.sel_inv_ex = (float)(rc / S.cell_d[0]);
 
     for (int a = 0; a < 3; ++a) S.cell_f[a] = (float)S.cell_d[a];
+    for (int a = 0; a < 3; ++a) S.inv_cell_f[a] = (float)S.inv_cell[a];
     S.inv_cell_fx = 1.0f / S.cell_f[0];
-    S.h_f = (float)p.h;
     S.rc2_f = (float)(rc * rc);
     S.rc2_prune = S.rc2_f * 1.00001f;
     S.prune = 1;
     S.hh001_f = (float)S.hh001;
-    S.nu0_f = (float)p.nu_0;
+    S.nu4_f = (float)S.nu4;
+    S.inv_hh_f = (float)S.inv_hh;
     S.P_bg_f = (float)S.P_bg;
     S.kw_a_f = (float)S.kw_a;
-    S.kg_a_f = (float)S.kg_a;
     S.inv_h_f = (float)(1.0 / p.h);
-    S.c0_f = (float)p.c_0;
-    S.rho0_f = (float)p.rho_0;
     S.inv_cp_f = (float)S.inv_cp_d;
     S.inv_rho0 = 1.0 / p.rho_0;
     S.inv_rho0_f = (float)(1.0 / p.rho_0);
@@ -238,6 +236,7 @@ void set_uniform_gap(int kernel, SceneDev& S, bool uniform, double gap0) {
     S.wg = uniform ? host_kernel_w(kernel, S, gap0) : 0.0;
     S.uniform_gap = S.wg > 0.0 ? 1 : 0;
     S.inv_wg = S.uniform_gap ? 1.0 / S.wg : 0.0;
+    S.tens_f = S.uniform_gap ? (float)(0.01 * S.kw_a / S.wg) : 0.f;
 }
 
 int32_t host_cell_key(const SceneDev& S, int dim, const double* x) {
@@ -354,15 +353,15 @@ struct SphHandle {
     int par = 0;
     bool have_fluid = false;
     int64_t steps_done = 0;
-    // FP32 launch shape: lanes per particle for continuity, momentum, Shepard; block size
-    int tune[4] = {1, 1, 1, 128};  // the autotuner's most frequent pick on large 2D and 3D scenes
-    // neighbour list of the FP32 form (momentum lanes code >= SPH_LANES_LIST - 1): grown
-    // on demand to the per-particle grid and the deepest scene (ensure_list)
-    NbrList nl{};
-    // stencil pruning of the FP32 walks (sph_set_stencil_pruning); default on in 3D only:
-    // measured on GB300, it saves 4-8% of a 3D step (25 neighbour rows, corner rows and
-    // cells beyond r_cut skipped) and costs 0-7% in 2D (few cells to skip, per-row bounds)
-    int prune = -1;  // -1: by dimension
+    // launch shape as set (sph_set_launch_shape); lanes: what the autotuner found for the FP32
+    // gathers (LaunchCtx::lanes), whose sums do not depend on it
+    int tune[4] = {1, 1, 1, 128};
+    int lanes = -1;
+    NbrList nl{};          // neighbour list of the FP32 form (ensure_list)
+    bool no_list = false;  // no room for it
+    // stencil pruning of the FP32 gathers (sph_set_stencil_pruning), on by default: the rows
+    // of a particle's stencil are bounded by its eight lanes together
+    int prune = 1;
     std::string err;
     std::vector<SceneRec> scenes;
     RangeAlloc cells, walls;
@@ -451,7 +450,6 @@ cudaError_t alloc_sorted(SphHandle* h, SortedState& s) {
     if (h->precision == SPH_PRECISION_FP32_COMPENSATED) {  // FP32 shadows of the gathers
         if ((e = dalloc(h, &s.fb, n)) != cudaSuccess) return e;
         if ((e = dalloc(h, &s.fc, n)) != cudaSuccess) return e;
-        if ((e = dalloc(h, &s.fd, n)) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
@@ -463,10 +461,6 @@ cudaError_t alloc_sorted(SphHandle* h, SortedState& s) {
 int32_t grid_rows(const SphHandle* h) {
     if (h->has_buffers) return (int32_t)h->cap;
     return (int32_t)std::max<int64_t>(1, std::min<int64_t>(h->cap, h->n_upper));
-}
-
-bool uses_list(const SphHandle* h) {
-    return h->precision == SPH_PRECISION_FP32_COMPENSATED && h->tune[1] >= SPH_LANES_LIST - 1;
 }
 
 // Neighbour-list entries a particle of spacing `gap` needs: the lattice points within
@@ -485,10 +479,11 @@ int32_t list_depth_for(int dim, double rc2, double gap) {
     return (int32_t)std::min<int64_t>(depth, 1024);
 }
 
-// Storage of the neighbour list for the current per-particle grid and scene depths;
-// reallocating drops the captured graphs (they hold its address).
+// Storage of the neighbour list of the FP32 form for the current per-particle grid and scene
+// depths; a larger one replaces it (and the captured graphs, which hold its address).  A
+// device without room for it leaves the momentum gather walking the cells.
 int32_t ensure_list(SphHandle* h) {
-    if (!uses_list(h)) return SPH_OK;
+    if (h->precision != SPH_PRECISION_FP32_COMPENSATED || h->no_list) return SPH_OK;
     int32_t depth = 8;
     for (const SceneRec& R : h->scenes)
         if (R.used) depth = std::max(depth, R.list_depth);
@@ -511,8 +506,8 @@ int32_t ensure_list(SphHandle* h) {
         cudaGetLastError();
         if (h->nl.e) cudaFree(h->nl.e);
         h->nl = NbrList{};
-        return fail(h, SPH_ERR_OOM, "no device memory for the neighbour list (" + std::to_string(stride) + " x " +
-                                        std::to_string(depth) + " entries); use a cell-walk momentum lanes code");
+        h->no_list = true;
+        return SPH_OK;
     }
     h->nl.kmax = depth;
     h->nl.stride = stride;
@@ -541,11 +536,7 @@ LaunchCtx make_ctx(SphHandle* h) {
     L.shepard = 0;
     L.force_reinit = 0;
     L.skip_reinit = 0;
-    L.block = h->tune[3];
-    L.tpp_continuity = h->tune[0];
-    L.tpp_momentum = h->tune[1];
-    L.list_momentum = uses_list(h);
-    if (L.list_momentum) L.tpp_momentum -= SPH_LANES_LIST;
+    L.lanes = h->lanes;
     L.nl = h->nl;
     if (h->has_buffers) {
         L.bf = h->B[h->par];
@@ -732,12 +723,13 @@ int32_t write_scene_walls(SphHandle* h, int s) {
     std::vector<char> bx(nw * vb, 0), bn(nw * vb, 0), bv(nw * vb, 0);
     std::vector<double> bg(nw), bT(nw), bk(nw);
     std::vector<int32_t> bkind(nw);
-    std::vector<float4> fa, fb, fc;
+    std::vector<float4> fa(nw), fb, fc;
+    std::vector<float> fk;
     const bool shadow = h->precision == SPH_PRECISION_FP32_COMPENSATED;
-    fa.resize(nw);
     if (shadow) {
         fb.resize(nw);
         fc.resize(nw);
+        fk.resize(nw);
     }
     for (int64_t q = 0; q < nw; ++q) {
         const int64_t w = order[q];
@@ -752,31 +744,19 @@ int32_t write_scene_walls(SphHandle* h, int s) {
         bkind[q] = R.wkind[w];
         const int32_t k = key[w] - S.cell_off;
         const int32_t cc[3] = {k % S.n[0], (k / S.n[0]) % S.n[1], k / (S.n[0] * S.n[1])};
-        if (!shadow) {  // selection position (select_pos in sph_coop.cuh)
-            float u[3] = {0.f, 0.f, 0.f};
+        float u[3] = {0.f, 0.f, 0.f};  // selection position (select_pos in sph_coop.cuh)
+        for (int a = 0; a < dim; ++a)
+            u[a] = (float)((R.wx[w * dim + a] - S.lo[a]) * S.inv_cell[a] - (double)cc[a]);
+        fa[q] = make_float4(u[0], u[1], u[2], (float)cc[0]);
+        if (shadow) {
+            float nr[3] = {0.f, 0.f, 0.f}, vr[3] = {0.f, 0.f, 0.f};
             for (int a = 0; a < dim; ++a) {
-                const double d = (R.wx[w * dim + a] - S.lo[a]) * S.inv_cell[a] - (double)cc[a];
-                u[a] = (float)std::fmin(std::fmax(d, -1e6), 1e6);
-            }
-            fa[q] = make_float4(u[0], u[1], u[2], (float)cc[0]);
-        } else {  // position relative to the origin of the wall's cell
-            float xr[3] = {0.f, 0.f, 0.f}, nr[3] = {0.f, 0.f, 0.f}, vr[3] = {0.f, 0.f, 0.f};
-            for (int a = 0; a < dim; ++a) {
-                xr[a] = (float)(R.wx[w * dim + a] - (S.lo[a] + (double)cc[a] * S.cell_d[a]));
                 nr[a] = (float)R.wn[w * dim + a];
                 vr[a] = (float)R.wv[w * dim + a];
             }
-            const float g = (float)R.wgap[w], T = (float)R.wT[w], kap = (float)R.wkappa[w];
-            const float thermo = R.wkind[w] == SPH_WALL_THERMOSTATIC ? 1.f : 0.f;
-            if (dim == 2) {
-                fa[q] = make_float4(xr[0], xr[1], nr[0], nr[1]);
-                fb[q] = make_float4(vr[0], vr[1], g, T);
-                fc[q] = make_float4(kap, thermo, 0.f, 0.f);
-            } else {
-                fa[q] = make_float4(xr[0], xr[1], xr[2], g);
-                fb[q] = make_float4(nr[0], nr[1], nr[2], T);
-                fc[q] = make_float4(vr[0], vr[1], vr[2], kap);
-            }
+            fb[q] = make_float4(nr[0], nr[1], nr[2], (float)R.wgap[w]);
+            fc[q] = make_float4(vr[0], vr[1], vr[2], (float)R.wT[w]);
+            fk[q] = (float)R.wkappa[w];
         }
     }
     cudaStream_t st = h->stream;
@@ -793,6 +773,7 @@ int32_t write_scene_walls(SphHandle* h, int s) {
         if (shadow) {
             SPH_CUDA(h, cudaMemcpyAsync(h->W.fb + o, fb.data(), nw * sizeof(float4), cudaMemcpyHostToDevice, st));
             SPH_CUDA(h, cudaMemcpyAsync(h->W.fc + o, fc.data(), nw * sizeof(float4), cudaMemcpyHostToDevice, st));
+            SPH_CUDA(h, cudaMemcpyAsync(h->W.fk + o, fk.data(), nw * sizeof(float), cudaMemcpyHostToDevice, st));
         }
     }
     SPH_CUDA(h, cudaMemcpyAsync(h->W.start + S.cell_off, start.data(), start.size() * 4, cudaMemcpyHostToDevice, st));
@@ -1068,10 +1049,16 @@ int32_t allocate_handle(SphHandle* h, int64_t cells) {
                 {&h->sc.tmp, (size_t)h->cap},        {&h->sc.count, ncell},
                 {&h->sc.start, ncell + 1},           {&h->sc.block_sums, ncell / 1024 + 2},
                 {&h->sc.status, 1},                  {&h->nbuf, 2},
-                {&h->sc.queue, 2},
+                {&h->sc.queue, 2},                   {&h->sc.n_walked, 1},
                 {&h->W.start, ncell + 1},            {&h->W.kind, wc}};
     for (auto& a : ints)
         if ((e = dalloc(h, a.p, a.n)) != cudaSuccess) return cuda_fail(nullptr, e, "scratch");
+    if (h->precision == SPH_PRECISION_FP32_COMPENSATED) {
+        const size_t sums = 2 * (size_t)(h->dim + (h->mode == 2 ? 1 : 0)) + 2;
+        if ((e = dalloc(h, &h->sc.walked, (size_t)h->cap)) != cudaSuccess) return cuda_fail(nullptr, e, "scratch");
+        if ((e = dalloc(h, &h->sc.walk_sums, (size_t)h->cap * sums)) != cudaSuccess)
+            return cuda_fail(nullptr, e, "scratch");
+    }
     if ((e = dalloc(h, &h->W.near, ncell + 1)) != cudaSuccess) return cuda_fail(nullptr, e, "scratch");
     if ((e = dalloc(h, &h->sc.scene_step, (size_t)h->scap)) != cudaSuccess) return cuda_fail(nullptr, e, "steps");
     if ((e = dalloc(h, &h->d_scenes, (size_t)h->scap)) != cudaSuccess) return cuda_fail(nullptr, e, "scenes");
@@ -1085,6 +1072,7 @@ int32_t allocate_handle(SphHandle* h, int64_t cells) {
     if (h->precision == SPH_PRECISION_FP32_COMPENSATED) {
         if ((e = dalloc(h, &h->W.fb, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
         if ((e = dalloc(h, &h->W.fc, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
+        if ((e = dalloc(h, &h->W.fk, wc)) != cudaSuccess) return cuda_fail(nullptr, e, "walls");
     }
     if ((e = dalloc(h, &h->d_stat_partials, 3 * 152)) != cudaSuccess) return cuda_fail(nullptr, e, "stats");
     if ((e = dalloc(h, &h->d_stat_out, 4)) != cudaSuccess) return cuda_fail(nullptr, e, "stats");
@@ -1140,7 +1128,7 @@ int32_t open_scene(SphHandle* h, const SphParams& p, int64_t wall_cap, int64_t f
     S.cell_off = (int32_t)coff;
     S.last_step = last_step;
     S.active = 1;
-    S.prune = h->prune >= 0 ? h->prune : (p.dim == 3 ? 1 : 0);
+    S.prune = h->prune;
     SceneRec& R = h->scenes[s];
     R = SceneRec();
     R.used = true;
@@ -1719,7 +1707,10 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
                 break;
             case SPH_STAGE_SCAN: launch_scan(Lh, 0); break;
             case SPH_STAGE_SORT: launch_place(Lh); break;
-            case SPH_STAGE_CONTINUITY: launch_physics(0, L); break;
+            case SPH_STAGE_CONTINUITY:
+                cudaMemsetAsync(h->sc.n_walked, 0, 4, st);  // continuity appends to the walked particles
+                launch_physics(0, L);
+                break;
             case SPH_STAGE_MOMENTUM: launch_physics(1, L); break;
             case SPH_STAGE_REINIT: launch_physics(1, Lr); break;
         }
@@ -1739,6 +1730,7 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
         }
     }
     // the momentum stage left arrivals in count[]: the next step expects it zeroed
+    SPH_CUDA(h, cudaMemsetAsync(h->sc.n_walked, 0, 4, st));
     SPH_CUDA(h, cudaMemsetAsync(h->sc.count, 0, sizeof(int32_t) * (size_t)h->scan_cells, st));
     // restore p and c (output-only fields) from the copy the placement stage wrote
     const size_t n = (size_t)h->cap;
@@ -1757,13 +1749,7 @@ int32_t sph_autotune(SphHandle* h, int32_t reps, int32_t* out) {
     if (!h->have_fluid) return fail(h, SPH_ERR_STATE, "no fluid uploaded");
     if (h->precision == SPH_PRECISION_FP32_COMPENSATED) {
         cudaStream_t st = h->stream;
-        // storage for the list candidates (kept only when a list shape wins; released
-        // with the handle)
-        const int saved1 = h->tune[1];
-        h->tune[1] = SPH_LANES_LIST + 1;
-        const bool have_list = ensure_list(h) == SPH_OK;
-        h->tune[1] = saved1;
-        if (!have_list) h->err.clear();
+        if (int32_t rc = ensure_list(h); rc != SPH_OK) return rc;
         cudaEvent_t e0, e1;
         SPH_CUDA(h, cudaEventCreate(&e0));
         SPH_CUDA(h, cudaEventCreate(&e1));
@@ -1773,95 +1759,34 @@ int32_t sph_autotune(SphHandle* h, int32_t reps, int32_t* out) {
         // overwrite them, so park them in the idle sorted buffer meanwhile
         SPH_CUDA(h, cudaMemcpyAsync(h->S[par ^ 1].p, h->S[par].p, nbytes, cudaMemcpyDeviceToDevice, st));
         SPH_CUDA(h, cudaMemcpyAsync(h->S[par ^ 1].c, h->S[par].c, nbytes, cudaMemcpyDeviceToDevice, st));
-        const int blocks[3] = {64, 128, 256};
-        // time `reps` launches of one stage at one shape; list: continuity records the
-        // neighbour list / momentum reads it
-        auto trial = [&](int stage, int tpp, int block, bool list) -> float {
+        // lanes sharing a particle, or a thread each: continuity then momentum as in a step
+        auto trial = [&](int lanes) -> float {
             LaunchCtx L = make_ctx(h);
             L.bs.npend = nullptr;  // trial launches mark no particle for the outlet
-            L.block = block;
-            L.tpp_continuity = L.tpp_momentum = tpp;
-            L.list_momentum = list ? 1 : 0;
-            L.nl = h->nl;
-            launch_physics(stage, L);  // warm-up
-            cudaEventRecord(e0, st);
-            for (int r = 0; r < reps; ++r) launch_physics(stage, L);
-            cudaEventRecord(e1, st);
-            cudaEventSynchronize(e1);
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            return ms;
-        };
-        struct Best {
-            float ms = 1e30f;
-            int tpp = 1, block = 128;
-        };
-        auto search = [&](int stage, const int* tpps, int ntpp, bool list) {
-            Best b;
-            for (int q = 0; q < ntpp; ++q)
-                for (int block : blocks) {
-                    if (tpps[q] == -1 && stage == 1 && block > 256) continue;
-                    const float ms = trial(stage, tpps[q], block, list);
-                    if (ms < b.ms) b = Best{ms, tpps[q], block};
-                }
-            return b;
-        };
-        const int walk_tpps[5] = {-1, 1, 2, 4, 8};  // -1: one lane, software-pipelined loop
-        const Best c_walk = search(0, walk_tpps, 5, false);
-        const Best m_walk = search(1, walk_tpps, 5, false);
-        Best c_list, m_list;
-        if (have_list) {
-            const int c_tpps[3] = {-1, 1, 2}, m_tpps[4] = {-1, 1, 2, 4};
-            c_list = search(0, c_tpps, 3, true);
-            // the momentum trials read the list the last continuity trial recorded
-            trial(0, c_list.tpp, c_list.block, true);
-            m_list = search(1, m_tpps, 4, true);
-        }
-        // the cell-walk pair against the list pair, each timed as it runs in a step
-        // (continuity then momentum, at the momentum stage's block size)
-        auto pair_ms = [&](const Best& c, const Best& m, bool list) -> float {
-            LaunchCtx L = make_ctx(h);
-            L.bs.npend = nullptr;
-            L.block = m.block;
-            L.tpp_continuity = c.tpp;
-            L.tpp_momentum = m.tpp;
-            L.list_momentum = list ? 1 : 0;
-            L.nl = h->nl;
-            launch_physics(0, L);
-            launch_physics(1, L);
-            const int n = std::max(reps, 5);
-            cudaEventRecord(e0, st);
-            for (int r = 0; r < n; ++r) {
+            L.lanes = lanes;
+            auto step = [&] {
+                cudaMemsetAsync(h->sc.n_walked, 0, 4, st);
                 launch_physics(0, L);
                 launch_physics(1, L);
-            }
+            };
+            step();  // warm-up
+            cudaEventRecord(e0, st);
+            for (int r = 0; r < std::max(reps, 5); ++r) step();
             cudaEventRecord(e1, st);
             cudaEventSynchronize(e1);
             float ms = 0.f;
             cudaEventElapsedTime(&ms, e0, e1);
             return ms;
         };
-        const bool pick_list = have_list && pair_ms(c_list, m_list, true) < pair_ms(c_walk, m_walk, false);
+        const float shared = trial(1), own = trial(0);
         SPH_CUDA(h, cudaGetLastError());
-        // one block size for all three stages: the momentum stage's (it dominates)
-        if (pick_list) {
-            h->tune[0] = c_list.tpp;
-            h->tune[1] = SPH_LANES_LIST + m_list.tpp;
-            h->tune[3] = m_list.block;
-        } else {
-            h->tune[0] = c_walk.tpp;
-            h->tune[1] = m_walk.tpp;
-            h->tune[3] = m_walk.block;
-        }
-        if (!pick_list && h->nl.e) {  // the list storage of the trials is not needed
-            SPH_CUDA(h, cudaStreamSynchronize(st));
-            cudaFree(h->nl.e);
-            if (h->nl.n) cudaFree(h->nl.n);
-            h->nl = NbrList{};
-        }
+        h->lanes = shared < own ? 1 : 0;
+        h->tune[0] = h->tune[1] = h->lanes ? 8 : 1;
+        h->tune[3] = h->lanes ? 256 : 128;
         // restore what the timed launches touched: p and c, and the arrivals left in
         // count[]; every other field they wrote is rebuilt by the next step before use
         SPH_CUDA(h, cudaMemsetAsync(h->sc.count, 0, sizeof(int32_t) * (size_t)h->scan_cells, st));
+        SPH_CUDA(h, cudaMemsetAsync(h->sc.n_walked, 0, 4, st));
         if (h->has_buffers) SPH_CUDA(h, cudaMemsetAsync(h->bs.npend, 0, 4, st));  // outlet marks of the trials
         SPH_CUDA(h, cudaMemcpyAsync(h->S[par].p, h->S[par ^ 1].p, nbytes, cudaMemcpyDeviceToDevice, st));
         SPH_CUDA(h, cudaMemcpyAsync(h->S[par].c, h->S[par ^ 1].c, nbytes, cudaMemcpyDeviceToDevice, st));

@@ -1,6 +1,7 @@
-// sph_coop.cuh — cooperative neighbour gathers of the plain FP64 form.
+// sph_coop.cuh — cooperative neighbour gathers: what the plain FP64 form (sph_fp64.cu) and
+// the FP32-compensated form (sph_fp32.cuh) share, and the building blocks of the former.
 //
-// GB300 has two FP64 lanes a SM and cycle (1/64 of FP32), so the gathers of this form are
+// GB300 has two FP64 lanes a SM and cycle (1/64 of FP32), so the gathers of the FP64 form are
 // bound by their FP64 instructions and, on small scenes, by how few SMs those run on.  Two
 // things follow, and both live here:
 //   * kCoopLanes lanes of a warp share one particle.  They first select its neighbours with
@@ -205,44 +206,60 @@ __device__ __forceinline__ bool inside_cut(double d2, const SceneDev& S) {
 // cell and the cell's x index (exact: a grid has at most 2^24 cells on an axis).
 template <int DIM, typename V>
 __device__ __forceinline__ float4 select_pos(const V& x, const SceneDev& S, const int32_t c[3]) {
-    float fu[3];
-    cell_units<DIM>(x, S, c, fu);
-    return make_float4(fu[0], fu[1], fu[2], (float)c[0]);
+    float4 p;
+    p.x = (float)fma(x.x - S.lo[0], S.inv_cell[0], -(double)c[0]);
+    p.y = (float)fma(x.y - S.lo[1], S.inv_cell[1], -(double)c[1]);
+    p.z = DIM == 3 ? (float)fma(comp(x, DIM - 1) - S.lo[2], S.inv_cell[2], -(double)c[2]) : 0.f;
+    p.w = (float)c[0];
+    return p;
+}
+__device__ __forceinline__ bool select_far(const float4& p) {
+    return !(fabsf(p.x) <= 64.f && fabsf(p.y) <= 64.f && fabsf(p.z) <= 64.f);
 }
 
+// |r|^2 with a fixed rounding sequence: every kernel of the FP32 form decides a pair alike.
+__device__ __forceinline__ float dist2(float rx, float ry, float rz) {
+    return __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, __fmul_rn(rz, rz)));
+}
+
+// Lengths of a selection: the cell edges, 1 / ex, and the bound on d^2 beyond which rows and
+// cells are left out (prune).
+struct SelectScale {
+    float ex, ey, ez, inv_ex, r2;
+    bool prune;
+};
+
 // The candidates of one particle in the cell list (start, pos), tested in FP32 and packed
-// into `list` (shared memory of the particle's lanes) in walk order (cells z, y, x); the
-// pair work `flush(cnt)` runs when the list is full and at the end.  me: the particle's
-// select_pos, c its cell, self its index in `pos` (-1: none).  Every lane of the warp calls
-// this together; a group without a particle passes on = false.
+// into a list in walk order (cells z, y, x): accept(j, d2) says whether candidate j is taken,
+// emit(slot, j, rx, ry, rz) lists it (r = x_i - x_j), CAP slots; the pair work
+// pairs(first, cnt, last) runs at the end (last) and before when a list of the warp is full:
+// the list then holds entries first .. first + cnt - 1 of the whole, and pairs returns how
+// many of them it left at its front.  me: the particle's select_pos, c its cell, self its
+// index in `pos` (-1: none).  Every lane of the warp calls this together; a group without a
+// particle passes on = false.
 //
-// The test keeps a relative margin of 1e-4 on r_cut^2: cell-relative differences within
-// the stencil carry an FP32 error of some 1e-6 cells.  A particle clamped into an edge cell
-// from further than 64 cells outside the grid, or with a non-finite position, is tested by
-// `within(j)` instead (FP64), so only candidates beyond r_cut are left out.
-template <int DIM, typename Within, typename Pairs>
-__device__ __forceinline__ void coop_select(const SceneDev& S, const int32_t* __restrict__ start,
-                                            const float4* __restrict__ pos, const int32_t c[3], const float4 me,
-                                            int self, bool on, int32_t* list, Within&& within,
-                                            Pairs&& pairs) {
-    constexpr int CAP = kCoopList<DIM>;
+// Pruning keeps a margin on r_cut^2 far above the FP32 rounding of positions within a few
+// cells.  Rows on the y/z grid boundary and the first and last x cells may hold particles
+// clamped from outside the grid and stay whole, as does the stencil of a particle itself far
+// outside its cell.
+template <int DIM, int CAP, typename Accept, typename Emit, typename Pairs>
+__device__ __forceinline__ void coop_select(const SceneDev& S, const SelectScale& sc,
+                                            const int32_t* __restrict__ start, const float4* __restrict__ pos,
+                                            const int32_t c[3], const float4 me, int self, bool on, Accept&& accept,
+                                            Emit&& emit, Pairs&& pairs) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & (kCoopLanes - 1);
     const int shift = (threadIdx.x & 31) & ~(kCoopLanes - 1);
     const unsigned below = (1u << lane) - 1u;
     const int m = S.reach;
     const int zr = DIM == 3 ? m : 0;
-    const float ex = S.sel_e[0], ey = S.sel_e[1], ez = S.sel_e[2];  // cell edges in units of r_cut
-    const float r2 = 1.0001f;
     const float nx = (float)S.n[0];
-    const bool wide = !(fabsf(me.x) <= 64.f && fabsf(me.y) <= 64.f && fabsf(me.z) <= 64.f);
+    const bool prune = sc.prune && !select_far(me);
     const int planes = DIM == 3 ? (int)__reduce_max_sync(full, (unsigned)zr) : 0;
     int first_entry = 0, cnt = 0;
     for (int dz = -planes; dz <= planes; ++dz) {
         // lane r holds row dy = r - 3 of this plane: its cells form one run [b, b + l1) of the
-        // sorted arrays, or two where a periodic axis wraps; cells beyond r_cut are skipped as
-        // in walk_cells_pruned (rows and cells at the grid's edge stay whole: they may hold
-        // clamped particles)
+        // sorted arrays, or two where a periodic axis wraps
         int b = 0, l1 = 0, b2 = 0, l2 = 0;
         const int dy = lane - 3, y = c[1] + dy, z = c[2] + dz;
         if (on && lane < 7 && dy >= -m && dy <= m && y >= 0 && y < S.n[1] &&
@@ -251,16 +268,16 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const int32_t* __
             int x0 = c[0] - m, x1 = c[0] + m;
             bool keep = true;
             const bool edge = y == 0 || y == S.n[1] - 1 || (DIM == 3 && (z == 0 || z == S.n[2] - 1));
-            if (!edge && !wide) {
-                const float gy = fmaxf(fmaxf((float)dy - me.y, me.y - (float)(dy + 1)), 0.f) * ey;
-                float rem = r2 - gy * gy;
+            if (!edge && prune) {
+                const float gy = fmaxf(fmaxf((float)dy - me.y, me.y - (float)(dy + 1)), 0.f) * sc.ey;
+                float rem = sc.r2 - gy * gy;
                 if (DIM == 3) {
-                    const float gz = fmaxf(fmaxf((float)dz - me.z, me.z - (float)(dz + 1)), 0.f) * ez;
+                    const float gz = fmaxf(fmaxf((float)dz - me.z, me.z - (float)(dz + 1)), 0.f) * sc.ez;
                     rem -= gz * gz;
                 }
                 keep = !(rem < 0.f);
                 if (keep && !S.periodic_x) {
-                    const float w = sqrtf(rem) * S.sel_inv_ex;
+                    const float w = sqrtf(rem) * sc.inv_ex;
                     const int a = c[0] + (int)floorf(me.x - w), e = c[0] + (int)floorf(me.x + w);
                     if (x0 > 0 && a > x0) x0 = min(a, S.n[0] - 1);
                     if (x1 < S.n[0] - 1 && e < x1) x1 = max(e, 0);
@@ -297,6 +314,7 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const int32_t* __
 #pragma unroll
         for (int r = 0; r < 6; ++r) ends[r] = __shfl_sync(full, end, r, kCoopLanes);
         const int first = end - l1 - l2;
+        const int shifted = b - first;  // candidate t of the plane is particle t + shifted of its row
         const bool wraps = __any_sync(full, l2 != 0);
         const int most = (int)__reduce_max_sync(full, (unsigned)total);
         const int rounds = dz == planes ? max(most, 1) : most;  // the last round runs the pairs
@@ -311,13 +329,11 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const int32_t* __
                 int r = 0;
 #pragma unroll
                 for (int k = 0; k < 6; ++k) r += t >= ends[k];
-                int q = t - __shfl_sync(full, first, r, kCoopLanes);  // place in the row
-                const int jb = __shfl_sync(full, b, r, kCoopLanes);
+                int q = t + __shfl_sync(full, shifted, r, kCoopLanes);
                 if (wraps) {
-                    const int n1 = __shfl_sync(full, l1, r, kCoopLanes), jb2 = __shfl_sync(full, b2, r, kCoopLanes);
-                    q = q < n1 ? jb + q : jb2 + (q - n1);
-                } else {
-                    q += jb;
+                    const int f = __shfl_sync(full, first, r, kCoopLanes), n1 = __shfl_sync(full, l1, r, kCoopLanes);
+                    const int jb2 = __shfl_sync(full, b2, r, kCoopLanes);
+                    if (t - f >= n1) q = jb2 + (t - f - n1);
                 }
                 dyf[h] = (float)(r - 3);
                 j[h] = t < total ? q : -1;
@@ -326,31 +342,50 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const int32_t* __
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                float cx = p[h].w - me.w;
+                float cx = me.w - p[h].w;
                 if (S.periodic_x) cx = cx > 0.5f * nx ? cx - nx : (cx < -0.5f * nx ? cx + nx : cx);
-                const float rx = (cx + (p[h].x - me.x)) * ex;
-                const float ry = (dyf[h] + (p[h].y - me.y)) * ey;
-                float d2 = rx * rx + ry * ry;
-                if (DIM == 3) {
-                    const float rz = ((float)dz + (p[h].z - me.z)) * ez;
-                    d2 += rz * rz;
-                }
+                const float rx = (cx + (me.x - p[h].x)) * sc.ex;
+                const float ry = ((me.y - p[h].y) - dyf[h]) * sc.ey;
+                const float rz = DIM == 3 ? ((me.z - p[h].z) - (float)dz) * sc.ez : 0.f;
                 bool take = j[h] >= 0 && j[h] != self;
-                if (take) take = wide ? within(j[h]) : d2 <= r2;
+                if (take) take = accept(j[h], dist2(rx, ry, rz));
                 const unsigned hit = (__ballot_sync(full, take) >> shift) & 0xffu;
-                if (take) list[cnt + __popc(hit & below)] = j[h];
+                if (take) emit(cnt + __popc(hit & below), j[h], rx, ry, rz);
                 cnt += __popc(hit);
             }
             const bool last = dz == planes && t0 + 2 * kCoopLanes >= rounds;
             if (last || __any_sync(full, cnt > CAP - 2 * kCoopLanes)) {
                 __syncwarp(full);
-                pairs(first_entry, cnt);
+                const int kept = pairs(first_entry, cnt, last);
                 __syncwarp(full);
-                first_entry += cnt;
-                cnt = 0;
+                first_entry += cnt - kept;
+                cnt = kept;
             }
         }
     }
+}
+
+// The next step's cell key of a particle that moved from x0 to x1: its FP32 cell position
+// decides it where the particle is clear of the cell boundaries (by 1e-4 cells, far above
+// the FP32 error) and of the grid's edge cells, the FP64 hash otherwise; the key is the
+// same.  The hash takes six FP64 instructions an axis, this two.
+template <int DIM, typename V>
+__device__ __forceinline__ int32_t moved_key(int32_t key, const float4& me, const V& x0, const V& x1,
+                                             const SceneDev& S) {
+    const float u[3] = {me.x + (float)(x1.x - x0.x) * S.inv_cell_f[0], me.y + (float)(x1.y - x0.y) * S.inv_cell_f[1],
+                        DIM == 3 ? me.z + (float)(comp(x1, DIM - 1) - comp(x0, DIM - 1)) * S.inv_cell_f[2] : 0.f};
+    int32_t c[3];
+    decode_cell(key, S, c);
+    bool sure = true;
+    int32_t k = key, stride = 1;
+#pragma unroll
+    for (int a = 0; a < DIM; ++a) {
+        const float f = floorf(u[a]), frac = u[a] - f;
+        sure &= frac > 1e-4f && frac < 1.f - 1e-4f && fabsf(f) <= 1.f && c[a] > 1 && c[a] < S.n[a] - 2;
+        k += (int32_t)f * stride;
+        stride *= S.n[a];
+    }
+    return sure ? k : cell_key<DIM>(x1, S);
 }
 
 // Adds a round of pair terms (entry e of the list in lane e of the particle's group, e0 <=

@@ -45,7 +45,7 @@ struct SceneDev {
     double cell_d[3];   // cell edge per axis; cell c starts at lo + c * cell_d
     int32_t n[3];
     int32_t reach;      // neighbour cells within +-reach (cells per r_cut)
-    int32_t prune;      // 1: the FP32 walks skip neighbour cells beyond r_cut (row_span)
+    int32_t prune;      // 1: the FP32 gathers skip neighbour cells beyond r_cut
     int32_t cell_off;   // first global cell of this scene
     int32_t ncells;
     int32_t periodic_x;
@@ -94,11 +94,12 @@ struct SceneDev {
 
     // FP32-compensated form
     float cell_f[3];   // cell edge per axis (float)
-    float h_f, rc2_f, hh001_f, nu0_f, P_bg_f;
-    float kw_a_f, kg_a_f, inv_h_f, c0_f, rho0_f, inv_cp_f, inv_rho0_f;
+    float inv_cell_f[3];
+    float rc2_f, hh001_f, inv_h_f, inv_hh_f, nu4_f, P_bg_f;
+    float kw_a_f, tens_f;  // tens_f: 0.01 kw_a / W(gap), when uniform_gap
+    float inv_cp_f, inv_rho0_f;
     float rc2_prune;    // rc2_f * (1 + 1e-5): conservative bound for the stencil pruning
     float inv_cell_fx;  // 1 / cell_f[0]
-    float pad_f;
 };
 
 // ---------------------------------------------------------------- vector types
@@ -129,12 +130,10 @@ struct SortedState {
     double* cp;
     int32_t* id;
     int32_t* scene;
-    // FP32 shadows (allocated only for the compensated form)
-    // (the FP64 form keeps fa = select_pos, see sph_coop.cuh, cell and vol as well)
-    float4* fa;   // 2D: (xr, yr, vx, vy)      3D: (xr, yr, zr, m)
-    float4* fb;   // 2D: (m, rho, P, gap)      3D: (vx, vy, vz, rho)
-    float4* fc;   // 2D: (T, kappa, cp, -)     3D: (P, gap, T, kappa)
-    float* fd;    // 3D: cp
+    // FP32 copies for the gathers (fb, fc: compensated form only)
+    float4* fa;   // selection position (select_pos): (x, y, z) relative to the cell in cell units, cell x
+    float4* fb;   // (vx, vy, vz, m kg_a / h)
+    float4* fc;   // (rho, P, T, kappa); rho and P after continuity
     int32_t* cell;  // cell key of the particle (global)
     double* vol;    // m / rho after continuity
 };
@@ -156,24 +155,20 @@ struct WallState {
     int32_t* kind;
     int32_t* start;  // global cells + 1
     uint8_t* near;   // global cells: 1 where a wall particle lies within +-reach cells
-    float4* fa;      // FP32: 2D (xr, yr, nx, ny)    3D (xr, yr, zr, gap); FP64: select_pos
-    float4* fb;      // FP32: 2D (vx, vy, gap, T)    3D (nx, ny, nz, T)
-    float4* fc;      // FP32: 2D (kappa, kind, -, -) 3D (vx, vy, vz, kappa)
+    float4* fa;      // selection position
+    float4* fb;      // FP32 form: (normal, gap)
+    float4* fc;      // FP32 form: (velocity, T)
+    float* fk;       // FP32 form: kappa
     int32_t* cell;
     int64_t n;
 };
 
-// Neighbour list of the FP32 form: the continuity gather records, in its walk order,
-// every neighbour within r_cut of each particle; the momentum gather of the same step
-// reads it instead of walking the cells again (the pairs are the same: positions do not
-// change between the two gathers).  Entry k of particle i is e[k * stride + i] =
-// (j - i) << 9 | (dz + m) << 6 | (dy + m) << 3 | (dx + m): j the sorted index of the
-// neighbour, (dx, dy, dz) the offset of j's cell from i's cell, m the reach in cells.
-// A one-lane writer fills entries 0, 1, ...; with two lanes, lane 0 fills them from 0 up
-// and lane 1 from kmax - 1 down.  n[i] = front | back << 16 (the entries written by the
-// two lanes), or kListWalk when they do not fit (more than kmax neighbours, j - i outside
-// 23 bits, or m > 3): momentum then walks the cells for i.  The list of i reads as
-// entries 0 .. front - 1, then kmax - 1 down to kmax - back.
+// Neighbour list of the FP32 form: continuity records, in walk order, the neighbours within
+// r_cut of each particle, and the momentum gather of the same step reads them instead of
+// walking the cells again.  Entry k of particle i is e[k * stride + i] = (j - i) << 9 |
+// (dz + 3) << 6 | (dy + 3) << 3 | (dx + 3): j the sorted index of the neighbour, (dx, dy, dz)
+// the offset of j's cell from i's cell.  n[i] is their number, or kListWalk when they do not
+// fit (more than kmax, or j - i outside 23 bits): momentum then walks the cells for i.
 struct NbrList {
     int32_t* e;
     int32_t* n;
@@ -193,6 +188,11 @@ struct SortScratch {
     int32_t* n_live;    // device scalar: live particles after the last sort
     int32_t* status;    // device scalar: status bits
     int32_t* queue;     // draws and finished blocks of a cooperative gather (coop_turns), both 0 between launches
+    // FP32 form, large scenes: the particles whose cells the momentum gather walks, their
+    // number (0 before continuity) and their sums of those walks (fluid, walls, Shepard)
+    int32_t* walked;
+    int32_t* n_walked;
+    float2* walk_sums;
     int64_t* scene_step;  // per scene: number of the step being run
     // non-null in a step whose scan runs over 1,024-cell tiles: the momentum epilogue adds
     // each particle's arrival to its tile's sum here (the scan then skips its tile pass)

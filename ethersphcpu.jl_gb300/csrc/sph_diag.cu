@@ -7,9 +7,9 @@
 // restatement: the key is the one the step's sort uses, and the neighbour test is the
 // one the gathers of the handle's form use (FP64: d^2 <= r_cut^2 in FP64 with the
 // products and sums rounded one by one, as k_momentum_fp64; FP32-compensated: the same
-// test in FP32 on cell-relative positions, as k_continuity_f32 records the neighbour
-// list, stencil pruning included).
-#include "sph_fp32.cuh"
+// test in FP32 on cell-relative positions, as coop_select takes it; the stencil pruning
+// leaves out only what that test rejects).
+#include "sph_coop.cuh"
 
 namespace sph {
 
@@ -63,20 +63,27 @@ __global__ void k_neighbours_f32(const SceneDev* __restrict__ scenes, SortedStat
     const int i = b + (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (i >= e) return;
     const SceneDev& S = scenes[st.scene[i]];
-    const float4 ai = st.fa[i];
-    const float xi[3] = {ai.x, ai.y, DIM == 3 ? ai.z : 0.f};
+    const float4 me = st.fa[i];
     int32_t c[3];
     decode_cell(st.cell[i], S, c);
     int32_t* out = ids ? ids + rows[i - b] : nullptr;
     int32_t cnt = 0;
-    auto load = [&](int j) { return st.fa[j]; };
-    walk<DIM, 1, false>(S, start, c, xi, 0, load, [&](int j, const float4& aj, float ox, float oy, float oz, int) {
-        if (j == i) return;
-        const float rx = xi[0] - ox - aj.x, ry = xi[1] - oy - aj.y;
-        const float rz = DIM == 3 ? xi[2] - oz - aj.z : 0.f;
-        if (!(dist2(rx, ry, rz) <= S.rc2_f)) return;
-        if (out) out[cnt] = st.id[j];
-        ++cnt;
+    const float nx = (float)S.n[0];
+    walk_cells<DIM>(S, start, c, [&](int jb, int je) {
+        for (int j = jb; j < je; ++j) {
+            if (j == i) continue;
+            const float4 p = st.fa[j];
+            int32_t cj[3];
+            decode_cell(st.cell[j], S, cj);
+            float cx = me.w - p.w;
+            if (S.periodic_x) cx = cx > 0.5f * nx ? cx - nx : (cx < -0.5f * nx ? cx + nx : cx);
+            const float rx = (cx + (me.x - p.x)) * S.cell_f[0];
+            const float ry = ((me.y - p.y) - (float)(cj[1] - c[1])) * S.cell_f[1];
+            const float rz = DIM == 3 ? ((me.z - p.z) - (float)(cj[2] - c[2])) * S.cell_f[2] : 0.f;
+            if (!(dist2(rx, ry, rz) <= S.rc2_f)) continue;
+            if (out) out[cnt] = st.id[j];
+            ++cnt;
+        }
     });
     if (counts) counts[i - b] = cnt;
 }

@@ -1,38 +1,34 @@
 // sph_fp32.cuh — FP32-compensated form of the continuity, momentum and Shepard gathers
 //
-// Pair arithmetic runs in FP32 on cell-relative positions: every particle carries
-// (x - origin of its cell) as floats, and a neighbour in the cell offset (dx, dy, dz)
-// sits at xr_j + (dx, dy, dz) * edge in the frame of particle i's cell, so r_vec is
-// formed from numbers of magnitude <= 2 r_cut with an absolute error of a few 1e-9 r_cut.
-// Continuity and force sums are Kahan-compensated FP32 accumulators; the result
-// (sum - compensation) goes to FP64 before the forward-Euler update, which runs in FP64
-// on the FP64 master position / velocity / density / temperature.  The Shepard sums
-// accumulate in FP64 (FP32 kernel values times FP64 volumes and masses).
+// Pair arithmetic runs in FP32 on cell-relative positions: every particle carries its
+// position relative to its cell, in cell units, and its cell's x index (select_pos), so the
+// vector to a neighbour dx cells away is (dx + (x_i - x_j)) edge, formed from numbers of
+// magnitude <= 4 with an error of some 1e-7 cells.  Continuity and force sums are
+// Kahan-compensated FP32 accumulators; the result (sum - compensation) goes to FP64 before
+// the forward-Euler update, which runs in FP64 on the FP64 master position / velocity /
+// density / temperature.  The Shepard sums accumulate in FP64 (FP32 kernel values times
+// FP64 volumes and masses).
 //
-// Each particle's neighbour walk is split over TPP consecutive lanes of a warp: lane t
-// takes candidates t, t+TPP, ... of every neighbour row (the x-cells of a row are one
-// virtual range), keeps its own compensated partial sums, and the lanes combine them
-// with an xor butterfly (FP32 TwoSum of the sums, the rounding errors joining the
-// compensations) — every lane ends with the bitwise same total, so results are
-// deterministic for a given TPP.  TPP and the block size are launch parameters picked by
-// the autotuner (more lanes per particle = more warps in flight to hide the dependent
-// neighbour loads).  With the neighbour-list shapes the continuity gather records each
-// particle's accepted neighbours (NbrList) and the momentum gather reads them instead of
-// walking the cells again; the walks may skip cells of a row beyond r_cut (row_span).
+// Continuity walks the cells, one thread a particle on large scenes and a lane a neighbour
+// row on small ones (the same sums, bit for bit), and records each particle's neighbours
+// (NbrList).  Momentum reads that list with eight lanes a particle: lane t takes entries
+// t, t + 8, ... with compensated partial sums of its own; its block's first warps merge them
+// (TwoSum of the sums, the rounding errors joining the compensations) and update the
+// particles, one thread each, because FP64 instructions, of which a GB300 SM runs 1/64 of
+// its FP32 rate, cost a warp the same however many lanes take part.  A particle whose list
+// does not fit is walked again (coop_select), in the same order.  No sum depends on the block
+// size, the batch or the pruning.
+//
 // On a re-initialisation step the momentum gather also forms the Shepard sums over the
-// same neighbours (FP32 kernel values, FP64 sums) and writes the re-initialised density:
-// the update and the re-initialisation are one kernel.
+// same neighbours and writes the re-initialised density: the update and the
+// re-initialisation are one kernel.
 //
 // Same terms, order of walls after fluid, and solve variants as sph_fp64.cu; the
 // formulas follow Continuity.jl, PressureForce.jl, ViscosityForce.jl, WallForce.jl,
 // ThermalConduction.jl, SelfAction/*.jl and ReconstructValue.jl.
 #pragma once
 
-#include <climits>
-#include <type_traits>
-
-#include "sph_physics.cuh"
-#include "sph_kernels.h"
+#include "sph_coop.cuh"
 
 namespace sph {
 
@@ -48,7 +44,6 @@ struct Kahan {
         c = (t - s) - y;
         s = t;
     }
-    __device__ __forceinline__ double value() const { return (double)s - (double)c; }
 };
 
 // x^n for n >= 0 by repeated squaring, without the compensation of jl_powi.
@@ -62,502 +57,229 @@ __device__ __forceinline__ double powi_plain(double x, int n) {
     return y;
 }
 
-template <int TPP>
-__device__ __forceinline__ unsigned group_mask() {
-    if (TPP == 32) return 0xffffffffu;
-    const unsigned lane = threadIdx.x & 31u;
-    return ((1u << TPP) - 1u) << (lane & ~(unsigned)(TPP - 1));
+// Adds a compensated sum (s, c) to another: the sums by an error-free TwoSum whose rounding
+// error joins the compensations.
+__device__ __forceinline__ void merge(Kahan& k, float s2, float c2) {
+    const float t = k.s + s2;
+    const float bp = t - k.s;
+    const float e = (k.s - (t - bp)) + (s2 - bp);
+    k.s = t;
+    k.c = (k.c + c2) - e;
 }
 
-// Combine the compensated sums of a particle's TPP lanes in place: the lanes' (s, c)
-// pairs are merged in FP32 (the sums by an error-free TwoSum whose rounding error joins
-// the compensations); every lane ends with the same bits, and one lane converts the
-// result with value() (FP64 work is slow on GB300: done once per particle).
-template <int TPP>
-__device__ __forceinline__ void group_combine(Kahan& k, unsigned mask) {
-#pragma unroll
-    for (int o = TPP / 2; o > 0; o >>= 1) {
-        const float s2 = __shfl_xor_sync(mask, k.s, o);
-        const float c2 = __shfl_xor_sync(mask, k.c, o);
-        const float t = k.s + s2;
-        const float bp = t - k.s;
-        const float e = (k.s - (t - bp)) + (s2 - bp);
-        k.s = t;
-        k.c = (k.c + c2) - e;
-    }
+// 1 / sqrt(a) and a / b by the hardware's approximations, subnormal arguments taken as zero
+// (q^2 and the divisors below are ordinary numbers).
+__device__ __forceinline__ float rsqrt_ftz(float a) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(a));
+    return y;
+}
+__device__ __forceinline__ float div_ftz(float a, float b) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmul_rn(a, y);
 }
 
-template <int TPP>
-__device__ __forceinline__ double group_sum(double v, unsigned mask) {
-#pragma unroll
-    for (int o = TPP / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
-    return v;
-}
-
-// W and dW/dr in FP32 (same polynomials as sph_physics.cuh).
+// F with dW/dr / r = (kg_a / h) F (finite at r = 0) and w with W = kw_a w at q = r / h;
+// inv_q = 1 / q (0 at q = 0).  Every product and sum is rounded as written (no contraction
+// left to the compiler), so each kernel that forms a pair gets the same bits.
 template <int KK>
-__device__ __forceinline__ void kernel_wdw_f(float q, const SceneDev& S, float& W, float& dW) {
-    if (KK == SPH_KERNEL_CUBIC_SPLINE) {
-        if (q < 1.f) {
-            W = S.kw_a_f * (3.f * q * q * (q - 2.f) + 4.f);
-            dW = S.kg_a_f * q * (3.f * q - 4.f);
-        } else if (q < 2.f) {
-            const float t = 2.f - q;
-            W = S.kw_a_f * t * t * t;
-            dW = -S.kg_a_f * t * t;
-        } else {
-            W = 0.f;
-            dW = 0.f;
-        }
-    } else if (KK == SPH_KERNEL_GAUSSIAN) {
-        if (q < 3.f) {
-            const float e = __expf(-q * q);
-            W = S.kw_a_f * e;
-            dW = S.kg_a_f * q * e;
-        } else {
-            W = 0.f;
-            dW = 0.f;
-        }
+__device__ __forceinline__ void kernel_fw(float q, float inv_q, float& F, float& w) {
+    if (KK == SPH_KERNEL_GAUSSIAN) {
+        const float e = q < 3.f ? __expf(-__fmul_rn(q, q)) : 0.f;
+        F = e;
+        w = e;
+    } else if (KK == SPH_KERNEL_CUBIC_SPLINE) {
+        const float t = fmaxf(__fsub_rn(2.f, q), 0.f);
+        const float t2 = __fmul_rn(t, t);
+        const bool in = q < 1.f;
+        F = in ? __fmaf_rn(3.f, q, -4.f) : -__fmul_rn(t2, inv_q);
+        w = in ? __fmaf_rn(__fmul_rn(3.f, __fmul_rn(q, q)), __fsub_rn(q, 2.f), 4.f) : __fmul_rn(t2, t);
     } else if (KK == SPH_KERNEL_WENDLAND_C2) {
-        if (q < 2.f) {
-            const float t = 2.f - q;
-            const float t3 = t * t * t;
-            W = S.kw_a_f * (t3 * t) * (1.f + 2.f * q) * 0.0625f;
-            dW = S.kg_a_f * q * t3;
-        } else {
-            W = 0.f;
-            dW = 0.f;
-        }
+        const float t = fmaxf(__fsub_rn(2.f, q), 0.f);
+        const float t2 = __fmul_rn(t, t);
+        F = __fmul_rn(t2, t);
+        w = __fmul_rn(__fmul_rn(t2, t2), __fmaf_rn(0.125f, q, 0.0625f));
     } else {
-        if (q < 2.f) {
-            const float t = 2.f - q;
-            const float t2 = t * t;
-            const float t5 = t2 * t2 * t;
-            W = S.kw_a_f * (t5 * t) * (35.f * q * q + 36.f * q + 12.f) * (1.f / 768.f);
-            dW = S.kg_a_f * (35.f / 96.f * q * q + 7.f / 48.f * q) * t5;
-        } else {
-            W = 0.f;
-            dW = 0.f;
-        }
+        const float t = fmaxf(__fsub_rn(2.f, q), 0.f);
+        const float t2 = __fmul_rn(t, t);
+        const float t5 = __fmul_rn(__fmul_rn(t2, t2), t);
+        F = __fmul_rn(t5, __fmaf_rn(35.f / 96.f, q, 7.f / 48.f));
+        w = __fmul_rn(__fmul_rn(t5, t), __fmaf_rn(__fmaf_rn(35.f / 768.f, q, 36.f / 768.f), q, 12.f / 768.f));
     }
 }
-
 template <int KK>
-__device__ __forceinline__ float kernel_w_f(float q, const SceneDev& S) {
-    float W, dW;
-    kernel_wdw_f<KK>(q, S, W, dW);
-    return W;
+__device__ __forceinline__ float kernel_w_f(float q) {
+    float F, w;
+    kernel_fw<KK>(q, 1.f, F, w);
+    return w;
 }
 
-// Neighbour rows in (z, y) order (within +-reach cells); inside a row the cells
-// x-reach .. x+reach (wrapping on a periodic axis, skipped off the grid) form one virtual
-// range that the TPP lanes share.  The callback gets the sorted index j and the offset
-// of j's cell from i's cell in metres.
-// A neighbour row whose cells x-m .. x+m do not wrap is one contiguous run of the
-// sorted arrays, [b, e); the cell of a candidate follows from the interior cell
-// boundaries (at most 2m = 6 of them): dx = dx0 + #(boundaries <= j).
-struct RowRun {
-    int b, e, dx0;
-    int bnd[6];
+constexpr int kSumStride = 36;  // row of lane sums in shared memory (a warp's lanes fall on different banks)
+
+// A pair with r_vec (metres) and the neighbour's index in e.
+template <int DIM, int KK>
+struct PairF {
+    float r[3], d2, F, w;
+    int j;
+    __device__ __forceinline__ PairF(const float4& e, const SceneDev& S) {
+        r[0] = e.x;
+        r[1] = e.y;
+        r[2] = DIM == 3 ? e.z : 0.f;
+        j = __float_as_int(e.w);
+        d2 = dist2(r[0], r[1], r[2]);
+        const float q2 = __fmul_rn(d2, S.inv_hh_f);
+        const float inv_q = q2 > 1e-30f ? rsqrt_ftz(q2) : 0.f;  // a coincident neighbour has q = 0
+        kernel_fw<KK>(__fmul_rn(q2, inv_q), inv_q, F, w);
+    }
 };
 
-__device__ __forceinline__ bool row_run(const SceneDev& S, const int32_t* __restrict__ start, int row, int cx,
-                                        int xlo, int xhi, RowRun& R) {
-    // a row whose full stencil wraps takes the cell-by-cell path whatever its pruned
-    // span: each row keeps one code path (one inlined copy of the pair terms, one rounding)
-    const int m = S.reach;
-    if (S.periodic_x && (cx - m < 0 || cx + m >= S.n[0])) return false;
-    const int x0 = cx + xlo < 0 ? 0 : cx + xlo;
-    const int x1 = cx + xhi >= S.n[0] ? S.n[0] - 1 : cx + xhi;
-    R.b = __ldg(start + row + x0);
-    R.e = __ldg(start + row + x1 + 1);
-    R.dx0 = x0 - cx;
-#pragma unroll
-    for (int q = 0; q < 6; ++q) {
-        const int cell = x0 + 1 + q;
-        R.bnd[q] = cell <= x1 ? __ldg(start + row + cell) : INT_MAX;
-    }
-    return true;
-}
+constexpr int kRowEntries = 16;  // list entries of a row (more: momentum walks the cells for the particle)
 
-// The cells of neighbour row (dy, dz) that can hold a particle within r_cut of particle i
-// (cell-relative position xi): offsets [xlo, xhi] in x, or false when none can.  Bounds
-// are taken from the cell extents with a relative margin of 1e-5 on r_cut^2 (far above
-// the FP32 rounding of the pair distance), so only candidates the distance test would
-// reject are skipped and the walk visits the accepted ones in the same order.  Particles
-// outside the domain are clamped into the grid's first and last cells with their true
-// positions: rows on the y/z grid boundary are kept whole, and the first and last x cells
-// are never trimmed away.
+// List entry of neighbour j of i in the cell (dx, dy, dz) away: (j - i) << 9 | (dz + 3) << 6 |
+// (dy + 3) << 3 | (dx + 3).
+__device__ __forceinline__ float code_offset(int32_t code, int shift) {  // the offset + 3 as a float
+    return __int_as_float(0x4b000000 | (code >> shift & 7)) - (8388608.f + 3.f);
+}
+// r_vec of the listed pair as coop_select forms it, and the neighbour's index.
 template <int DIM>
-__device__ __forceinline__ bool row_span(const SceneDev& S, const int32_t c[3], const float xi[3], int y, int z,
-                                         int dy, int dz, int& xlo, int& xhi) {
-    const int m = S.reach;
-    xlo = -m;
-    xhi = m;
-    if (!S.prune) return true;
-    if (y == 0 || y == S.n[1] - 1 || (DIM == 3 && (z == 0 || z == S.n[2] - 1))) return true;
-    const float ey = S.cell_f[1];
-    const float gy = fmaxf(fmaxf((float)dy * ey - xi[1], xi[1] - (float)(dy + 1) * ey), 0.f);
-    float g2 = gy * gy;
-    if (DIM == 3) {
-        const float ez = S.cell_f[2];
-        const float gz = fmaxf(fmaxf((float)dz * ez - xi[2], xi[2] - (float)(dz + 1) * ez), 0.f);
-        g2 += gz * gz;
-    }
-    const float rem = S.rc2_prune - g2;
-    if (rem < 0.f) return false;
-    const float w = sqrtf(rem);
-    int lo = (int)floorf((xi[0] - w) * S.inv_cell_fx);
-    int hi = (int)floorf((xi[0] + w) * S.inv_cell_fx);
-    lo = lo < -m ? -m : lo;
-    hi = hi > m ? m : hi;
-    if (!S.periodic_x) {
-        if (c[0] - m <= 0) {
-            lo = -m;
-            hi = hi < -c[0] ? -c[0] : hi;
-        }
-        if (c[0] + m >= S.n[0] - 1) {
-            hi = m;
-            lo = lo > S.n[0] - 1 - c[0] ? S.n[0] - 1 - c[0] : lo;
-        }
-    }
-    xlo = lo;
-    xhi = hi;
-    return lo <= hi;
+__device__ __forceinline__ float4 listed(int32_t code, const float4& me, const float4& p, int j, const SceneDev& S) {
+    const float rx = ((me.x - p.x) - code_offset(code, 0)) * S.cell_f[0];
+    const float ry = ((me.y - p.y) - code_offset(code, 3)) * S.cell_f[1];
+    const float rz = DIM == 3 ? ((me.z - p.z) - code_offset(code, 6)) * S.cell_f[2] : 0.f;
+    return make_float4(rx, ry, rz, __int_as_float(j));
 }
-
-__device__ __forceinline__ int run_dx(const RowRun& R, int j) {
-    return R.dx0 + (j >= R.bnd[0]) + (j >= R.bnd[1]) + (j >= R.bnd[2]) + (j >= R.bnd[3]) + (j >= R.bnd[4]) +
-           (j >= R.bnd[5]);
-}
-
-// Cell offset of a candidate in metres, and its neighbour-list code (see NbrList).
-// The product is rounded on its own (no contraction into the caller's subtraction), so
-// the cell walk and the list walk form bitwise the same pair vectors.
-__device__ __forceinline__ float cell_offset(int d, float edge) { return __fmul_rn((float)d, edge); }
-__device__ __forceinline__ int row_code(int dy, int dz, int m) { return ((dz + m) << 6) | ((dy + m) << 3); }
-
-// |r|^2 with a fixed rounding sequence: the continuity gather's test and the momentum
-// gather's test agree bit for bit, so the neighbour list holds exactly the pairs the
-// momentum walk would accept.
-__device__ __forceinline__ float dist2(float rx, float ry, float rz) {
-    return __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, __fmul_rn(rz, rz)));
-}
-
-template <int DIM, int TPP, typename F>
-__device__ __forceinline__ void walk_lanes(const SceneDev& S, const int32_t* __restrict__ start, const int32_t c[3],
-                                           const float xi[3], int lane, F&& f) {
-    const int m = S.reach;
-    const int zr = DIM == 3 ? m : 0;
-    for (int dz = -zr; dz <= zr; ++dz) {
-        const int z = c[2] + dz;
-        if (DIM == 3 && (z < 0 || z >= S.n[2])) continue;
-        for (int dy = -m; dy <= m; ++dy) {
-            const int y = c[1] + dy;
-            if (y < 0 || y >= S.n[1]) continue;
-            const int row = S.cell_off + (z * S.n[1] + y) * S.n[0];
-            const float oy = cell_offset(dy, S.cell_f[1]);
-            const float oz = DIM == 3 ? cell_offset(dz, S.cell_f[2]) : 0.f;
-            const int rc = row_code(dy, dz, m) + m;
-            int xlo, xhi;
-            if (!row_span<DIM>(S, c, xi, y, z, dy, dz, xlo, xhi)) continue;
-            // the row's cells are one virtual range v = 0 .. (sum of lengths)-1; lane t
-            // takes v = t, t+TPP, ...
-            RowRun R;
-            if (row_run(S, start, row, c[0], xlo, xhi, R)) {
-                for (int j = R.b + lane; j < R.e; j += TPP) {
-                    const int dx = run_dx(R, j);
-                    f(j, cell_offset(dx, S.cell_f[0]), oy, oz, rc + dx);
-                }
-                continue;
-            }
-            int prefix = 0;  // a wrapping row of a periodic axis: cell by cell
-            for (int dx = xlo; dx <= xhi; ++dx) {
-                int x = c[0] + dx;
-                x = x < 0 ? x + S.n[0] : (x >= S.n[0] ? x - S.n[0] : x);
-                const int b = __ldg(start + row + x);
-                const int e = __ldg(start + row + x + 1);
-                const float ox = cell_offset(dx, S.cell_f[0]);
-                const int first = (lane - prefix) & (TPP - 1);
-                for (int j = b + first; j < e; j += TPP) f(j, ox, oy, oz, rc + dx);
-                prefix += e - b;
-            }
-        }
-    }
-}
-
-// The same walk, software-pipelined: the loads of a lane's next candidate (load(j)) are
-// issued before the current candidate is processed (f(j, data, ...)), so the memory
-// latency of one overlaps the arithmetic of the other.  Few warps per scheduler (small
-// scenes) cannot hide that latency by switching warps.
-template <int DIM, int TPP, typename L, typename F>
-__device__ __forceinline__ void walk_lanes_pf(const SceneDev& S, const int32_t* __restrict__ start,
-                                              const int32_t c[3], const float xi[3], int lane, L&& load, F&& f) {
-    const int m = S.reach;
-    const int zr = DIM == 3 ? m : 0;
-    for (int dz = -zr; dz <= zr; ++dz) {
-        const int z = c[2] + dz;
-        if (DIM == 3 && (z < 0 || z >= S.n[2])) continue;
-        for (int dy = -m; dy <= m; ++dy) {
-            const int y = c[1] + dy;
-            if (y < 0 || y >= S.n[1]) continue;
-            const int row = S.cell_off + (z * S.n[1] + y) * S.n[0];
-            const float oy = cell_offset(dy, S.cell_f[1]);
-            const float oz = DIM == 3 ? cell_offset(dz, S.cell_f[2]) : 0.f;
-            const int rc = row_code(dy, dz, m) + m;
-            int xlo, xhi;
-            if (!row_span<DIM>(S, c, xi, y, z, dy, dz, xlo, xhi)) continue;
-            RowRun R;
-            if (row_run(S, start, row, c[0], xlo, xhi, R)) {
-                int j = R.b + lane;
-                if (j >= R.e) continue;
-                auto d = load(j);
-                for (;;) {
-                    const int jn = j + TPP;
-                    const bool more = jn < R.e;
-                    decltype(d) dn = d;
-                    if (more) dn = load(jn);
-                    const int dx = run_dx(R, j);
-                    f(j, d, cell_offset(dx, S.cell_f[0]), oy, oz, rc + dx);
-                    if (!more) break;
-                    j = jn;
-                    d = dn;
-                }
-                continue;
-            }
-            int prefix = 0;  // a wrapping row of a periodic axis: cell by cell
-            for (int dx = xlo; dx <= xhi; ++dx) {
-                int x = c[0] + dx;
-                x = x < 0 ? x + S.n[0] : (x >= S.n[0] ? x - S.n[0] : x);
-                const int b = __ldg(start + row + x);
-                const int e = __ldg(start + row + x + 1);
-                const float ox = cell_offset(dx, S.cell_f[0]);
-                int j = b + ((lane - prefix) & (TPP - 1));
-                prefix += e - b;
-                if (j >= e) continue;
-                auto d = load(j);
-                for (;;) {
-                    const int jn = j + TPP;
-                    const bool more = jn < e;
-                    decltype(d) dn = d;
-                    if (more) dn = load(jn);
-                    f(j, d, ox, oy, oz, rc + dx);
-                    if (!more) break;
-                    j = jn;
-                    d = dn;
-                }
-            }
-        }
-    }
-}
-
-// Walk with (PF) or without software pipelining; body(j, load(j), ox, oy, oz, code).
-template <int DIM, int TPP, bool PF, typename L, typename F>
-__device__ __forceinline__ void walk(const SceneDev& S, const int32_t* __restrict__ start, const int32_t c[3],
-                                     const float xi[3], int lane, L&& load, F&& body) {
-    if constexpr (PF) {
-        walk_lanes_pf<DIM, TPP>(S, start, c, xi, lane, load, body);
-    } else {
-        walk_lanes<DIM, TPP>(S, start, c, xi, lane, [&](int j, float ox, float oy, float oz, int code) {
-            body(j, load(j), ox, oy, oz, code);
-        });
-    }
-}
-
-// Entry k of particle i.
-__device__ __forceinline__ const int32_t* list_entry(const NbrList& nl, int k, int i) {
-    return nl.e + (int64_t)k * nl.stride + i;
-}
-
-// Walk of particle i's neighbour list (cnt entries, NbrList): lane t takes entries t,
-// t+TPP, ...; the PF form loads the next entry and its neighbour's data before the
-// current neighbour is processed.  body as for walk().
-template <int DIM, int TPP, bool PF, typename L, typename F>
-__device__ __forceinline__ void walk_list(const SceneDev& S, const NbrList& nl, int i, int cnt, int lane, L&& load,
-                                          F&& body) {
-    const int m = S.reach;
-    // the list is entries [0, front) followed by entries kmax - 1 down to kmax - back
-    const int front = cnt & 0xffff, back = cnt >> 16;
-    cnt = front + back;
-    auto entry = [&](int k) { return __ldg(list_entry(nl, k < front ? k : nl.kmax - 1 - (k - front), i)); };
-    auto off = [&](int32_t x, float& ox, float& oy, float& oz) {
-        ox = cell_offset((x & 7) - m, S.cell_f[0]);
-        oy = cell_offset(((x >> 3) & 7) - m, S.cell_f[1]);
-        oz = DIM == 3 ? cell_offset(((x >> 6) & 7) - m, S.cell_f[2]) : 0.f;
-    };
-    if constexpr (PF) {
-        int k = lane;
-        if (k >= cnt) return;
-        int32_t x = entry(k);
-        int j = i + (x >> 9);
-        auto d = load(j);
-        for (;;) {
-            const int kn = k + TPP;
-            const bool more = kn < cnt;
-            int32_t xn = x;
-            int jn = j;
-            decltype(d) dn = d;
-            if (more) {
-                xn = entry(kn);
-                jn = i + (xn >> 9);
-                dn = load(jn);
-            }
-            float ox, oy, oz;
-            off(x, ox, oy, oz);
-            body(j, d, ox, oy, oz, 0);
-            if (!more) break;
-            k = kn;
-            x = xn;
-            j = jn;
-            d = dn;
-        }
-    } else {
-        // the next entry is loaded while the current neighbour is processed, so only the
-        // neighbour's own load stays on each iteration's chain of memory round trips
-        int k = lane;
-        if (k >= cnt) return;
-        int32_t x = entry(k);
-        for (;;) {
-            const int kn = k + TPP;
-            const bool more = kn < cnt;
-            const int32_t xn = more ? entry(kn) : 0;
-            const int j = i + (x >> 9);
-            float ox, oy, oz;
-            off(x, ox, oy, oz);
-            body(j, load(j), ox, oy, oz, 0);
-            if (!more) break;
-            k = kn;
-            x = xn;
-        }
-    }
-}
-
-struct Cand2 {
-    float4 a, b;
-};
-struct Cand3 {
-    float4 a, b, c;
-};
-struct WallCand {
-    float4 a, b, c;
-    int kind;
-};
-// A fluid candidate of the momentum gather on a re-initialisation step: the FP32
-// shadows plus the FP64 volume m/rho and mass of the Shepard sums.
-struct Cand3S {
-    float4 a, b, c;
-    double vol, m;
-};
 
 // -------------------------------------------------------------------- K4 (FP32)
-// LIST (one lane per particle): also records the neighbours within r_cut in nl.
-template <int DIM, int KK, int TPP, bool PF, bool LIST>
-__global__ void k_continuity_f32(const SceneDev* __restrict__ scenes, SortedState st, SortScratch sc, int32_t cap,
-                                 BufferState bf, NbrList nl) {
-    pdl_wait();
-    static_assert(!LIST || TPP <= 2, "the neighbour list is written by one or two lanes per particle");
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / TPP, lane = t % TPP;
-    if (i >= cap || i >= *sc.n_live) return;
-    const int32_t s = st.scene[i];
-    const SceneDev& S = scenes[s];
-    if (!scene_runs(S, sc.scene_step[s])) return;
-    const int32_t* __restrict__ start = sc.start;
-    const float4 ai = st.fa[i];
-    float xi[3], vi[3];
-    if (DIM == 2) {
-        xi[0] = ai.x; xi[1] = ai.y; xi[2] = 0.f;
-        vi[0] = ai.z; vi[1] = ai.w; vi[2] = 0.f;
-    } else {
-        const float4 bi = st.fb[i];
-        xi[0] = ai.x; xi[1] = ai.y; xi[2] = ai.z;
-        vi[0] = bi.x; vi[1] = bi.y; vi[2] = bi.z;
-    }
-    int32_t c[3];
-    decode_cell(st.cell[i], S, c);
-    Kahan drho;
-    int cnt = 0;
-    bool list_ok = !LIST || S.reach <= 3;
-    // lane 0 fills the particle's list from entry 0 up, lane 1 (two-lane writer) from
-    // entry kmax - 1 down; the count word holds both counts (NbrList)
-    int32_t* lp = LIST ? nl.e + (lane == 0 ? (int64_t)0 : (int64_t)(nl.kmax - 1) * nl.stride) + i : nullptr;
-    const int64_t lstep = lane == 0 ? nl.stride : -nl.stride;
-    if (LIST) {  // every candidate lies between the first and the last neighbour row
-        const int m = S.reach;
-        const int zl = DIM == 3 ? max(c[2] - m, 0) : 0, zh = DIM == 3 ? min(c[2] + m, S.n[2] - 1) : 0;
-        const int lo = __ldg(start + S.cell_off + (zl * S.n[1] + max(c[1] - m, 0)) * S.n[0]);
-        const int hi = __ldg(start + S.cell_off + (zh * S.n[1] + min(c[1] + m, S.n[1] - 1) + 1) * S.n[0]);
-        list_ok &= i - lo < kListDelta && hi - i <= kListDelta;
-    }
-    auto load = [&](int j) { return Cand2{st.fa[j], st.fb[j]}; };
-    walk<DIM, TPP, PF>(S, start, c, xi, lane, load, [&](int j, const Cand2& cd, float ox, float oy, float oz, int code) {
-        if (j == i) return;
-        const float4 aj = cd.a;
-        const float4 bj = cd.b;
-        const float rx = xi[0] - ox - aj.x, ry = xi[1] - oy - aj.y;
-        const float rz = DIM == 3 ? xi[2] - oz - aj.z : 0.f;
-        const float d2 = dist2(rx, ry, rz);
-        if (!(d2 <= S.rc2_f)) return;
-        if (LIST) {  // coincident neighbours are listed too: the Shepard sums count them
-            if (cnt < nl.kmax) {
-                *lp = (int32_t)(((uint32_t)(j - i) << 9) | (uint32_t)code);
-                lp += lstep;
-            } else {
-                list_ok = false;
-            }
-            ++cnt;
+// The cells of neighbour row (dy, dz) of a particle, as one run [b, e) of the sorted arrays
+// or two where a periodic axis wraps, in x order; cells beyond r_cut are left out (prune)
+// with the margins and exceptions of coop_select.
+template <int DIM>
+__device__ __forceinline__ void row_runs(const SceneDev& S, const int32_t* __restrict__ start, const int32_t c[3],
+                                         const float4& me, bool prune, int dy, int dz, int& b, int& e, int& b2,
+                                         int& e2) {
+    b = e = b2 = e2 = 0;
+    const int m = S.reach, y = c[1] + dy, z = c[2] + dz;
+    if (dy < -m || dy > m || y < 0 || y >= S.n[1]) return;
+    if (DIM == 3 ? (dz < -m || dz > m || z < 0 || z >= S.n[2]) : dz > 0) return;
+    int x0 = c[0] - m, x1 = c[0] + m;
+    if (prune && y != 0 && y != S.n[1] - 1 && (DIM == 2 || (z != 0 && z != S.n[2] - 1))) {
+        const float gy = fmaxf(fmaxf((float)dy - me.y, me.y - (float)(dy + 1)), 0.f) * S.cell_f[1];
+        float rem = S.rc2_prune - gy * gy;
+        if (DIM == 3) {
+            const float gz = fmaxf(fmaxf((float)dz - me.z, me.z - (float)(dz + 1)), 0.f) * S.cell_f[2];
+            rem -= gz * gz;
         }
-        // a coincident neighbour (d2 == 0) gets 1/r = 0, hence r = 0, dW = 0 and no
-        // continuity term, without a branch in the walk
-        const float inv_r = d2 > 0.f ? rsqrtf(d2) : 0.f;
-        const float r = d2 * inv_r;
-        float W, dW;
-        kernel_wdw_f<KK>(r * S.inv_h_f, S, W, dW);
-        const float s = dW * inv_r;
-        float vx, vy, vz, mj;
-        if (DIM == 2) {
-            vx = vi[0] - aj.z;
-            vy = vi[1] - aj.w;
-            vz = 0.f;
-            mj = bj.x;
-        } else {
-            vx = vi[0] - bj.x;
-            vy = vi[1] - bj.y;
-            vz = vi[2] - bj.z;
-            mj = aj.w;
+        if (rem < 0.f) return;
+        if (!S.periodic_x) {
+            const float w = sqrtf(rem) * S.inv_cell_fx;
+            const int a = c[0] + (int)floorf(me.x - w), q = c[0] + (int)floorf(me.x + w);
+            if (x0 > 0 && a > x0) x0 = min(a, S.n[0] - 1);
+            if (x1 < S.n[0] - 1 && q < x1) x1 = max(q, 0);
         }
-        drho.add(mj * s * (vx * rx + vy * ry + vz * rz));
-    });
-    group_combine<TPP>(drho, group_mask<TPP>());
-    int n_back = 0;  // entries of lane 1 (two-lane writer)
-    if (LIST && TPP == 2) {
-        n_back = __shfl_xor_sync(group_mask<TPP>(), cnt, 1);
-        list_ok &= __shfl_xor_sync(group_mask<TPP>(), (int)list_ok, 1) != 0;
     }
-    if (lane != 0) return;
-    double dr = drho.value();
-    if (LIST) {
-        list_ok &= cnt + n_back <= nl.kmax;
-        nl.n[i] = list_ok ? (cnt | (n_back << 16)) : kListWalk;
+    const int32_t* s = start + S.cell_off + (z * S.n[1] + y) * S.n[0];
+    const int lo = max(x0, 0), hi = min(x1, S.n[0] - 1);
+    if (lo <= hi) {
+        b = __ldg(s + lo);
+        e = __ldg(s + hi + 1);
     }
+    if (S.periodic_x && (x0 < 0 || x1 >= S.n[0])) {
+        b2 = __ldg(s + (x0 < 0 ? x0 + S.n[0] : 0));
+        e2 = __ldg(s + (x0 < 0 ? S.n[0] : x1 - S.n[0] + 1));
+        if (x0 < 0) {  // the wrapped cells come first in x order
+            const int tb = b, te = e;
+            b = b2;
+            e = e2;
+            b2 = tb;
+            e2 = te;
+        }
+        if (b >= e) {  // the first run is empty only where both are
+            b = b2;
+            e = e2;
+            b2 = e2 = 0;
+        }
+    }
+}
+
+// One run of candidates of particle i: those within r_cut are passed to f(j, r, dx + 3, data)
+// with r = x_i - x_j; data = load(j), loaded with the position before the candidate in front
+// of it is tested.
+template <int DIM, typename Load, typename F>
+__device__ __forceinline__ void run_walk(const SceneDev& S, const float4* __restrict__ pos, int i, const float4& me,
+                                         int j, int e, float dyf, float dzf, Load&& load, F&& f) {
+    if (j >= e) return;
+    const float nx = (float)S.n[0];
+    float4 p = __ldg(pos + j);
+    auto data = load(j);
+    for (;;) {
+        const int jn = j + 1;
+        float4 pn = p;
+        auto dn = data;
+        if (jn < e) {
+            pn = __ldg(pos + jn);
+            dn = load(jn);
+        }
+        float cx = me.w - p.w;
+        if (S.periodic_x) cx = cx > 0.5f * nx ? cx - nx : (cx < -0.5f * nx ? cx + nx : cx);
+        const float rx = ((me.x - p.x) + cx) * S.cell_f[0];
+        const float ry = ((me.y - p.y) - dyf) * S.cell_f[1];
+        const float rz = DIM == 3 ? ((me.z - p.z) - dzf) * S.cell_f[2] : 0.f;
+        if (dist2(rx, ry, rz) <= S.rc2_f && j != i)
+            f(j, make_float4(rx, ry, rz, __int_as_float(j)), __float_as_int((8388608.f + 3.f) - cx) & 7, data);
+        if (jn >= e) return;
+        j = jn;
+        p = pn;
+        data = dn;
+    }
+}
+
+// The continuity terms of a run into `sum`, each neighbour listed by emit(code).
+template <int DIM, int KK, typename Emit>
+__device__ __forceinline__ void run_pairs(const SceneDev& S, const SortedState& st, int i, const float4& me,
+                                          const float4& vi, int j, int e, float dyf, float dzf, int tag, Kahan& sum,
+                                          Emit&& emit) {
+    run_walk<DIM>(S, st.fa, i, me, j, e, dyf, dzf, [&](int q) { return __ldg(st.fb + q); },
+                  [&](int q, const float4& r, int dx3, const float4& v) {
+                      emit((int32_t)((uint32_t)(q - i) << 9) | tag | dx3);
+                      const PairF<DIM, KK> p(r, S);
+                      float dot = __fmaf_rn(__fsub_rn(vi.x, v.x), r.x, __fmul_rn(__fsub_rn(vi.y, v.y), r.y));
+                      if (DIM == 3) dot = __fmaf_rn(__fsub_rn(vi.z, v.z), r.z, dot);
+                      sum.add(__fmul_rn(__fmul_rn(v.w, p.F), dot));
+                  });
+}
+
+// Whether every neighbour of particle i fits a list entry (23 bits of j - i).
+template <int DIM>
+__device__ __forceinline__ bool entries_fit(const SceneDev& S, const int32_t* __restrict__ start, const int32_t c[3],
+                                            int i) {
+    const int m = S.reach;
+    const int zl = DIM == 3 ? max(c[2] - m, 0) : 0, zh = DIM == 3 ? min(c[2] + m, S.n[2] - 1) : 0;
+    const int32_t* s = start + S.cell_off;
+    const int lo = __ldg(s + (zl * S.n[1] + max(c[1] - m, 0)) * S.n[0]);
+    const int hi = __ldg(s + (zh * S.n[1] + min(c[1] + m, S.n[1] - 1) + 1) * S.n[0]);
+    return i - lo < kListDelta && hi - i < kListDelta;
+}
+
+// The density update and equation of state of particle i with its continuity sum.
+template <int DIM, int KK>
+__device__ __forceinline__ void continuity_update(const SceneDev& S, const SortedState& st, const BufferState& bf,
+                                                  int i, float2 sum) {
+    double dr = (double)sum.x - (double)sum.y;
     if (bf.n) {  // inlet/outlet buffer neighbours, FP64
         using V = typename VecT<DIM>::T;
+        int32_t c[3];
+        decode_cell(st.cell[i], S, c);
         dr += buffer_drho<DIM, KK>(S, bf, c, ((const V*)st.x)[i], ((const V*)st.v)[i]);
     }
-    // Tait equation of state (UpdatePressure.jl:8-16) with one FP64 division and plain
-    // powers: FP64 is slow on GB300, and these values feed FP32 pair terms (P, c) or FP64
-    // sums (vol) where their last-bit differences from the reference's rounding do not show.
-    // (Evaluated in FP32 instead, on the relative change rho/rho0 - 1, it took 4 more
-    // registers and fewer resident warps: slower on GB300.)
-    // loads first: stores to the state arrays would otherwise order them (possible aliasing)
-    double rho = st.rho[i];
+    // Tait equation of state (UpdatePressure.jl:8-16) in FP64 with one reciprocal and plain
+    // powers: the values feed FP32 pair terms (P) or FP64 sums (vol), where last-bit
+    // differences from the reference's rounding do not show.
     const double m_i = st.m[i];
-    const float4 fb_i = st.fb[i];
-    const float4 fc_i = DIM == 3 ? st.fc[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    rho += dr * S.dt;
-    const double inv_rho = 1.0 / rho;
+    const double rho = fma(dr, S.dt, st.rho[i]);
+    const double inv_rho = rcp_rn_range(rho) ? rcp3(rho) : 1.0 / rho;
     const double rr = rho * S.inv_rho0;
-    const double p = S.b * (powi_plain(rr, S.gamma) - 1.0) + S.p0;
+    const double p = fma(S.b, powi_plain(rr, S.gamma) - 1.0, S.p0);
     const double cs =
         S.c0 * ((S.gamma & 1) ? powi_plain(rr, (S.gamma - 1) >> 1) : sqrt(powi_plain(rr, S.gamma - 1)));
     const double P = p * inv_rho * inv_rho;
@@ -566,280 +288,362 @@ __global__ void k_continuity_f32(const SceneDev* __restrict__ scenes, SortedStat
     st.c[i] = cs;
     st.P[i] = P;
     st.vol[i] = m_i * inv_rho;
-    if (DIM == 2) {
-        st.fb[i] = make_float4(fb_i.x, (float)rho, (float)P, fb_i.w);
-    } else {
-        st.fb[i] = make_float4(fb_i.x, fb_i.y, fb_i.z, (float)rho);
-        st.fc[i] = make_float4((float)P, fc_i.y, fc_i.z, fc_i.w);
+    *reinterpret_cast<float2*>(st.fc + i) = make_float2((float)rho, (float)P);
+}
+
+// Large scenes: one thread a particle.  A row's terms are one compensated sum and the rows'
+// sums are merged in order; k_continuity_rows_f32 forms the same sums with a lane a row.
+template <int DIM, int KK>
+__global__ void __launch_bounds__(128) k_continuity_f32(const SceneDev* __restrict__ scenes, SortedState st,
+                                                        SortScratch sc, int32_t cap, BufferState bf, NbrList nl,
+                                                        WallState wl) {
+    pdl_wait();
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cap || i >= *sc.n_live) return;
+    const SceneDev& S = scenes[st.scene[i]];
+    if (!scene_runs(S, sc.scene_step[st.scene[i]])) return;
+    const float4 me = st.fa[i], vi = st.fb[i];
+    int32_t c[3];
+    decode_cell(st.cell[i], S, c);
+    const int zr = DIM == 3 ? S.reach : 0;
+    const bool prune = S.prune && !select_far(me);
+    const bool fits = nl.e && entries_fit<DIM>(S, sc.start, c, i);
+    const int room = fits ? nl.kmax : 0;
+    int32_t* entry = nl.e + i;
+    int cnt = 0;
+    bool listed_all = fits;
+    Kahan total;
+    auto emit = [&](int32_t code) {
+        if (cnt < room) {
+            *entry = code;
+            entry += nl.stride;
+        }
+        ++cnt;
+    };
+    int b, e, b2, e2;
+    row_runs<DIM>(S, sc.start, c, me, prune, -S.reach, -zr, b, e, b2, e2);
+#pragma unroll 1
+    for (int dz = -zr; dz <= zr; ++dz) {
+#pragma unroll 1
+        for (int dy = -S.reach; dy <= S.reach; ++dy) {
+            int nb, ne, nb2, ne2;  // the next row's runs, loaded before this row is walked
+            const bool turn = dy == S.reach;
+            row_runs<DIM>(S, sc.start, c, me, prune, turn ? -S.reach : dy + 1, turn ? (DIM == 3 ? dz + 1 : 4) : dz, nb,
+                          ne, nb2, ne2);
+            Kahan row;
+            const int before = cnt;
+            const int tag = (dz + 3) << 6 | (dy + 3) << 3;
+#pragma unroll 1
+            while (b < e) {
+                run_pairs<DIM, KK>(S, st, i, me, vi, b, e, (float)dy, (float)dz, tag, row, emit);
+                b = b2;
+                e = e2;
+                b2 = e2 = 0;
+            }
+            merge(total, row.s, row.c);
+            listed_all &= cnt - before <= kRowEntries;
+            b = nb;
+            e = ne;
+            b2 = nb2;
+            e2 = ne2;
+        }
     }
+    const bool walk = !(listed_all && cnt <= room);
+    if (nl.e) nl.n[i] = walk ? kListWalk : cnt;
+    if (walk || (wl.n > 0 && wl.near[st.cell[i]])) sc.walked[atomicAdd(sc.n_walked, 1)] = i;
+    continuity_update<DIM, KK>(S, st, bf, i, make_float2(total.s, total.c));
+}
+
+// Small scenes: eight lanes a particle, lane r the row dy = r - 3 of each plane, so the chain
+// of loads a particle waits for is a row's instead of the whole stencil's.  A block of 256
+// threads takes 32 particles; its first warp updates them.
+template <int DIM, int KK>
+__global__ void __launch_bounds__(256) k_continuity_rows_f32(const SceneDev* __restrict__ scenes, SortedState st,
+                                                             SortScratch sc, int32_t cap, BufferState bf, NbrList nl) {
+    pdl_wait();
+    const unsigned full = 0xffffffffu;
+    __shared__ int32_t rows[kRowEntries * 256];
+    __shared__ float2 sums[32];
+    const int g = threadIdx.x / kCoopLanes, lane = threadIdx.x % kCoopLanes;
+    const int i0 = blockIdx.x * (blockDim.x / kCoopLanes);
+    const int n = min(cap, *sc.n_live);
+    if (i0 >= n) return;  // the whole block
+    {
+        const int i = min(i0 + g, n - 1);
+        const SceneDev& S = scenes[st.scene[i]];
+        const bool on = i0 + g < n && scene_runs(S, sc.scene_step[st.scene[i]]);
+        const float4 me = st.fa[i], vi = st.fb[i];
+        int32_t c[3];
+        decode_cell(st.cell[i], S, c);
+        const bool prune = S.prune && !select_far(me);
+        bool fits = on && nl.e && entries_fit<DIM>(S, sc.start, c, i);
+        int32_t* mine = rows + threadIdx.x;
+        int count = 0;
+        Kahan total;
+        const int planes = DIM == 3 ? (int)__reduce_max_sync(full, (unsigned)S.reach) : 0;
+        for (int dz = -planes; dz <= planes; ++dz) {
+            const int dy = lane - 3;
+            int b = 0, e = 0, b2 = 0, e2 = 0, cnt = 0;
+            if (on && lane < 7) row_runs<DIM>(S, sc.start, c, me, prune, dy, dz, b, e, b2, e2);
+            Kahan row;
+            const int tag = (dz + 3) << 6 | lane << 3;
+#pragma unroll 1
+            while (b < e) {
+                run_pairs<DIM, KK>(S, st, i, me, vi, b, e, (float)dy, (float)dz, tag, row, [&](int32_t code) {
+                    if (cnt < kRowEntries) mine[cnt * 256] = code;
+                    ++cnt;
+                });
+                b = b2;
+                e = e2;
+                b2 = e2 = 0;
+            }
+            __syncwarp(full);
+#pragma unroll
+            for (int r = 0; r < 7; ++r) {  // the rows' sums in order, in every lane
+                const float s = __shfl_sync(full, row.s, r, kCoopLanes), k = __shfl_sync(full, row.c, r, kCoopLanes);
+                merge(total, s, k);
+            }
+            int end = cnt;  // the places of the rows' entries in the list
+#pragma unroll
+            for (int o = 1; o < kCoopLanes; o <<= 1) {
+                const int v = __shfl_up_sync(full, end, o, kCoopLanes);
+                if (lane >= o) end += v;
+            }
+            const int all = __shfl_sync(full, end, kCoopLanes - 1, kCoopLanes);
+            const bool small = __ballot_sync(full, cnt > kRowEntries) >> ((threadIdx.x & 31) - lane) << 24 == 0;
+            fits &= small && count + all <= nl.kmax;
+            if (fits)
+                for (int q = 0; q < cnt; ++q) nl.e[(int64_t)(count + end - cnt + q) * nl.stride + i] = mine[q * 256];
+            count += all;
+        }
+        if (lane == 0) {
+            sums[g] = make_float2(total.s, total.c);
+            if (on && nl.e) nl.n[i] = fits ? count : kListWalk;
+        }
+    }
+    __syncthreads();
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= blockDim.x / kCoopLanes || i >= n) return;
+    const SceneDev& S = scenes[st.scene[i]];
+    if (!scene_runs(S, sc.scene_step[st.scene[i]])) return;
+    continuity_update<DIM, KK>(S, st, bf, i, sums[threadIdx.x]);
 }
 
 // -------------------------------------------------------------------- K5 (FP32)
-// The walks without software pipelining are held to 64 registers (1024 threads x 64 =
-// one SM's register file): 32 resident warps instead of 24 hide more of the dependent
-// neighbour loads on large scenes (about 10% faster at 1M particles), at the cost of a
-// few spilled bytes in the thermal variant.  The pipelined walk keeps its registers (its
-// prefetched candidate would spill) and is therefore limited to blocks of 256 threads.
-// LIST: the fluid neighbours come from the list the continuity gather recorded (the
-// cell walk for a particle whose list did not fit).
-// SHEP: the momentum gather of density re-initialisation steps.  It takes the particles
-// of the scenes whose step re-initialises (every running scene when `sel` is set): the
-// fluid walk also sums W m_j/rho_j and W m_j (ReconstructValue.jl:28-50) in FP64, and the
-// particle's density leaves the step as the Shepard quotient instead of the continuity
-// update.  Without SHEP, `sel` set leaves those particles to the SHEP launch of the same
-// step (a batch whose scenes re-initialise at different steps runs both): every particle
-// goes through the kernel of its own scene's step kind, so a scene's result does not
-// depend on the other scenes of its batch.
-template <int DIM, int KK, int MODE, int TPP, bool PF, bool LIST, bool SHEP>
-__global__ void __launch_bounds__(PF ? 256 : 1024) k_momentum_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl,
-                               SortScratch sc, int32_t cap, BufferState bf, BufferScratch bs, BufferRules br,
-                               NbrList nl, int sel) {
-    pdl_wait();
-    using V = typename VecT<DIM>::T;
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    const int i = t / TPP, lane = t % TPP;
-    if (i >= cap || i >= *sc.n_live) return;
-    const int32_t s = st.scene[i];
-    const SceneDev& S = scenes[s];
-    const int64_t step_s = sc.scene_step[s];
-    const bool runs = scene_runs(S, step_s);
-    const bool reinit_scene = runs && is_step(step_s, S.reinit_interval);
-    if constexpr (SHEP) {
-        if (!(runs && (sel || reinit_scene))) return;
-    } else {
-        if (sel && reinit_scene) return;
+// A particle's own FP32 values in the momentum terms.
+struct SelfF {
+    float4 x, v, f;  // select_pos; (velocity, m kg_a / h); (rho, P, T, kappa)
+    float inv_cp2;   // 2 / cp
+    float tens;      // 0.01 kw_a / W(gap_i)
+    double gap;      // read when the gaps differ
+};
+// The sums of a particle or of one of its lanes.
+template <int DIM, bool HEAT>
+struct SumsF {
+    Kahan dv[DIM], dT;
+    __device__ __forceinline__ void add(const float t[DIM + 1]) {
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) dv[k].add(t[k]);
+        if (HEAT) dT.add(t[DIM]);
     }
-    if (!runs) {
-        if (lane == 0) carry_frozen<DIM>(i, S, st, nx, sc);
-        return;
+    __device__ __forceinline__ void merge_in(const SumsF& o) {
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) merge(dv[k], o.dv[k].s, o.dv[k].c);
+        if (HEAT) merge(dT, o.dT.s, o.dT.c);
     }
-    const float4 ai = st.fa[i];
-    const float4 bi = st.fb[i];
-    float xi[3], vi[3], m_i, rho_i, P_i, gap_i;
-    float T_i = 0.f, kap_i = 0.f, cp_i = 1.f;
-    if (DIM == 2) {
-        xi[0] = ai.x; xi[1] = ai.y; xi[2] = 0.f;
-        vi[0] = ai.z; vi[1] = ai.w; vi[2] = 0.f;
-        m_i = bi.x; rho_i = bi.y; P_i = bi.z; gap_i = bi.w;
-        if (MODE == kModeThermal) {
-            const float4 ci = st.fc[i];
-            T_i = ci.x; kap_i = ci.y; cp_i = ci.z;
+};
+
+template <int DIM, int KK, bool HEAT>
+__device__ __forceinline__ SelfF self_f(const SceneDev& S, const SortedState& st, int i) {
+    SelfF a;
+    a.x = st.fa[i];
+    a.v = st.fb[i];
+    a.f = st.fc[i];
+    a.inv_cp2 = HEAT ? 2.f / (float)st.cp[i] : 0.f;
+    a.gap = 0.0;
+    a.tens = S.tens_f;
+    if (!S.uniform_gap) {
+        a.gap = st.gap[i];
+        a.tens = 0.01f / kernel_w_f<KK>((float)a.gap * S.inv_h_f);
+    }
+    return a;
+}
+
+// Terms of a fluid pair: acceleration t[0 .. DIM-1] and heating t[DIM]; returns w (W / kw_a).
+// Pressure with its tensile part (PressureForce.jl:14-19), viscosity (ViscosityForce.jl:15-23;
+// mu_i + mu_j = nu0 (rho_i + rho_j)), heat (ThermalConduction.jl:15-21).
+template <int DIM, int KK, bool HEAT>
+__device__ __forceinline__ float pair_terms(const SceneDev& S, const SortedState& st, const SelfF& a, const float4& r,
+                                            const float4& vj, const float4& fj, float t[DIM + 1]) {
+    const PairF<DIM, KK> p(r, S);
+    float prho2 = __fadd_rn(a.f.y, fj.y);
+    const float tens =
+        S.uniform_gap ? S.tens_f : 0.01f / kernel_w_f<KK>((float)(0.5 * (a.gap + st.gap[p.j])) * S.inv_h_f);
+    prho2 = __fmaf_rn(__fmul_rn(fabsf(prho2), p.w), tens, prho2);
+    const float mF = __fmul_rn(vj.w, p.F);
+    const float dh = __fadd_rn(p.d2, S.hh001_f);
+    const float mFd = __fmul_rn(mF, p.d2);
+    const float gp = -__fmul_rn(mF, prho2);
+    const float gv = div_ftz(__fmul_rn(mFd, S.nu4_f), __fmul_rn(__fadd_rn(a.f.x, fj.x), dh));
+    t[0] = __fmaf_rn(gp, p.r[0], __fmul_rn(gv, __fsub_rn(a.v.x, vj.x)));
+    t[1] = __fmaf_rn(gp, p.r[1], __fmul_rn(gv, __fsub_rn(a.v.y, vj.y)));
+    if (DIM == 3) t[DIM - 1] = __fmaf_rn(gp, p.r[2], __fmul_rn(gv, __fsub_rn(a.v.z, vj.z)));
+    if (HEAT) {
+        const float keq = div_ftz(__fmul_rn(2.f, __fmul_rn(a.f.w, fj.w)), __fadd_rn(a.f.w, fj.w));
+        const float h = div_ftz(__fmul_rn(mFd, keq), __fmul_rn(__fmul_rn(a.f.x, fj.x), dh));
+        t[DIM] = __fmul_rn(__fmul_rn(h, __fsub_rn(a.f.z, fj.z)), a.inv_cp2);
+    }
+    return p.w;
+}
+
+// A neighbour's terms of the Shepard sums (ReconstructValue.jl:28-50), FP64; w = W / kw_a.
+__device__ __forceinline__ void shepard_terms(const SceneDev& S, const SortedState& st, float w, int j, double& sw,
+                                              double& sws) {
+    const double W = (double)__fmul_rn(S.kw_a_f, w);
+    sw = fma(W, st.vol[j], sw);
+    sws = fma(W, st.m[j], sws);
+}
+
+// Terms of a wall pair: the compulsive force (WallForce.jl:15-28), background pressure
+// (PressureForce.jl:29-33), viscosity (ViscosityForce.jl:34-44), heat (ThermalConduction.jl:
+// 31-35).
+template <int DIM, int KK, int MODE>
+__device__ __forceinline__ void wall_terms(const SceneDev& S, const WallState& wl, const SelfF& a, float c_i,
+                                           const float4& r, float t[DIM + 1]) {
+    constexpr bool HEAT = MODE == kModeThermal;
+    const PairF<DIM, KK> p(r, S);
+    const float4 wn = wl.fb[p.j], wv = wl.fc[p.j];  // (normal, gap), (velocity, T)
+    const float gw = wn.w;
+    const float v0 = __fsub_rn(a.v.x, wv.x), v1 = __fsub_rn(a.v.y, wv.y), v2 = DIM == 3 ? __fsub_rn(a.v.z, wv.z) : 0.f;
+    float vert = __fmaf_rn(v0, wn.x, __fmul_rn(v1, wn.y)), psi = __fmaf_rn(p.r[0], wn.x, __fmul_rn(p.r[1], wn.y));
+    if (DIM == 3) {
+        vert = __fmaf_rn(v2, wn.z, vert);
+        psi = __fmaf_rn(p.r[2], wn.z, psi);
+    }
+    psi = fabsf(psi);
+    float wf = 0.f;
+    const float along = sqrtf(fmaxf(__fmaf_rn(-psi, psi, p.d2), 0.f));
+    const float q = psi / gw;
+    if (!(q > 1.f || along > gw)) {
+        const float pxi = fabsf(__fmul_rn(__fadd_rn(1.f, cospif(along / gw)), 0.5f));
+        const float beta = vert > 0.f ? 0.f : c_i;
+        wf = __fmul_rn(__fmul_rn(__fmul_rn(__fmaf_rn(beta, fabsf(vert), __fmul_rn(0.01f, __fmul_rn(c_i, c_i))), S.inv_h_f),
+                                 fabsf(__fsub_rn(1.f, q))),
+                       __fmul_rn(rsqrtf(q), pxi));
+    }
+    const float mF = __fmul_rn(a.v.w, p.F);
+    float gp = 0.f;
+    if (MODE == kModeWallPressure || HEAT) {
+        const float pw = __fadd_rn(a.f.y, S.P_bg_f);
+        gp = -__fmul_rn(__fmaf_rn(__fmul_rn(fabsf(pw), p.w), a.tens, pw), mF);
+    }
+    const float mFd = __fmul_rn(mF, p.d2);
+    const float den = __fmul_rn(a.f.x, __fadd_rn(p.d2, S.hh001_f));
+    const float gv = div_ftz(__fmul_rn(__fmul_rn(0.5f, S.nu4_f), mFd), den);
+    const float along_n = __fmaf_rn(-gv, vert, wf);
+    t[0] = __fmaf_rn(along_n, wn.x, __fmaf_rn(gp, p.r[0], __fmul_rn(gv, v0)));
+    t[1] = __fmaf_rn(along_n, wn.y, __fmaf_rn(gp, p.r[1], __fmul_rn(gv, v1)));
+    if (DIM == 3) t[DIM - 1] = __fmaf_rn(along_n, wn.z, __fmaf_rn(gp, p.r[2], __fmul_rn(gv, v2)));
+    if (HEAT) {
+        t[DIM] = 0.f;
+        if (wl.kind[p.j] == SPH_WALL_THERMOSTATIC) {
+            const float k = __fmul_rn(__fmul_rn(S.inv_cp_f, __fadd_rn(a.f.w, wl.fk[p.j])), S.inv_rho0_f);
+            t[DIM] = __fmul_rn(div_ftz(__fmul_rn(k, mFd), den), __fsub_rn(a.f.z, wv.w));
         }
-    } else {
-        xi[0] = ai.x; xi[1] = ai.y; xi[2] = ai.z; m_i = ai.w;
-        vi[0] = bi.x; vi[1] = bi.y; vi[2] = bi.z; rho_i = bi.w;
-        const float4 ci = st.fc[i];
-        P_i = ci.x; gap_i = ci.y;
-        if (MODE == kModeThermal) {
-            T_i = ci.z; kap_i = ci.w; cp_i = st.fd[i];
-        }
     }
-    const float c_i = (float)st.c[i];
-    const float mu_i = S.nu0_f * rho_i;
-    const float inv_h = S.inv_h_f;
-    const float inv_Wg_i = 1.f / kernel_w_f<KK>(gap_i * inv_h, S);
-    const float inv_cp_i = 1.f / cp_i;
+}
+
+// The cell walks of the momentum gather: the walls, and the fluid of a particle whose list did
+// not fit (`walk`).  The eight lanes of a group walk for its particle i, lane r the rows
+// dy = r - 3 of every plane, and merge their sums in order: every lane of the group ends with
+// `fluid` and `wall` whole.  shepard(w, j) takes a fluid neighbour's Shepard terms.  All lanes
+// of the warp call this together.
+template <int DIM, int KK, int MODE, typename Shepard>
+__device__ __forceinline__ void coop_rows(const SceneDev& S, const SortedState& st, const WallState& wl,
+                                          const int32_t* __restrict__ start, int i, const SelfF& a, bool walk,
+                                          bool walls, SumsF<DIM, MODE == kModeThermal>& fluid,
+                                          SumsF<DIM, MODE == kModeThermal>& wall, Shepard&& shepard) {
+    constexpr bool HEAT = MODE == kModeThermal;
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & (kCoopLanes - 1), dy = lane - 3;
     int32_t c[3];
     decode_cell(st.cell[i], S, c);
-    Kahan dv[3], dT;
-    double sw = 0.0, sws = 0.0;  // Shepard sums (FP64)
-
-    // every load of a candidate is issued before its distance test (one memory round
-    // trip per candidate), and before the previous candidate is processed
-    using CandF = std::conditional_t<SHEP, Cand3S, Cand3>;
-    auto load_f = [&](int j) {
-        CandF d;
-        d.a = st.fa[j];
-        d.b = st.fb[j];
-        d.c = (DIM == 3 || MODE == kModeThermal) ? st.fc[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-        if constexpr (SHEP) {
-            d.vol = st.vol[j];
-            d.m = st.m[j];
-        }
-        return d;
-    };
-    auto pair = [&](int j, const CandF& cd, float ox, float oy, float oz, int) {
-        if (j == i) return;
-        const float4 aj = cd.a;
-        const float4 bj = cd.b;
-        const float4 cj = cd.c;
-        const float rx = xi[0] - ox - aj.x, ry = xi[1] - oy - aj.y;
-        const float rz = DIM == 3 ? xi[2] - oz - aj.z : 0.f;
-        const float d2 = dist2(rx, ry, rz);
-        if (!(d2 <= S.rc2_f)) return;
-        if (d2 == 0.f) {  // a coincident neighbour: no force, W(0) in the Shepard sums
-            if constexpr (SHEP) {
-                const double W0 = (double)kernel_w_f<KK>(0.f, S);
-                sw += W0 * cd.vol;
-                sws += W0 * cd.m;
-            }
-            return;
-        }
-        const float inv_r = rsqrtf(d2);
-        const float r = d2 * inv_r;
-        float W, dW;
-        kernel_wdw_f<KK>(r * inv_h, S, W, dW);
-        if constexpr (SHEP) {
-            sw += (double)W * cd.vol;
-            sws += (double)W * cd.m;
-        }
-        float vx, vy, vz, m_j, rho_j, P_j, gap_j;
-        float T_j = 0.f, kap_j = 0.f;
-        if (DIM == 2) {
-            vx = vi[0] - aj.z; vy = vi[1] - aj.w; vz = 0.f;
-            m_j = bj.x; rho_j = bj.y; P_j = bj.z; gap_j = bj.w;
-            if (MODE == kModeThermal) {
-                T_j = cj.x; kap_j = cj.y;
-            }
-        } else {
-            vx = vi[0] - bj.x; vy = vi[1] - bj.y; vz = vi[2] - bj.z;
-            m_j = aj.w; rho_j = bj.w;
-            P_j = cj.x; gap_j = cj.y;
-            if (MODE == kModeThermal) {
-                T_j = cj.z; kap_j = cj.w;
-            }
-        }
-        // pressure (PressureForce.jl:14-19), tensile term included
-        float prho2 = P_i + P_j;
-        const float inv_Wg = S.uniform_gap ? inv_Wg_i : 1.f / kernel_w_f<KK>(0.5f * (gap_i + gap_j) * inv_h, S);
-        prho2 += fabsf(prho2) * 0.01f * W * inv_Wg;
-        // viscosity (ViscosityForce.jl:15-23)
-        const float sum_rho = rho_i + rho_j;
-        const float f = __fdividef(4.f * (mu_i + S.nu0_f * rho_j) * r * dW, sum_rho * sum_rho * (r * r + S.hh001_f));
-        const float gp = -m_j * prho2 * dW * inv_r;  // pressure term along r_vec
-        const float gv = m_j * f;                    // viscosity term along v_ij
-        dv[0].add(gp * rx + gv * vx);
-        dv[1].add(gp * ry + gv * vy);
-        if (DIM == 3) dv[2].add(gp * rz + gv * vz);
-        if (MODE == kModeThermal) {  // ThermalConduction.jl:15-21
-            const float keq = __fdividef(2.f * kap_i * kap_j, kap_i + kap_j);
-            const float dq = __fdividef(2.f * keq * r * dW, rho_i * rho_j * (r * r + S.hh001_f)) * (T_i - T_j);
-            dT.add(dq * m_j * inv_cp_i);
+    const bool prune = S.prune && !select_far(a.x);
+    const float c_i = (float)st.c[i];
+    const int planes = DIM == 3 ? (int)__reduce_max_sync(full, walk || walls ? (unsigned)S.reach : 0u) : 0;
+    const bool any_walk = __any_sync(full, walk), any_walls = __any_sync(full, walls);
+    auto rows = [&](const int32_t* starts, const float4* pos, int self, int dz, auto&& term) {
+        int b, e, b2, e2;
+        row_runs<DIM>(S, starts, c, a.x, prune, dy, dz, b, e, b2, e2);
+#pragma unroll 1
+        while (b < e) {
+            run_walk<DIM>(S, pos, self, a.x, b, e, (float)dy, (float)dz, [](int) { return 0; },
+                          [&](int j, const float4& r, int, int) { term(j, r); });
+            b = b2;
+            e = e2;
+            b2 = e2 = 0;
         }
     };
-    if constexpr (LIST) {
-        const int cnt = nl.n[i];
-        if (cnt != kListWalk) walk_list<DIM, TPP, PF>(S, nl, i, cnt, lane, load_f, pair);
-        else walk<DIM, TPP, PF>(S, sc.start, c, xi, lane, load_f, pair);
-    } else {
-        walk<DIM, TPP, PF>(S, sc.start, c, xi, lane, load_f, pair);
+#pragma unroll 1
+    for (int dz = -planes; dz <= planes; ++dz) {
+        if (any_walk && walk && lane < 7)
+            rows(start, st.fa, i, dz, [&](int j, const float4& r) {
+                float t[DIM + 1];
+                shepard(pair_terms<DIM, KK, HEAT>(S, st, a, r, st.fb[j], st.fc[j], t), j);
+                fluid.add(t);
+            });
+        if (any_walls && walls && lane < 7)
+            rows(wl.start, wl.fa, -1, dz, [&](int, const float4& r) {
+                float t[DIM + 1];
+                wall_terms<DIM, KK, MODE>(S, wl, a, c_i, r, t);
+                wall.add(t);
+            });
     }
-
-    if (wl.n > 0 && wl.near[st.cell[i]]) {  // walls only where a wall cell is within reach
-        auto load_w = [&](int w) {
-            WallCand d;
-            d.a = wl.fa[w];
-            d.b = wl.fb[w];
-            d.c = (DIM == 3 || MODE == kModeThermal) ? wl.fc[w] : make_float4(0.f, 0.f, 0.f, 0.f);
-            d.kind = (DIM == 3 && MODE == kModeThermal) ? wl.kind[w] : 0;
-            return d;
-        };
-        walk<DIM, TPP, PF>(S, wl.start, c, xi, lane, load_w, [&](int w, const WallCand& cd, float ox, float oy,
-                                                                   float oz, int) {
-            const float4 wa = cd.a;
-            const float4 wb = cd.b;
-            const float4 wc = cd.c;
-            float rv[3], n[3], vv[3], gw, Tw = 0.f, kw = 0.f;
-            bool thermo = false;
-            if (DIM == 2) {
-                rv[0] = xi[0] - ox - wa.x; rv[1] = xi[1] - oy - wa.y; rv[2] = 0.f;
-                n[0] = wa.z; n[1] = wa.w; n[2] = 0.f;
-                vv[0] = vi[0] - wb.x; vv[1] = vi[1] - wb.y; vv[2] = 0.f;
-                gw = wb.z;
-                if (MODE == kModeThermal) {
-                    Tw = wb.w; kw = wc.x; thermo = wc.y != 0.f;
-                }
-            } else {
-                rv[0] = xi[0] - ox - wa.x; rv[1] = xi[1] - oy - wa.y; rv[2] = xi[2] - oz - wa.z;
-                gw = wa.w;
-                n[0] = wb.x; n[1] = wb.y; n[2] = wb.z;
-                vv[0] = vi[0] - wc.x; vv[1] = vi[1] - wc.y; vv[2] = vi[2] - wc.z;
-                if (MODE == kModeThermal) {
-                    Tw = wb.w; kw = wc.w; thermo = cd.kind == SPH_WALL_THERMOSTATIC;
-                }
-            }
-            const float d2 = rv[0] * rv[0] + rv[1] * rv[1] + rv[2] * rv[2];
-            if (!(d2 <= S.rc2_f)) return;
-            const float inv_r = d2 > 0.f ? rsqrtf(d2) : 0.f;
-            const float r = d2 * inv_r;
-            float W, dW;
-            kernel_wdw_f<KK>(r * inv_h, S, W, dW);
-            const float vert = vv[0] * n[0] + vv[1] * n[1] + vv[2] * n[2];
-            float acc[3] = {0.f, 0.f, 0.f};
-            {  // WallForce.jl:15-28
-                const float psi = fabsf(rv[0] * n[0] + rv[1] * n[1] + rv[2] * n[2]);
-                const float xi_ = sqrtf(fmaxf(r * r - psi * psi, 0.f));
-                const float q = psi / gw;
-                if (!(q > 1.f || xi_ > gw)) {
-                    const float pxi = fabsf((1.f + cospif(xi_ / gw)) * 0.5f);
-                    const float beta = vert > 0.f ? 0.f : 1.f;
-                    const float rpsi =
-                        (0.01f * c_i * c_i + beta * c_i * fabsf(vert)) * inv_h * fabsf(1.f - q) * rsqrtf(q);
-                    const float wf = rpsi * pxi;
-                    acc[0] += wf * n[0];
-                    acc[1] += wf * n[1];
-                    acc[2] += wf * n[2];
-                }
-            }
-            if (MODE == kModeWallPressure || MODE == kModeThermal) {  // PressureForce.jl:29-33
-                float prho2 = P_i + S.P_bg_f;
-                prho2 += fabsf(prho2) * 0.01f * W * inv_Wg_i;
-                const float gp = -m_i * prho2 * dW * inv_r;
-                acc[0] += gp * rv[0];
-                acc[1] += gp * rv[1];
-                acc[2] += gp * rv[2];
-            }
-            {  // ViscosityForce.jl:34-44
-                const float sum_rho = 2.f * rho_i;
-                const float f = __fdividef(8.f * mu_i * r * dW, sum_rho * sum_rho * (r * r + S.hh001_f));
-                const float gv = m_i * f;
-                acc[0] += gv * (vv[0] - vert * n[0]);
-                acc[1] += gv * (vv[1] - vert * n[1]);
-                acc[2] += gv * (vv[2] - vert * n[2]);
-            }
-            dv[0].add(acc[0]);
-            dv[1].add(acc[1]);
-            if (DIM == 3) dv[2].add(acc[2]);
-            if (MODE == kModeThermal && thermo) {  // ThermalConduction.jl:31-35
-                const float dq =
-                    __fdividef(S.inv_cp_f * (kap_i + kw) * r * dW * S.inv_rho0_f, rho_i * (r * r + S.hh001_f)) *
-                    (T_i - Tw);
-                dT.add(dq * m_i);
-            }
-        });
-    }
-
-    const unsigned mask = group_mask<TPP>();
+    __syncwarp(full);
+    auto merged = [&](Kahan& k) {
+        Kahan m;
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) group_combine<TPP>(dv[k], mask);
-    if (MODE == kModeThermal) group_combine<TPP>(dT, mask);
-    if constexpr (SHEP) {
-        sw = group_sum<TPP>(sw, mask);
-        sws = group_sum<TPP>(sws, mask);
-    }
-    if (lane != 0) return;
+        for (int r = 0; r < 7; ++r)
+            merge(m, __shfl_sync(full, k.s, r, kCoopLanes), __shfl_sync(full, k.c, r, kCoopLanes));
+        k = m;
+    };
+    auto merge_all = [&](SumsF<DIM, HEAT>& s) {
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) merged(s.dv[k]);
+        if (HEAT) merged(s.dT);
+    };
+    if (any_walk) merge_all(fluid);
+    if (any_walls) merge_all(wall);
+}
+
+// The update of particle i with its sums: FP64 forward Euler on the masters
+// (UpdateTemperature/Velocity/Position.jl), the re-initialised density with the particle's
+// own W(0) term (SHEP; ReconstructValue.jl:51-55), the out-of-domain check and the next
+// step's cell arrival.
+template <int DIM, int KK, int MODE, bool SHEP>
+__device__ __forceinline__ void momentum_update(const SceneDev& S, const SortedState& st, const NextState& nx,
+                                                const SortScratch& sc, const BufferState& bf, const BufferScratch& bs,
+                                                const BufferRules& br, int i, int64_t step,
+                                                const SumsF<DIM, MODE == kModeThermal>& sum, double sw, double sws) {
+    using V = typename VecT<DIM>::T;
+    constexpr bool HEAT = MODE == kModeThermal;
     double dvd[DIM];
 #pragma unroll
-    for (int k = 0; k < DIM; ++k) dvd[k] = dv[k].value();
-    const double dTd = MODE == kModeThermal ? dT.value() : 0.0;
-
-    // ---- FP64 forward Euler on the masters (UpdateTemperature/Velocity/Position.jl)
-    const int64_t step = sc.scene_step[s];
+    for (int k = 0; k < DIM; ++k) dvd[k] = (double)sum.dv[k].s - (double)sum.dv[k].c;
+    const double dTd = HEAT ? (double)sum.dT.s - (double)sum.dT.c : 0.0;
     const V x0 = ((const V*)st.x)[i];
     const V v0 = ((const V*)st.v)[i];
-    const double rho_d = st.rhoc[i];  // loaded before the stores below (possible aliasing)
-    if constexpr (SHEP) {  // the particle's own W(0) term (ReconstructValue.jl:51-55)
-        sw += S.k0 * st.vol[i];
-        sws += S.k0 * st.m[i];
-    }
+    const double rho_d = st.rhoc[i];
     if (MODE == kModeBuffers && bf.n) {  // inlet/outlet buffer neighbours, FP64
         const double gap_d = st.gap[i];
+        int32_t c[3];
+        decode_cell(st.cell[i], S, c);
         buffer_dv<DIM, KK>(S, bf, c, x0, v0, rho_d, st.P[i], gap_d, kernel_w<KK>(gap_d, S), S.nu0 * rho_d, dvd);
     }
     const double dt = S.dt;
     double body[DIM];
-    if (MODE == kModeThermal) {
-        const double Tn = st.T[i] + dt * dTd;
+    if (HEAT) {
+        const double Tn = fma(dt, dTd, st.T[i]);
 #pragma unroll
         for (int k = 0; k < DIM; ++k) body[k] = S.bous[k] * (Tn - S.t0);
         nx.T[i] = Tn;
@@ -874,7 +678,11 @@ __global__ void __launch_bounds__(PF ? 256 : 1024) k_momentum_f32(const SceneDev
     }
     ((V*)nx.x)[i] = xo;
     ((V*)nx.v)[i] = vo;
-    nx.rho[i] = SHEP ? sws / sw : rho_d;
+    if constexpr (SHEP) {  // with the particle's own W(0) term (ReconstructValue.jl:51-55)
+        nx.rho[i] = (sws + S.k0 * st.m[i]) / (sw + S.k0 * st.vol[i]);
+    } else {
+        nx.rho[i] = rho_d;
+    }
 
     bool finite = bits_finite(rho_d);
 #pragma unroll
@@ -894,79 +702,307 @@ __global__ void __launch_bounds__(PF ? 256 : 1024) k_momentum_f32(const SceneDev
         if (k < bs.cap) bs.pend[k] = i;
         else atomicOr(sc.status, kStatusBufferOverflow);
     } else {
-        cell_arrival(sc, i, cell_key<DIM>(xo, S));
+        cell_arrival(sc, i, moved_key<DIM>(st.cell[i], st.fa[i], x0, xo, S));
     }
+}
+
+// A particle takes part in a momentum launch (SHEP: of re-initialisation steps) when its
+// scene runs and its step is of the launch's kind; `sel`: with SHEP, every running scene;
+// without, the re-initialising scenes are left to the SHEP launch of the same step (a batch
+// whose scenes re-initialise at different steps runs both): every particle goes through the
+// kernel of its own scene's step kind, so a scene's result does not depend on its batch.
+template <bool SHEP>
+__device__ __forceinline__ bool takes_part(const SceneDev& S, int64_t step, int sel) {
+    const bool runs = scene_runs(S, step);
+    if (SHEP) return runs && (sel || is_step(step, S.reinit_interval));
+    return runs && !(sel && is_step(step, S.reinit_interval));
+}
+
+// Large scenes, the cell walks: eight lanes for each particle that continuity listed as
+// walked (near a wall, or without a list; in any order), their sums into sc.walk_sums for
+// k_momentum_f32.  Walked by that kernel's own threads, a wall cost every lane of a warp with
+// one particle near it, and half the time of a 3D dam break's momentum gather.
+template <int DIM, int KK, int MODE, bool SHEP>
+__global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
+    k_walks_f32(const SceneDev* __restrict__ scenes, SortedState st, WallState wl, SortScratch sc, NbrList nl, int sel) {
+    pdl_wait();
+    constexpr bool HEAT = MODE == kModeThermal;
+    constexpr int kSums = DIM + (HEAT ? 1 : 0);
+    const int n = *sc.n_walked, lane = threadIdx.x % kCoopLanes;
+    const int stride = gridDim.x * (blockDim.x / kCoopLanes);
+    for (int q0 = (blockIdx.x * blockDim.x + (threadIdx.x & ~31)) / kCoopLanes; q0 < n; q0 += stride) {
+        const int q = q0 + (threadIdx.x & 31) / kCoopLanes;
+        const int i = sc.walked[min(q, n - 1)];
+        const SceneDev& S = scenes[st.scene[i]];
+        const bool on = q < n && takes_part<SHEP>(S, sc.scene_step[st.scene[i]], sel);
+        const bool walk = on && (!nl.e || nl.n[i] == kListWalk), walls = on && wl.n > 0 && wl.near[st.cell[i]];
+        SumsF<DIM, HEAT> fluid, wall;
+        double sw = 0.0, sws = 0.0;
+        coop_rows<DIM, KK, MODE>(S, st, wl, sc.start, i, self_f<DIM, KK, HEAT>(S, st, i), walk, walls, fluid, wall,
+                                 [&](float wk, int j) { if constexpr (SHEP) shepard_terms(S, st, wk, j, sw, sws); });
+        if constexpr (SHEP) {
+            sw = coop_sum(sw);
+            sws = coop_sum(sws);
+        }
+        if (on && lane == 0) {
+            float2* out = sc.walk_sums + (int64_t)i * (2 * kSums + 2);
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) {
+                out[k] = make_float2(fluid.dv[k].s, fluid.dv[k].c);
+                out[kSums + k] = make_float2(wall.dv[k].s, wall.dv[k].c);
+            }
+            if (HEAT) {
+                out[DIM] = make_float2(fluid.dT.s, fluid.dT.c);
+                out[kSums + DIM] = make_float2(wall.dT.s, wall.dT.c);
+            }
+            if constexpr (SHEP) {
+                reinterpret_cast<double*>(out)[2 * kSums] = sw;
+                reinterpret_cast<double*>(out)[2 * kSums + 1] = sws;
+            }
+        }
+    }
+}
+
+// Large scenes: one thread a particle.  Eight sums take the entries of the list in turns, as
+// the lanes of k_momentum_lanes_f32 do, so both give the same bits; a warp's threads read the
+// same entry of 32 consecutive particles, whose neighbours lie side by side.
+template <int DIM, int KK, int MODE, bool SHEP>
+__global__ void __launch_bounds__(128, 4)
+    k_momentum_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl, SortScratch sc,
+                   int32_t cap, BufferState bf, BufferScratch bs, BufferRules br, NbrList nl, int sel) {
+    pdl_wait();
+    constexpr bool HEAT = MODE == kModeThermal;
+    constexpr int kSums = DIM + (HEAT ? 1 : 0);
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= cap || i >= *sc.n_live) return;
+    const SceneDev& S = scenes[st.scene[i]];
+    const int64_t step = sc.scene_step[st.scene[i]];
+    if (!takes_part<SHEP>(S, step, sel)) {
+        if (!SHEP && !scene_runs(S, step)) carry_frozen<DIM>(i, S, st, nx, sc);
+        return;
+    }
+    const SelfF a = self_f<DIM, KK, HEAT>(S, st, i);
+    const int count = nl.e ? nl.n[i] : kListWalk;
+    SumsF<DIM, HEAT> acc[kCoopLanes];
+    if (count != kListWalk) {
+        // the next eight entries are loaded before the current eight are processed
+        const int32_t* entry = nl.e + i;
+        const int64_t stride = nl.stride;
+        int32_t next[kCoopLanes];
+#pragma unroll
+        for (int u = 0; u < kCoopLanes; ++u) next[u] = u < count ? __ldg(entry + u * stride) : 0;
+#pragma unroll 1
+        for (int k = 0; k < count; k += kCoopLanes) {
+            int32_t code[kCoopLanes];
+#pragma unroll
+            for (int u = 0; u < kCoopLanes; ++u) {
+                code[u] = next[u];
+                next[u] = k + kCoopLanes + u < count ? __ldg(entry + (k + kCoopLanes + u) * stride) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < kCoopLanes; ++u) {
+                const int j = i + (code[u] >> 9);
+                const float4 r = listed<DIM>(code[u], a.x, __ldg(st.fa + j), j, S);
+                float t[DIM + 1];
+                pair_terms<DIM, KK, HEAT>(S, st, a, r, __ldg(st.fb + j), __ldg(st.fc + j), t);
+                if (k + u < count) acc[u].add(t);
+            }
+        }
+    }
+#pragma unroll
+    for (int u = 1; u < kCoopLanes; ++u) acc[0].merge_in(acc[u]);
+    double sw = 0.0, sws = 0.0;
+    if constexpr (SHEP) {  // the Shepard sums, in a second pass over the list
+        double w8[kCoopLanes] = {}, ws8[kCoopLanes] = {};
+        const int32_t* entry = nl.e + i;
+        const int entries = count != kListWalk ? count : 0;
+#pragma unroll 1
+        for (int k = 0; k < entries; k += kCoopLanes)
+#pragma unroll
+            for (int u = 0; u < kCoopLanes; ++u) {
+                const int32_t code = k + u < entries ? __ldg(entry + (k + u) * nl.stride) : 0;
+                const int j = i + (code >> 9);
+                const PairF<DIM, KK> p(listed<DIM>(code, a.x, __ldg(st.fa + j), j, S), S);
+                if (k + u < entries) shepard_terms(S, st, p.w, j, w8[u], ws8[u]);
+            }
+        // (the order of coop_sum)
+        sw = ((w8[0] + w8[1]) + (w8[2] + w8[3])) + ((w8[4] + w8[5]) + (w8[6] + w8[7]));
+        sws = ((ws8[0] + ws8[1]) + (ws8[2] + ws8[3])) + ((ws8[4] + ws8[5]) + (ws8[6] + ws8[7]));
+    }
+    if (count == kListWalk || (wl.n > 0 && wl.near[st.cell[i]])) {  // the cell walks (k_walks_f32)
+        const float2* in = sc.walk_sums + (int64_t)i * (2 * kSums + 2);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+#pragma unroll
+            for (int k = 0; k < DIM; ++k) merge(acc[0].dv[k], in[h * kSums + k].x, in[h * kSums + k].y);
+            if (HEAT) merge(acc[0].dT, in[h * kSums + DIM].x, in[h * kSums + DIM].y);
+        }
+        if (SHEP && count == kListWalk) {
+            sw = reinterpret_cast<const double*>(in)[2 * kSums];
+            sws = reinterpret_cast<const double*>(in)[2 * kSums + 1];
+        }
+    }
+    momentum_update<DIM, KK, MODE, SHEP>(S, st, nx, sc, bf, bs, br, i, step, acc[0], sw, sws);
+}
+
+// Small scenes: eight lanes a particle, lane t the
+// entries t, t + 8, ... of its list, or a neighbour row of the walls (and of the fluid, for a
+// particle whose list did not fit).  A block of 256 threads takes 32 particles; its first
+// warp merges the lanes' sums and updates the particles.
+template <int DIM, int KK, int MODE, bool SHEP>
+__global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
+    k_momentum_lanes_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl,
+                         SortScratch sc, int32_t cap, BufferState bf, BufferScratch bs, BufferRules br, NbrList nl,
+                         int sel) {
+    pdl_wait();
+    constexpr bool HEAT = MODE == kModeThermal;
+    constexpr int kSums = DIM + (HEAT ? 1 : 0), kParts = kCoopLanes + 1;
+    const unsigned full = 0xffffffffu;
+    __shared__ float2 sums[kSums * kParts * kSumStride];
+    __shared__ double shep[SHEP ? 64 : 1];
+    const int g = threadIdx.x / kCoopLanes, lane = threadIdx.x % kCoopLanes;
+    const int i0 = blockIdx.x * (blockDim.x / kCoopLanes);
+    const int n = min(cap, *sc.n_live);
+    if (i0 >= n) return;  // the whole block
+    {
+        const int i = min(i0 + g, n - 1);
+        const SceneDev& S = scenes[st.scene[i]];
+        const bool on = i0 + g < n && takes_part<SHEP>(S, sc.scene_step[st.scene[i]], sel);
+        const SelfF a = self_f<DIM, KK, HEAT>(S, st, i);
+        SumsF<DIM, HEAT> sum;
+        double sw = 0.0, sws = 0.0;  // Shepard sums (ReconstructValue.jl:28-50), FP64
+        const int count = on ? (nl.e ? nl.n[i] : kListWalk) : 0;
+        auto shepard = [&](float w, int j) { if constexpr (SHEP) shepard_terms(S, st, w, j, sw, sws); };
+        if (count != kListWalk && lane < count) {
+            // the entry two rounds ahead and the neighbour one round ahead are loaded before the
+            // current pair is processed
+            const int32_t* entry = nl.e + i + lane * nl.stride;
+            const int64_t ahead = kCoopLanes * nl.stride;
+            int32_t code = __ldg(entry), next = 0;
+            if (lane + kCoopLanes < count) next = __ldg(entry += ahead);
+            int j = i + (code >> 9);
+            float4 p = __ldg(st.fa + j), v = __ldg(st.fb + j), f = __ldg(st.fc + j);
+            for (int k = lane;;) {
+                const bool more = k + kCoopLanes < count;
+                const float4 r = listed<DIM>(code, a.x, p, j, S);
+                const float4 vj = v, fj = f;
+                if (more) {
+                    code = next;
+                    j = i + (code >> 9);
+                    p = __ldg(st.fa + j);
+                    v = __ldg(st.fb + j);
+                    f = __ldg(st.fc + j);
+                    if (k + 2 * kCoopLanes < count) next = __ldg(entry += ahead);
+                }
+                float t[DIM + 1];
+                const float w = pair_terms<DIM, KK, HEAT>(S, st, a, r, vj, fj, t);
+                shepard(w, __float_as_int(r.w));
+                sum.add(t);
+                if (!more) break;
+                k += kCoopLanes;
+            }
+        }
+        __syncwarp(full);
+        const bool walk = count == kListWalk, walls = on && wl.n > 0 && wl.near[st.cell[i]];
+        SumsF<DIM, HEAT> wall;
+        if (__any_sync(full, walk || walls)) {
+            SumsF<DIM, HEAT> fluid;
+            coop_rows<DIM, KK, MODE>(S, st, wl, sc.start, i, a, walk, walls, fluid, wall, shepard);
+            if (walk && lane == 0) sum = fluid;
+        }
+        if constexpr (SHEP) {
+            sw = coop_sum(sw);
+            sws = coop_sum(sws);
+        }
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) sums[(k * kParts + lane) * kSumStride + g] = make_float2(sum.dv[k].s, sum.dv[k].c);
+        if (HEAT) sums[(DIM * kParts + lane) * kSumStride + g] = make_float2(sum.dT.s, sum.dT.c);
+        if (lane == 0) {
+#pragma unroll
+            for (int k = 0; k < DIM; ++k)
+                sums[(k * kParts + kCoopLanes) * kSumStride + g] = make_float2(wall.dv[k].s, wall.dv[k].c);
+            if (HEAT) sums[(DIM * kParts + kCoopLanes) * kSumStride + g] = make_float2(wall.dT.s, wall.dT.c);
+            if constexpr (SHEP) {
+                shep[g] = sw;
+                shep[32 + g] = sws;
+            }
+        }
+    }
+    __syncthreads();
+    const int i = i0 + threadIdx.x;
+    if (threadIdx.x >= blockDim.x / kCoopLanes || i >= n) return;
+    const SceneDev& S = scenes[st.scene[i]];
+    const int64_t step = sc.scene_step[st.scene[i]];
+    if (!takes_part<SHEP>(S, step, sel)) {
+        if (!SHEP && !scene_runs(S, step)) carry_frozen<DIM>(i, S, st, nx, sc);
+        return;
+    }
+    auto merged = [&](int k) {
+        const float2* q = sums + k * kParts * kSumStride + threadIdx.x;
+        Kahan t;
+        t.s = q[0].x;
+        t.c = q[0].y;
+#pragma unroll
+        for (int l = 1; l < kParts; ++l) merge(t, q[l * kSumStride].x, q[l * kSumStride].y);
+        return t;
+    };
+    SumsF<DIM, HEAT> sum;
+#pragma unroll
+    for (int k = 0; k < DIM; ++k) sum.dv[k] = merged(k);
+    if (HEAT) sum.dT = merged(DIM);
+    momentum_update<DIM, KK, MODE, SHEP>(S, st, nx, sc, bf, bs, br, i, step, sum, SHEP ? shep[threadIdx.x] : 0.0,
+                                         SHEP ? shep[32 + threadIdx.x] : 0.0);
 }
 
 // -------------------------------------------------------------------- launchers
-// SHEP selects the momentum gather of re-initialisation steps; its instantiations live in
-// translation units of their own (the *_shep.cu files), so the two sets compile in parallel.
-template <int DIM, int KK, int MODE, int TPP, bool PF, bool LIST, bool SHEP>
-void launch_momentum(const LaunchCtx& L, int grid, int block) {
-    launch_dep(k_momentum_f32<DIM, KK, MODE, TPP, PF, LIST, SHEP>, grid, block, L.stream, L.scenes, L.st, L.nx, L.wl,
-               L.sc, L.cap, L.bf, L.bs, L.br, L.nl, SHEP ? L.force_reinit : L.skip_reinit);
+// A lane a row (continuity) and eight lanes a particle (momentum) below this many particles,
+// a thread a particle from there on.
+constexpr int64_t kLanesBelow = 40000;
+
+template <int DIM, int KK, int MODE>
+void launch_momentum(const LaunchCtx& L) {
+    const int sel = L.shepard ? L.force_reinit : L.skip_reinit;
+    if (L.lanes) {
+        auto kernel = L.shepard ? k_momentum_lanes_f32<DIM, KK, MODE, true> : k_momentum_lanes_f32<DIM, KK, MODE, false>;
+        launch_dep(kernel, (L.cap + 31) / 32, 256, L.stream, L.scenes, L.st, L.nx, L.wl, L.sc, L.cap, L.bf, L.bs, L.br,
+                   L.nl, sel);
+        return;
+    }
+    auto walks = L.shepard ? k_walks_f32<DIM, KK, MODE, true> : k_walks_f32<DIM, KK, MODE, false>;
+    launch_dep(walks, 152 * 3, 256, L.stream, L.scenes, L.st, L.wl, L.sc, L.nl, sel);
+    auto kernel = L.shepard ? k_momentum_f32<DIM, KK, MODE, true> : k_momentum_f32<DIM, KK, MODE, false>;
+    launch_dep(kernel, (L.cap + 127) / 128, 128, L.stream, L.scenes, L.st, L.nx, L.wl, L.sc, L.cap, L.bf, L.bs, L.br,
+               L.nl, sel);
 }
 
-template <int DIM, int KK, int TPP, bool PF, bool LIST, bool SHEP>
-void launch_tpp(int stage, int mode, const LaunchCtx& L) {
-    const int block = L.block > 0 ? L.block : 128;
-    const int grid = (int)(((int64_t)L.cap * TPP + block - 1) / block);
+template <int DIM, int KK>
+void launch_kk(int stage, const LaunchCtx& C) {
+    LaunchCtx L = C;
+    if (L.lanes < 0) L.lanes = L.cap < kLanesBelow;
     if (stage == 0) {
-        if constexpr (!SHEP && (!LIST || TPP <= 2))
-            launch_dep(k_continuity_f32<DIM, KK, TPP, PF, LIST>, grid, block, L.stream, L.scenes, L.st, L.sc, L.cap,
+        if (L.lanes)
+            launch_dep(k_continuity_rows_f32<DIM, KK>, (L.cap + 31) / 32, 256, L.stream, L.scenes, L.st, L.sc, L.cap,
                        L.bf, L.nl);
-    } else if (mode == kModeFluidWall) {
-        launch_momentum<DIM, KK, kModeFluidWall, TPP, PF, LIST, SHEP>(L, grid, block);
-    } else if (mode == kModeWallPressure) {
-        launch_momentum<DIM, KK, kModeWallPressure, TPP, PF, LIST, SHEP>(L, grid, block);
-    } else if (mode == kModeBuffers) {
-        launch_momentum<DIM, KK, kModeBuffers, TPP, PF, LIST, SHEP>(L, grid, block);
-    } else {
-        launch_momentum<DIM, KK, kModeThermal, TPP, PF, LIST, SHEP>(L, grid, block);
+        else
+            launch_dep(k_continuity_f32<DIM, KK>, (L.cap + 127) / 128, 128, L.stream, L.scenes, L.st, L.sc, L.cap, L.bf,
+                       L.nl, L.wl);
+        return;
+    }
+    switch (L.mode) {
+        case kModeFluidWall: launch_momentum<DIM, KK, kModeFluidWall>(L); break;
+        case kModeWallPressure: launch_momentum<DIM, KK, kModeWallPressure>(L); break;
+        case kModeBuffers: launch_momentum<DIM, KK, kModeBuffers>(L); break;
+        default: launch_momentum<DIM, KK, kModeThermal>(L);
     }
 }
 
-// Lanes code: 1, 2, 4, 8 lanes per particle; -1: one lane with a software-pipelined
-// candidate loop (pays off when few warps are resident, i.e. small scenes).  The cell
-// walks (LIST false) take every code for every stage; with the neighbour list (LIST
-// true) continuity runs one or two lanes (1, -1 or 2; the two-lane list writer loads
-// each lane's next candidate ahead, as -1 does: on GB300 5-22% faster than without in
-// 2D and 3D) and momentum 1, 2, 4 or -1 lanes (there two pipelined lanes were 30-60%
-// slower: the prefetched candidate of three float4 costs the occupancy).
-template <int DIM, int KK, bool LIST, bool SHEP>
-void launch_kk(int stage, const LaunchCtx& L) {
-    const int tpp = stage == 0 ? L.tpp_continuity : L.tpp_momentum;
-    if constexpr (LIST) {
-        if (stage == 0) {
-            if (tpp == -1) launch_tpp<DIM, KK, 1, true, true, SHEP>(stage, L.mode, L);
-            else if (tpp == 2) launch_tpp<DIM, KK, 2, true, true, SHEP>(stage, L.mode, L);
-            else launch_tpp<DIM, KK, 1, false, true, SHEP>(stage, L.mode, L);
-            return;
-        }
-        switch (tpp) {
-            case -1: launch_tpp<DIM, KK, 1, true, true, SHEP>(stage, L.mode, L); break;
-            case 1: launch_tpp<DIM, KK, 1, false, true, SHEP>(stage, L.mode, L); break;
-            case 2: launch_tpp<DIM, KK, 2, false, true, SHEP>(stage, L.mode, L); break;
-            default: launch_tpp<DIM, KK, 4, false, true, SHEP>(stage, L.mode, L); break;
-        }
-    } else {
-        switch (tpp) {
-            case -1: launch_tpp<DIM, KK, 1, true, false, SHEP>(stage, L.mode, L); break;
-            case 1: launch_tpp<DIM, KK, 1, false, false, SHEP>(stage, L.mode, L); break;
-            case 2: launch_tpp<DIM, KK, 2, false, false, SHEP>(stage, L.mode, L); break;
-            case 8: launch_tpp<DIM, KK, 8, false, false, SHEP>(stage, L.mode, L); break;
-            default: launch_tpp<DIM, KK, 4, false, false, SHEP>(stage, L.mode, L); break;
-        }
-    }
-}
-
-template <int DIM, bool LIST, bool SHEP>
+template <int DIM>
 void dispatch(int stage, const LaunchCtx& L) {
     switch (L.kernel) {
-        case SPH_KERNEL_CUBIC_SPLINE: launch_kk<DIM, SPH_KERNEL_CUBIC_SPLINE, LIST, SHEP>(stage, L); break;
-        case SPH_KERNEL_GAUSSIAN: launch_kk<DIM, SPH_KERNEL_GAUSSIAN, LIST, SHEP>(stage, L); break;
-        case SPH_KERNEL_WENDLAND_C2: launch_kk<DIM, SPH_KERNEL_WENDLAND_C2, LIST, SHEP>(stage, L); break;
-        default: launch_kk<DIM, SPH_KERNEL_WENDLAND_C4, LIST, SHEP>(stage, L); break;
+        case SPH_KERNEL_CUBIC_SPLINE: launch_kk<DIM, SPH_KERNEL_CUBIC_SPLINE>(stage, L); break;
+        case SPH_KERNEL_GAUSSIAN: launch_kk<DIM, SPH_KERNEL_GAUSSIAN>(stage, L); break;
+        case SPH_KERNEL_WENDLAND_C2: launch_kk<DIM, SPH_KERNEL_WENDLAND_C2>(stage, L); break;
+        default: launch_kk<DIM, SPH_KERNEL_WENDLAND_C4>(stage, L); break;
     }
 }
 

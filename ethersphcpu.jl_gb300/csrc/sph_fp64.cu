@@ -65,6 +65,25 @@ __device__ __forceinline__ bool within_cut(const V& xi, const V& xj, const Scene
     return norm_sq<DIM>(rv) <= S.rc2;
 }
 
+// Selection into a list of indices with a relative margin of 1e-4 on r_cut^2 (cell-relative
+// differences within the stencil carry an FP32 error of some 1e-6 cells): only candidates
+// beyond r_cut are left out.  A particle far outside its cell (clamped from outside the
+// grid) or with a non-finite position is tested by within(j), in FP64.
+template <int DIM, typename Within, typename Pairs>
+__device__ __forceinline__ void select_64(const SceneDev& S, const int32_t* __restrict__ start,
+                                          const float4* __restrict__ pos, const int32_t c[3], const float4& me,
+                                          int self, bool on, int32_t* list, Within&& within, Pairs&& pairs) {
+    const SelectScale scale{S.sel_e[0], S.sel_e[1], S.sel_e[2], S.sel_inv_ex, 1.0001f, true};
+    const bool far = select_far(me);
+    coop_select<DIM, kCoopList<DIM>>(
+        S, scale, start, pos, c, me, self, on, [&](int j, float d2) { return far ? within(j) : d2 <= 1.0001f; },
+        [&](int slot, int j, float, float, float) { list[slot] = j; },
+        [&](int first, int cnt, bool) {
+            pairs(first, cnt);
+            return 0;
+        });
+}
+
 template <int DIM, int KK>
 __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
     k_continuity_fp64(const SceneDev* __restrict__ scenes, SortedState st, SortScratch sc, int32_t cap, BufferState bf) {
@@ -87,7 +106,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
         int32_t c[3];
         decode_cell(st.cell[i], S, c);
         double drho = 0.0;
-        coop_select<DIM>(
+        select_64<DIM>(
             S, sc.start, st.fa, c, st.fa[i], i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
             [&](int first, int cnt) {
                 int k = (lane - first) & (kCoopLanes - 1);
@@ -229,7 +248,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
         // PressureForce.jl:14-19, ViscosityForce.jl:15-23, ThermalConduction.jl:15-21.  With
         // mu = nu0 rho the viscosity factor is 4 nu0 m_j r dW / ((rho_i + rho_j) (r^2 + 0.01 h^2));
         // heat is taken as aT = sum m_j/rho_j kappa_j r dW / ((kappa_i + kappa_j) (r^2 + 0.01 h^2)) T_ij
-        coop_select<DIM>(
+        select_64<DIM>(
             S, sc.start, st.fa, c, me, i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
             [&](int first, int cnt) {
                 rounds(first, cnt, [&](int k, int e0, int e1) {
@@ -340,7 +359,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
             const double Pw = P_i + S.P_bg;
             const double Wg_i = uniform ? S.wg : kernel_w<KK>(gap_i, S);
             const double nu_rho = 2.0 * S.nu0 / rho_i;  // 8 mu_i / (2 rho_i)^2
-            coop_select<DIM>(
+            select_64<DIM>(
                 S, wl.start, wl.fa, c, me, -1, walls, list, [&](int j) { return within_cut<DIM>(xi, wx[j], S); },
                 [&](int first, int cnt) {
                     rounds(first, cnt, [&](int k, int e0, int e1) {
@@ -524,7 +543,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
             if (k < bs.cap) bs.pend[k] = i;
             else atomicOr(sc.status, kStatusBufferOverflow);
         } else {
-            cell_arrival(sc, i, cell_key<DIM>(xo, S));
+            cell_arrival(sc, i, moved_key<DIM>(st.cell[i], st.fa[i], xi, xo, S));
         }
     };
     coop_turns(min(cap, *sc.n_live), sc.queue, gather, update);

@@ -34,13 +34,8 @@ struct LaunchCtx {
     int shepard;
     int force_reinit;
     int skip_reinit;
-    // launch shape of the FP32 gathers (lanes per particle, threads per block)
-    int block;
-    int tpp_continuity, tpp_momentum;
-    // list_momentum != 0: continuity (one or two lanes) records the neighbour list and momentum
-    // reads it (tpp_momentum lanes per particle)
-    int list_momentum;
-    NbrList nl;
+    int lanes;   // FP32 gathers: 1 lanes share a particle, 0 a thread each, -1 by the particle count
+    NbrList nl;  // neighbour list of the FP32 form (e null: momentum walks the cells)
     // inlet/outlet buffers (bf.n == nullptr: none): current and next sorted buffers
     BufferState bf, bf2;
     BufferScratch bs;
@@ -72,13 +67,6 @@ void launch_physics_fp64(int stage, const LaunchCtx& L);
 void launch_physics_fp32(int stage, const LaunchCtx& L);
 void launch_physics_fp32_2d(int stage, const LaunchCtx& L);
 void launch_physics_fp32_3d(int stage, const LaunchCtx& L);
-void launch_physics_fp32_list_2d(int stage, const LaunchCtx& L);
-void launch_physics_fp32_list_3d(int stage, const LaunchCtx& L);
-// the momentum gathers of re-initialisation steps (L.shepard set)
-void launch_momentum_fp32_2d_shep(const LaunchCtx& L);
-void launch_momentum_fp32_3d_shep(const LaunchCtx& L);
-void launch_momentum_fp32_list_2d_shep(const LaunchCtx& L);
-void launch_momentum_fp32_list_3d_shep(const LaunchCtx& L);
 
 // Buffer particles after the gathers of a step (K4-K5): move them, copy inlet particles
 // that crossed into the fluid, move the fluid particles K5 marked to the outlet, drop

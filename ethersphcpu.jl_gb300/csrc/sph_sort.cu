@@ -232,8 +232,8 @@ __global__ void k_fill(SortScratch sc, const int32_t* __restrict__ id, int32_t c
     sc.tmp[sc.start[key] + sc.slot[i]] = id[i];
 }
 
-// CARRY (FP32 shadows of a step): the FP32 copies of the per-particle constants (m, gap,
-// kappa, cp) are taken from the particle's current shadows instead of being converted from
+// CARRY (FP32 shadows of a step): the FP32 copies of the per-particle constants (m kg_a/h,
+// kappa) are taken from the particle's current shadows instead of being converted from
 // FP64 again (the FP64 pipe is 1/64 of the FP32 rate on GB300); after an upload the
 // shadows do not exist yet and are converted.
 template <int DIM, bool THERMAL, bool SHADOW, bool CARRY>
@@ -243,6 +243,7 @@ __global__ void k_place(const SceneDev* __restrict__ scenes, SortedState src, Ne
     using V = typename VecT<DIM>::T;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     // count[] and the tile sums have been scanned: clear them for the next step's arrivals
+    if (i == 0) *sc.n_walked = 0;
     for (int k = i; k < ncells; k += gridDim.x * blockDim.x) sc.count[k] = 0;
     for (int k = i; k < ncells / kScanTileCells + 1; k += gridDim.x * blockDim.x) sc.block_sums[k] = 0;
     if (i >= cap || i >= *sc.n_live) return;
@@ -253,7 +254,7 @@ __global__ void k_place(const SceneDev* __restrict__ scenes, SortedState src, Ne
     // each load after the previous store (one memory round trip per field)
     const V x = ((const V*)nx.x)[i];
     const V v = ((const V*)nx.v)[i];
-    const double rho = nx.rho[i], p = src.p[i], c = src.c[i], m = src.m[i], gap = src.gap[i];
+    const double rho = nx.rho[i], p = src.p[i], cs = src.c[i], m = src.m[i], gap = src.gap[i];
     const int32_t myid = src.id[i], scn = src.scene[i];
     double T = 0.0, kap = 0.0, cpv = 1.0;
     if (THERMAL) {
@@ -262,34 +263,13 @@ __global__ void k_place(const SceneDev* __restrict__ scenes, SortedState src, Ne
         cpv = src.cp[i];
     }
     // FP32 constants: carried from the current shadows, or converted
-    float m_f, gap_f, kap_f = 0.f, cp_f = 1.f;
+    float mk_f = 0.f, kap_f = 0.f;
     if constexpr (SHADOW && CARRY) {
-        if constexpr (DIM == 2) {
-            const float4 b = src.fb[i];
-            m_f = b.x;
-            gap_f = b.w;
-            if (THERMAL) {
-                const float4 cc = src.fc[i];
-                kap_f = cc.y;
-                cp_f = cc.z;
-            }
-        } else {
-            const float4 a = src.fa[i];
-            const float4 cc = src.fc[i];
-            m_f = a.w;
-            gap_f = cc.y;
-            if (THERMAL) {
-                kap_f = cc.w;
-                cp_f = src.fd[i];
-            }
-        }
-    } else {
-        m_f = (float)m;
-        gap_f = (float)gap;
-        if (THERMAL) {
-            kap_f = (float)kap;
-            cp_f = (float)cpv;
-        }
+        mk_f = src.fb[i].w;
+        if (THERMAL) kap_f = src.fc[i].w;
+    } else if constexpr (SHADOW) {
+        mk_f = (float)(m * scenes[scn].kg_h);
+        if (THERMAL) kap_f = (float)kap;
     }
     const int32_t b = sc.start[key], e = sc.start[key + 1];
     int32_t rank = 0;
@@ -299,7 +279,7 @@ __global__ void k_place(const SceneDev* __restrict__ scenes, SortedState src, Ne
     ((V*)dst.v)[d] = v;
     dst.rho[d] = rho;
     dst.p[d] = p;
-    dst.c[d] = c;
+    dst.c[d] = cs;
     dst.m[d] = m;
     dst.gap[d] = gap;
     dst.id[d] = myid;
@@ -309,31 +289,15 @@ __global__ void k_place(const SceneDev* __restrict__ scenes, SortedState src, Ne
         dst.kappa[d] = kap;
         dst.cp[d] = cpv;
     }
-    if (!SHADOW) {  // the FP64 gathers' cell and selection position
-        const SceneDev& S = scenes[scn];
-        int32_t c[3];
-        decode_cell(key, S, c);
-        dst.cell[d] = key;
-        dst.fa[d] = select_pos<DIM>(x, S, c);
-    }
-    if (SHADOW) {  // FP32 shadows: position relative to the origin of the particle's cell
-        const SceneDev& S = scenes[scn];
-        const int32_t k = key - S.cell_off;
-        const int32_t cx = k % S.n[0], cy = (k / S.n[0]) % S.n[1], cz = k / (S.n[0] * S.n[1]);
-        const float xr = (float)(x.x - __dadd_rn(S.lo[0], __dmul_rn((double)cx, S.cell_d[0])));
-        const float yr = (float)(x.y - __dadd_rn(S.lo[1], __dmul_rn((double)cy, S.cell_d[1])));
-        dst.cell[d] = key;
-        if constexpr (DIM == 2) {
-            dst.fa[d] = make_float4(xr, yr, (float)v.x, (float)v.y);
-            dst.fb[d] = make_float4(m_f, (float)rho, 0.f, gap_f);
-            dst.fc[d] = make_float4((float)T, kap_f, cp_f, 0.f);
-        } else {
-            const float zr = (float)(x.z - __dadd_rn(S.lo[2], __dmul_rn((double)cz, S.cell_d[2])));
-            dst.fa[d] = make_float4(xr, yr, zr, m_f);
-            dst.fb[d] = make_float4((float)v.x, (float)v.y, (float)v.z, (float)rho);
-            dst.fc[d] = make_float4(0.f, gap_f, (float)T, kap_f);
-            dst.fd[d] = cp_f;
-        }
+    // the gathers' cell and FP32 copies
+    const SceneDev& S = scenes[scn];
+    int32_t c[3];
+    decode_cell(key, S, c);
+    dst.cell[d] = key;
+    dst.fa[d] = select_pos<DIM>(x, S, c);
+    if constexpr (SHADOW) {
+        dst.fb[d] = make_float4((float)v.x, (float)v.y, DIM == 3 ? (float)comp(v, DIM - 1) : 0.f, mk_f);
+        dst.fc[d] = make_float4((float)rho, 0.f, (float)T, kap_f);
     }
 }
 
