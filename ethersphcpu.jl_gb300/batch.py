@@ -150,10 +150,10 @@ class Batch:
     def download(self, sid: int, capacity: int | None = None) -> dict:
         cap = capacity if capacity is not None else self.info(sid)["n_fluid"]
         d = self.dim
-        out = {k: np.empty((cap, d)) for k in ("x", "v")}
         names = ["rho", "p", "c", "mass", "gap"] + (["t", "kappa", "cp"] if self.thermal else [])
-        for k in names:
-            out[k] = np.empty(cap)
+        block = np.empty((2 * d + len(names)) * cap)  # one behind the other: a whole scene is one copy
+        out = {k: block[q * d * cap: (q + 1) * d * cap].reshape(cap, d) for q, k in enumerate(("x", "v"))}
+        out.update({k: block[(2 * d + q) * cap: (2 * d + q + 1) * cap] for q, k in enumerate(names)})
         n = C.c_int64()
         ptr = lambda k: _abi.dptr(out[k]) if k in out else None
         self._check(self.lib.sph_batch_download_scene(self.h, sid, cap, C.byref(n), ptr("x"), ptr("v"), ptr("rho"),

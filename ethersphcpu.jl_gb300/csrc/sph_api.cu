@@ -340,6 +340,11 @@ struct SphHandle {
     int32_t scap = 1;
     cudaStream_t stream = nullptr;
     std::vector<void*> allocs;
+    // the state's arrays lie in one allocation (allocate_handle): its base (null while the
+    // sizes are added up), its bytes so far, and whether take() deals from it
+    char* arena = nullptr;
+    size_t arena_used = 0;
+    bool in_arena = false;
     SortedState S[2]{};
     NextState N{};
     WallState W{};
@@ -349,7 +354,10 @@ struct SphHandle {
     double* d_stat_partials = nullptr;
     double* d_stat_out = nullptr;
     unsigned long long* d_pair_counts = nullptr;
-    int64_t* h_pinned = nullptr;  // [0]: step upload, [1]: status, [2..3]: ranges
+    // words of small transfers (word()); [0]: step upload, [1]: status, [2..3]: ranges
+    int64_t host_words[4] = {};
+    int64_t* h_pinned = nullptr;
+    int word_uses = 0;
     int par = 0;
     bool have_fluid = false;
     int64_t steps_done = 0;
@@ -409,24 +417,32 @@ int cuda_fail(SphHandle* h, cudaError_t e, const char* what) {
         if (_e != cudaSuccess) return cuda_fail((h), _e, #call);   \
     } while (0)
 
+// Zeroed device memory: the next 256-byte aligned piece of the handle's arena while that is
+// laid out, an allocation of its own otherwise.
+cudaError_t take(SphHandle* h, void** p, size_t bytes) {
+    if (h->in_arena) {
+        *p = h->arena ? h->arena + h->arena_used : nullptr;
+        h->arena_used += (bytes + 255) / 256 * 256;
+        return cudaSuccess;
+    }
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) return e;
+    h->allocs.push_back(*p);
+    return cudaMemsetAsync(*p, 0, bytes, h->stream);
+}
+
 template <typename T>
 cudaError_t dalloc(SphHandle* h, T** p, size_t count) {
     void* q = nullptr;
-    cudaError_t e = cudaMalloc(&q, std::max<size_t>(count, 1) * sizeof(T));
-    if (e != cudaSuccess) return e;
-    h->allocs.push_back(q);
-    *p = (T*)q;
-    return cudaMemsetAsync(q, 0, std::max<size_t>(count, 1) * sizeof(T), h->stream);
+    cudaError_t e = take(h, &q, std::max<size_t>(count, 1) * sizeof(T));
+    if (e == cudaSuccess) *p = (T*)q;
+    return e;
 }
 
 size_t vec_bytes(int dim) { return dim == 2 ? sizeof(double2) : sizeof(double4_32a); }
 
 cudaError_t alloc_vec(SphHandle* h, void** p, size_t n) {
-    const size_t bytes = std::max<size_t>(n, 1) * vec_bytes(h->dim);
-    cudaError_t e = cudaMalloc(p, bytes);
-    if (e != cudaSuccess) return e;
-    h->allocs.push_back(*p);
-    return cudaMemsetAsync(*p, 0, bytes, h->stream);
+    return take(h, p, std::max<size_t>(n, 1) * vec_bytes(h->dim));
 }
 
 cudaError_t alloc_sorted(SphHandle* h, SortedState& s) {
@@ -627,17 +643,33 @@ void set_n_upper(SphHandle* h, int64_t n) {
     h->n_upper = n;
 }
 
+// Host word k of a transfer that is waited for before the next.  Page-locking costs a handle
+// 100 us and unlocking 160, and saves some 5 us a transfer: a handle pins its words when it
+// has used them kWordUses times, which a run of one call (a handle made, run once and closed)
+// does not reach.
+constexpr int kWordUses = 8;
+int64_t* word(SphHandle* h, int k) {
+    if (!h->h_pinned && ++h->word_uses >= kWordUses &&
+        cudaMallocHost((void**)&h->h_pinned, sizeof(h->host_words)) != cudaSuccess) {
+        cudaGetLastError();
+        h->h_pinned = nullptr;
+        h->word_uses = INT_MIN;  // no page to lock: go on without
+    }
+    return (h->h_pinned ? h->h_pinned : h->host_words) + k;
+}
+
 int32_t read_live(SphHandle* h, int32_t* n) {
-    SPH_CUDA(h, cudaMemcpyAsync(&h->h_pinned[2], h->nbuf + h->par, 4, cudaMemcpyDeviceToHost, h->stream));
+    int64_t* w = word(h, 2);
+    SPH_CUDA(h, cudaMemcpyAsync(w, h->nbuf + h->par, 4, cudaMemcpyDeviceToHost, h->stream));
     SPH_CUDA(h, cudaStreamSynchronize(h->stream));
-    std::memcpy(n, &h->h_pinned[2], 4);
+    std::memcpy(n, w, 4);
     return SPH_OK;
 }
 
 // [begin, end) of scene s in the sorted arrays.
 int32_t scene_range(SphHandle* h, int s, int32_t* b, int32_t* e) {
     const SceneRec& R = h->scenes[s];
-    int32_t v[2];
+    int32_t* v = (int32_t*)word(h, 2);
     SPH_CUDA(h, cudaMemcpyAsync(&v[0], h->sc.start + R.dev.cell_off, 4, cudaMemcpyDeviceToHost, h->stream));
     SPH_CUDA(h, cudaMemcpyAsync(&v[1], h->sc.start + R.dev.cell_off + R.dev.ncells, 4, cudaMemcpyDeviceToHost,
                                 h->stream));
@@ -654,8 +686,9 @@ int32_t upload_scene_const(SphHandle* h, int s) {
 }
 
 int32_t set_scene_step(SphHandle* h, int s, int64_t step) {
-    h->h_pinned[0] = step;
-    SPH_CUDA(h, cudaMemcpyAsync(h->sc.scene_step + s, &h->h_pinned[0], 8, cudaMemcpyHostToDevice, h->stream));
+    int64_t* w = word(h, 0);
+    *w = step;
+    SPH_CUDA(h, cudaMemcpyAsync(h->sc.scene_step + s, w, 8, cudaMemcpyHostToDevice, h->stream));
     SPH_CUDA(h, cudaStreamSynchronize(h->stream));
     h->scenes[s].step_host = step;
     return SPH_OK;
@@ -882,11 +915,11 @@ int32_t append_fluid(SphHandle* h, int s, int32_t n_before, int64_t n, const dou
             SPH_CUDA(h, cudaMemcpyAsync(d.cp + o, cp, n * 8, cudaMemcpyHostToDevice, st));
         }
     }
-    h->h_pinned[2] = 0;
+    int64_t* w = word(h, 2);
     const int32_t total = (int32_t)(n_before + n);
     set_n_upper(h, total);
-    std::memcpy(&h->h_pinned[2], &total, 4);
-    SPH_CUDA(h, cudaMemcpyAsync(h->nbuf + h->par, &h->h_pinned[2], 4, cudaMemcpyHostToDevice, st));
+    std::memcpy(w, &total, 4);
+    SPH_CUDA(h, cudaMemcpyAsync(h->nbuf + h->par, w, 4, cudaMemcpyHostToDevice, st));
     SPH_CUDA(h, cudaStreamSynchronize(st));  // host staging buffers die at return
     return resort(h);
 }
@@ -918,8 +951,9 @@ void ascending_id_order(const std::vector<int32_t>& ids, std::vector<int32_t>& o
 }
 
 // Download the live particles of scene s in ascending id: the rows are put in that order
-// on the device (one gather launch into a staging buffer), then each requested array is
-// copied straight into the caller's memory.
+// on the device (one gather launch into a staging buffer), then the requested arrays are
+// copied straight into the caller's memory, those that lie one behind the other there (as
+// Batch.download lays them out) as one: a pageable copy costs 10-15 us however small.
 int32_t download_scene(SphHandle* h, int s, int64_t capacity, int64_t* n_out, double* x, double* v, double* rho,
                        double* p, double* c, double* mass, double* gap, double* t, double* kappa, double* cp,
                        int64_t* ids_out) {
@@ -970,16 +1004,25 @@ int32_t download_scene(SphHandle* h, int s, int64_t capacity, int64_t* n_out, do
         launch_gather_rows(st, dim, d_order, n, b, d.x, d.v, F, d_out);
     }
     SPH_CUDA(h, cudaGetLastError());
-    double* o = d_out;
-    if (x) {
-        SPH_CUDA(h, cudaMemcpyAsync(x, o, (size_t)n * dim * 8, cudaMemcpyDeviceToHost, st));
-        o += n * dim;
+    struct {
+        double* to;
+        size_t words;
+    } part[10] = {};
+    int parts = 0;
+    auto add = [&](double* to, size_t words) {
+        if (parts && (uintptr_t)(part[parts - 1].to) + part[parts - 1].words * 8 == (uintptr_t)to)
+            part[parts - 1].words += words;
+        else
+            part[parts++] = {to, words};
+    };
+    if (x) add(x, (size_t)n * dim);
+    if (v) add(v, (size_t)n * dim);
+    for (int f = 0; f < F.n; ++f) add(out_of[f], (size_t)n);
+    const double* o = d_out;
+    for (int q = 0; q < parts; ++q) {
+        SPH_CUDA(h, cudaMemcpyAsync(part[q].to, o, part[q].words * 8, cudaMemcpyDeviceToHost, st));
+        o += part[q].words;
     }
-    if (v) {
-        SPH_CUDA(h, cudaMemcpyAsync(v, o, (size_t)n * dim * 8, cudaMemcpyDeviceToHost, st));
-        o += n * dim;
-    }
-    for (int f = 0; f < F.n; ++f) SPH_CUDA(h, cudaMemcpyAsync(out_of[f], o + (size_t)f * n, n * 8, cudaMemcpyDeviceToHost, st));
     SPH_CUDA(h, cudaStreamSynchronize(st));
     return SPH_OK;
 }
@@ -1030,10 +1073,9 @@ int32_t step_all_async(SphHandle* h, int64_t nsteps) {
     return SPH_OK;
 }
 
-int32_t allocate_handle(SphHandle* h, int64_t cells) {
+// The device arrays of a handle's state.
+int32_t allocate_state(SphHandle* h, int64_t cells) {
     cudaError_t e;
-    if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
-        return cuda_fail(nullptr, e, "stream");
     for (int b = 0; b < 2; ++b)
         if ((e = alloc_sorted(h, h->S[b])) != cudaSuccess) return cuda_fail(nullptr, e, "sorted state");
     if ((e = alloc_vec(h, &h->N.x, h->cap)) != cudaSuccess) return cuda_fail(nullptr, e, "next x");
@@ -1077,8 +1119,28 @@ int32_t allocate_handle(SphHandle* h, int64_t cells) {
     if ((e = dalloc(h, &h->d_stat_partials, 3 * 152)) != cudaSuccess) return cuda_fail(nullptr, e, "stats");
     if ((e = dalloc(h, &h->d_stat_out, 4)) != cudaSuccess) return cuda_fail(nullptr, e, "stats");
     if ((e = dalloc(h, &h->d_pair_counts, 2)) != cudaSuccess) return cuda_fail(nullptr, e, "pairs");
-    if ((e = cudaMallocHost((void**)&h->h_pinned, sizeof(int64_t) * 4)) != cudaSuccess)
-        return cuda_fail(nullptr, e, "pinned");
+    return SPH_OK;
+}
+
+// A handle's stream and state.  The state is one allocation, laid out in two
+// passes over allocate_state (sizes, then pointers), and one memset: the some forty
+// allocations, memsets and frees of a handle with an allocation an array took most of what a
+// short run spends outside its steps.
+int32_t allocate_handle(SphHandle* h, int64_t cells) {
+    cudaError_t e;
+    if ((e = cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking)) != cudaSuccess)
+        return cuda_fail(nullptr, e, "stream");
+    h->in_arena = true;
+    int32_t rc = allocate_state(h, cells);
+    if (rc != SPH_OK) return rc;
+    const size_t bytes = h->arena_used;
+    if ((e = cudaMalloc((void**)&h->arena, bytes)) != cudaSuccess) return cuda_fail(nullptr, e, "state");
+    h->allocs.push_back(h->arena);
+    if ((e = cudaMemsetAsync(h->arena, 0, bytes, h->stream)) != cudaSuccess) return cuda_fail(nullptr, e, "state");
+    h->arena_used = 0;
+    rc = allocate_state(h, cells);
+    h->in_arena = false;
+    if (rc != SPH_OK) return rc;
     if ((e = cudaStreamSynchronize(h->stream)) != cudaSuccess) return cuda_fail(nullptr, e, "create sync");
     h->total_cells = (int32_t)cells;
     h->cells.init(cells);
@@ -1327,11 +1389,12 @@ int32_t sph_synchronize(SphHandle* h) {
     NvtxRange nvtx_range("sph_synchronize");
     if (!h) return fail(nullptr, SPH_ERR_ARG, "null handle");
     cudaStream_t st = h->stream;
-    SPH_CUDA(h, cudaMemcpyAsync(&h->h_pinned[1], h->sc.status, 4, cudaMemcpyDeviceToHost, st));
+    int64_t* w = word(h, 1);
+    SPH_CUDA(h, cudaMemcpyAsync(w, h->sc.status, 4, cudaMemcpyDeviceToHost, st));
     SPH_CUDA(h, cudaMemsetAsync(h->sc.status, 0, 4, st));
     SPH_CUDA(h, cudaStreamSynchronize(st));
     int32_t status = 0;
-    std::memcpy(&status, &h->h_pinned[1], 4);
+    std::memcpy(&status, w, 4);
     bool nan_check = h->prm.nan_check;
     for (const SceneRec& R : h->scenes) nan_check |= R.used && R.dev.nan_check;
     if ((status & kStatusNonFinite) && nan_check)
