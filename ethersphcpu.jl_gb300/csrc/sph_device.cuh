@@ -25,11 +25,15 @@ constexpr int32_t kDeadKey = 0x7fffffff;
 // Programmatic dependent launch between the kernels of a step (launch_dep): the next
 // kernel's launch is prepared while its predecessor in the stream finishes; pdl_wait()
 // blocks until the predecessor grid has completed and its writes are visible (a no-op
-// when the kernel was launched without the attribute).  Every step kernel calls it first,
-// before it touches device memory.  No kernel triggers its dependents early: blocks of the
+// when the kernel was launched without the attribute).  A step kernel calls it first, before
+// it touches device memory.  A kernel whose successor has nothing to do before its wait does
+// not trigger it early: blocks of the
 // next kernel parked on the wait took SM slots from the tail of the current one (a
 // 65k-particle step on GB300: 0.0652 ms with an early trigger, 0.0642 ms without
 // programmatic launches, 0.0622 ms with the trigger at block exit, as here).
+// A predecessor may let its successor start early where that has work of its own to do before
+// it waits (pdl_trigger, after its own pdl_wait: what came before it is then visible to both).
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Status bits written by kernels (atomicOr) and read by the host after a step.

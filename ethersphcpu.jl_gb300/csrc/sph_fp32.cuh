@@ -726,6 +726,7 @@ template <int DIM, int KK, int MODE, bool SHEP>
 __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
     k_walks_f32(const SceneDev* __restrict__ scenes, SortedState st, WallState wl, SortScratch sc, NbrList nl, int sel) {
     pdl_wait();
+    pdl_trigger();  // k_momentum_f32 takes its lists meanwhile: it needs the walks' sums last
     constexpr bool HEAT = MODE == kModeThermal;
     constexpr int kSums = DIM + (HEAT ? 1 : 0);
     const int n = *sc.n_walked, lane = threadIdx.x % kCoopLanes;
@@ -765,19 +766,27 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
 
 // Large scenes: one thread a particle.  Eight sums take the entries of the list in turns, as
 // the lanes of k_momentum_lanes_f32 do, so both give the same bits; a warp's threads read the
-// same entry of 32 consecutive particles, whose neighbours lie side by side.
+// same entry of 32 consecutive particles, whose neighbours lie side by side.  It runs beside
+// k_walks_f32, which starts it once continuity's results are visible, and waits for it where it
+// needs the walks' sums and before it writes anything (every thread waits: the grid must not
+// end before the walks).  Both together against one after the other: 17.0 against 24.1 us on
+// a 65,536-particle cavity (54 -> 47 us a step), 216 against 228 on a million particles,
+// 315 against 330 on a 432,000-particle 3D dam break.
 template <int DIM, int KK, int MODE, bool SHEP>
 __global__ void __launch_bounds__(128, 4)
     k_momentum_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl, SortScratch sc,
                    int32_t cap, BufferState bf, BufferScratch bs, BufferRules br, NbrList nl, int sel) {
-    pdl_wait();
     constexpr bool HEAT = MODE == kModeThermal;
     constexpr int kSums = DIM + (HEAT ? 1 : 0);
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= cap || i >= *sc.n_live) return;
+    if (i >= cap || i >= *sc.n_live) {
+        pdl_wait();
+        return;
+    }
     const SceneDev& S = scenes[st.scene[i]];
     const int64_t step = sc.scene_step[st.scene[i]];
     if (!takes_part<SHEP>(S, step, sel)) {
+        pdl_wait();
         if (!SHEP && !scene_runs(S, step)) carry_frozen<DIM>(i, S, st, nx, sc);
         return;
     }
@@ -829,6 +838,7 @@ __global__ void __launch_bounds__(128, 4)
         sw = ((w8[0] + w8[1]) + (w8[2] + w8[3])) + ((w8[4] + w8[5]) + (w8[6] + w8[7]));
         sws = ((ws8[0] + ws8[1]) + (ws8[2] + ws8[3])) + ((ws8[4] + ws8[5]) + (ws8[6] + ws8[7]));
     }
+    pdl_wait();
     if (count == kListWalk || (wl.n > 0 && wl.near[st.cell[i]])) {  // the cell walks (k_walks_f32)
         const float2* in = sc.walk_sums + (int64_t)i * (2 * kSums + 2);
 #pragma unroll
