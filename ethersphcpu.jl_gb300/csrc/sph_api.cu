@@ -1091,7 +1091,7 @@ int32_t allocate_state(SphHandle* h, int64_t cells) {
                 {&h->sc.tmp, (size_t)h->cap},        {&h->sc.count, ncell},
                 {&h->sc.start, ncell + 1},           {&h->sc.block_sums, ncell / 1024 + 2},
                 {&h->sc.status, 1},                  {&h->nbuf, 2},
-                {&h->sc.queue, 2},                   {&h->sc.n_walked, 1},
+                {&h->sc.queue, 4},                   {&h->sc.n_walked, 1},
                 {&h->W.start, ncell + 1},            {&h->W.kind, wc}};
     for (auto& a : ints)
         if ((e = dalloc(h, a.p, a.n)) != cudaSuccess) return cuda_fail(nullptr, e, "scratch");

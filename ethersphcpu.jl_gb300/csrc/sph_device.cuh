@@ -191,7 +191,8 @@ struct SortScratch {
     int32_t* block_sums;
     int32_t* n_live;    // device scalar: live particles after the last sort
     int32_t* status;    // device scalar: status bits
-    int32_t* queue;     // draws and finished blocks of a cooperative gather (coop_turns), both 0 between launches
+    int32_t* queue;     // draws and finished blocks of a cooperative gather (coop_turns), 0 between launches;
+                        // a pair for continuity, a pair for momentum, which starts beside it
     // FP32 form, large scenes: the particles whose cells the momentum gather walks, their
     // number (0 before continuity) and their sums of those walks (fluid, walls, Shepard)
     int32_t* walked;
