@@ -361,6 +361,7 @@ template <int DIM, int KK>
 __global__ void __launch_bounds__(256) k_continuity_rows_f32(const SceneDev* __restrict__ scenes, SortedState st,
                                                              SortScratch sc, int32_t cap, BufferState bf, NbrList nl) {
     pdl_wait();
+    pdl_trigger();
     const unsigned full = 0xffffffffu;
     __shared__ int32_t rows[kRowEntries * 256];
     __shared__ float2 sums[32];
@@ -858,13 +859,14 @@ __global__ void __launch_bounds__(128, 4)
 // Small scenes: eight lanes a particle, lane t the
 // entries t, t + 8, ... of its list, or a neighbour row of the walls (and of the fluid, for a
 // particle whose list did not fit).  A block of 256 threads takes 32 particles; its first
-// warp merges the lanes' sums and updates the particles.
+// warp merges the lanes' sums and updates the particles.  Continuity starts it early: the
+// chain of loads to a particle's scene and own values is then over when the lists are there
+// (a step of a 5,000-particle dam break 23.5 -> 22.7 us).
 template <int DIM, int KK, int MODE, bool SHEP>
 __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
     k_momentum_lanes_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl,
                          SortScratch sc, int32_t cap, BufferState bf, BufferScratch bs, BufferRules br, NbrList nl,
                          int sel) {
-    pdl_wait();
     constexpr bool HEAT = MODE == kModeThermal;
     constexpr int kSums = DIM + (HEAT ? 1 : 0), kParts = kCoopLanes + 1;
     const unsigned full = 0xffffffffu;
@@ -873,12 +875,19 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
     const int g = threadIdx.x / kCoopLanes, lane = threadIdx.x % kCoopLanes;
     const int i0 = blockIdx.x * (blockDim.x / kCoopLanes);
     const int n = min(cap, *sc.n_live);
-    if (i0 >= n) return;  // the whole block
+    if (i0 >= n) {  // the whole block
+        pdl_wait();
+        return;
+    }
     {
+        // what continuity does not write is loaded before the wait
         const int i = min(i0 + g, n - 1);
         const SceneDev& S = scenes[st.scene[i]];
         const bool on = i0 + g < n && takes_part<SHEP>(S, sc.scene_step[st.scene[i]], sel);
-        const SelfF a = self_f<DIM, KK, HEAT>(S, st, i);
+        const bool walls = on && wl.n > 0 && wl.near[st.cell[i]];
+        SelfF a = self_f<DIM, KK, HEAT>(S, st, i);
+        pdl_wait();
+        a.f = st.fc[i];
         SumsF<DIM, HEAT> sum;
         double sw = 0.0, sws = 0.0;  // Shepard sums (ReconstructValue.jl:28-50), FP64
         const int count = on ? (nl.e ? nl.n[i] : kListWalk) : 0;
@@ -913,7 +922,7 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
             }
         }
         __syncwarp(full);
-        const bool walk = count == kListWalk, walls = on && wl.n > 0 && wl.near[st.cell[i]];
+        const bool walk = count == kListWalk;
         SumsF<DIM, HEAT> wall;
         if (__any_sync(full, walk || walls)) {
             SumsF<DIM, HEAT> fluid;
