@@ -364,7 +364,7 @@ struct SphHandle {
     // launch shape as set (sph_set_launch_shape); lanes: what the autotuner found for the FP32
     // gathers (LaunchCtx::lanes), whose sums do not depend on it
     int tune[4] = {1, 1, 1, 128};
-    int lanes = -1;
+    int lanes[2] = {-1, -1};
     NbrList nl{};          // neighbour list of the FP32 form (ensure_list)
     bool no_list = false;  // no room for it
     // stencil pruning of the FP32 gathers (sph_set_stencil_pruning), on by default: the rows
@@ -552,7 +552,8 @@ LaunchCtx make_ctx(SphHandle* h) {
     L.shepard = 0;
     L.force_reinit = 0;
     L.skip_reinit = 0;
-    L.lanes = h->lanes;
+    L.lanes[0] = h->lanes[0];
+    L.lanes[1] = h->lanes[1];
     L.nl = h->nl;
     if (h->has_buffers) {
         L.bf = h->B[h->par];
@@ -1822,11 +1823,13 @@ int32_t sph_autotune(SphHandle* h, int32_t reps, int32_t* out) {
         // overwrite them, so park them in the idle sorted buffer meanwhile
         SPH_CUDA(h, cudaMemcpyAsync(h->S[par ^ 1].p, h->S[par].p, nbytes, cudaMemcpyDeviceToDevice, st));
         SPH_CUDA(h, cudaMemcpyAsync(h->S[par ^ 1].c, h->S[par].c, nbytes, cudaMemcpyDeviceToDevice, st));
-        // lanes sharing a particle, or a thread each: continuity then momentum as in a step
-        auto trial = [&](int lanes) -> float {
+        // lanes sharing a particle in both gathers, in continuity only, or a thread each:
+        // continuity then momentum as in a step
+        auto trial = [&](int continuity, int momentum) -> float {
             LaunchCtx L = make_ctx(h);
             L.bs.npend = nullptr;  // trial launches mark no particle for the outlet
-            L.lanes = lanes;
+            L.lanes[0] = continuity;
+            L.lanes[1] = momentum;
             auto step = [&] {
                 cudaMemsetAsync(h->sc.n_walked, 0, 4, st);
                 launch_physics(0, L);
@@ -1841,11 +1844,13 @@ int32_t sph_autotune(SphHandle* h, int32_t reps, int32_t* out) {
             cudaEventElapsedTime(&ms, e0, e1);
             return ms;
         };
-        const float shared = trial(1), own = trial(0);
+        const float both = trial(1, 1), rows = trial(1, 0), none = trial(0, 0);
         SPH_CUDA(h, cudaGetLastError());
-        h->lanes = shared < own ? 1 : 0;
-        h->tune[0] = h->tune[1] = h->lanes ? 8 : 1;
-        h->tune[3] = h->lanes ? 256 : 128;
+        h->lanes[0] = std::min(both, rows) < none;
+        h->lanes[1] = both < std::min(rows, none);
+        h->tune[0] = h->lanes[0] ? 8 : 1;
+        h->tune[1] = h->lanes[1] ? 8 : 1;
+        h->tune[3] = h->lanes[1] ? 256 : 128;
         // restore what the timed launches touched: p and c, and the arrivals left in
         // count[]; every other field they wrote is rebuilt by the next step before use
         SPH_CUDA(h, cudaMemsetAsync(h->sc.count, 0, sizeof(int32_t) * (size_t)h->scan_cells, st));

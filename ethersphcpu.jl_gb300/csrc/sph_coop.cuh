@@ -15,8 +15,9 @@
 //     warp updates its 32 particles, one a lane.  (Warps with a fixed share of 32 particles
 //     left the FP64 units idle for a third of the time, shares of 8 ran the update on a
 //     quarter of a warp.)  No warp waits for another.
-//   * a particle's sums do not depend on the batch, the warp or its other particles: where a scene at rest cancels large terms (pressure and wall forces) the
-//     terms are rounded and added in the reference's own order (pair_kernel, add_terms);
+//   * a particle's sums do not depend on the batch, the warp or its other particles: where a
+//     scene at rest cancels large terms (pressure and wall forces) the terms are rounded and
+//     added in the reference's own order (pair_kernel, add_terms);
 //     the other sums are taken by lane, lane t entries t, t + 8, ..., and the lanes' sums
 //     added in one fixed order.
 #pragma once

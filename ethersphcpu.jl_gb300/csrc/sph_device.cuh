@@ -27,8 +27,7 @@ constexpr int32_t kDeadKey = 0x7fffffff;
 // blocks until the predecessor grid has completed and its writes are visible (a no-op
 // when the kernel was launched without the attribute).  A step kernel calls it first, before
 // it touches device memory.  A kernel whose successor has nothing to do before its wait does
-// not trigger it early: blocks of the
-// next kernel parked on the wait took SM slots from the tail of the current one (a
+// not trigger it early: blocks of the next kernel parked on the wait took SM slots from the tail of the current one (a
 // 65k-particle step on GB300: 0.0652 ms with an early trigger, 0.0642 ms without
 // programmatic launches, 0.0622 ms with the trigger at block exit, as here).
 // A predecessor may let its successor start early where that has work of its own to do before
@@ -110,10 +109,6 @@ struct SceneDev {
 template <int DIM> struct VecT;
 template <> struct VecT<2> { using T = double2; };
 template <> struct VecT<3> { using T = double4_32a; };  // 32-byte aligned: one 256-bit access
-
-template <int DIM> struct FVec;
-template <> struct FVec<2> { using T = float2; };
-template <> struct FVec<3> { using T = float4; };
 
 __device__ __forceinline__ double comp(const double2& a, int k) { return k == 0 ? a.x : a.y; }
 __device__ __forceinline__ double comp(const double4_32a& a, int k) { return k == 0 ? a.x : (k == 1 ? a.y : a.z); }
@@ -290,12 +285,6 @@ __device__ __forceinline__ int32_t cell_coord(double x, const SceneDev& S, int a
     const double f = floor(u);
     if (f >= (double)(S.n[a] - 1)) return S.n[a] - 1;
     return (int32_t)f;
-}
-
-// Whether coordinate lies outside the grid (the particle was clamped into an edge cell).
-__device__ __forceinline__ bool outside_grid(double x, const SceneDev& S, int a) {
-    const double u = (x - S.lo[a]) * S.inv_cell[a];
-    return !(u >= 0.0) || u >= (double)S.n[a];
 }
 
 __device__ __forceinline__ void decode_cell(int32_t key, const SceneDev& S, int32_t c[3]) {

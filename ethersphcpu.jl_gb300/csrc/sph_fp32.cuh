@@ -11,13 +11,19 @@
 //
 // Continuity walks the cells, one thread a particle on large scenes and a lane a neighbour
 // row on small ones (the same sums, bit for bit), and records each particle's neighbours
-// (NbrList).  Momentum reads that list with eight lanes a particle: lane t takes entries
-// t, t + 8, ... with compensated partial sums of its own; its block's first warps merge them
-// (TwoSum of the sums, the rounding errors joining the compensations) and update the
+// (NbrList).  Momentum reads that list, on small scenes with eight lanes a particle: lane t
+// takes entries t, t + 8, ... with compensated partial sums of its own; its block's first warp merges them
+// (TwoSum of the sums, the rounding errors joining the compensations) and updates the
 // particles, one thread each, because FP64 instructions, of which a GB300 SM runs 1/64 of
-// its FP32 rate, cost a warp the same however many lanes take part.  A particle whose list
-// does not fit is walked again (coop_select), in the same order.  No sum depends on the block
-// size, the batch or the pruning.
+// its FP32 rate, cost a warp the same however many lanes take part.  On large scenes a thread
+// takes a particle and forms the same eight sums.  The cells of the walls, and of a particle
+// whose list does not fit, are walked with a lane a neighbour row (coop_rows).  No sum depends
+// on the variant, the batch or the pruning.
+//
+// What bounds them: on small scenes the chain of loads and rounds of one particle, on large
+// ones the issue of instructions (continuity issues in 73 of 100 cycles, momentum in 43 to 54
+// with 16 warps an SM for its eight sums, waiting on neighbours from L2); the bytes would take
+// a fifth of the time.
 //
 // On a re-initialisation step the momentum gather also forms the Shepard sums over the
 // same neighbours and writes the re-initialised density: the update and the
@@ -292,7 +298,10 @@ __device__ __forceinline__ void continuity_update(const SceneDev& S, const Sorte
 }
 
 // Large scenes: one thread a particle.  A row's terms are one compensated sum and the rows'
-// sums are merged in order; k_continuity_rows_f32 forms the same sums with a lane a row.
+// sums are merged in order; k_continuity_rows_f32 forms the same sums with a lane a row.  The
+// next row's cell starts and the next candidate's data are loaded ahead.  22.2 -> 19.7 us on a
+// 65,536-particle cavity, 170 -> 172 on a million particles (momentum reads the list it records
+// now), 418 -> 359 on a 432,000-particle 3D dam break.
 template <int DIM, int KK>
 __global__ void __launch_bounds__(128) k_continuity_f32(const SceneDev* __restrict__ scenes, SortedState st,
                                                         SortScratch sc, int32_t cap, BufferState bf, NbrList nl,
@@ -355,13 +364,17 @@ __global__ void __launch_bounds__(128) k_continuity_f32(const SceneDev* __restri
 }
 
 // Small scenes: eight lanes a particle, lane r the row dy = r - 3 of each plane, so the chain
-// of loads a particle waits for is a row's instead of the whole stencil's.  A block of 256
-// threads takes 32 particles; its first warp updates them.
+// of loads a particle waits for is a row's instead of the whole stencil's (21.5 -> 7.4 us on a
+// 5,000-particle dam break, 30.2 -> 10.5 on a 15,000-particle channel).  A block of 256
+// threads takes 32 particles; its first warp updates them.  Where a thread a particle takes the
+// momentum gather (threads), the particles it walks the cells for are listed as in
+// k_continuity_f32.
 template <int DIM, int KK>
 __global__ void __launch_bounds__(256) k_continuity_rows_f32(const SceneDev* __restrict__ scenes, SortedState st,
-                                                             SortScratch sc, int32_t cap, BufferState bf, NbrList nl) {
+                                                             SortScratch sc, int32_t cap, BufferState bf, NbrList nl,
+                                                             WallState wl, bool threads) {
     pdl_wait();
-    pdl_trigger();
+    if (!threads) pdl_trigger();
     const unsigned full = 0xffffffffu;
     __shared__ int32_t rows[kRowEntries * 256];
     __shared__ float2 sums[32];
@@ -420,6 +433,8 @@ __global__ void __launch_bounds__(256) k_continuity_rows_f32(const SceneDev* __r
         if (lane == 0) {
             sums[g] = make_float2(total.s, total.c);
             if (on && nl.e) nl.n[i] = fits ? count : kListWalk;
+            if (threads && on && (!fits || (wl.n > 0 && wl.near[st.cell[i]])))
+                sc.walked[atomicAdd(sc.n_walked, 1)] = i;
         }
     }
     __syncthreads();
@@ -772,7 +787,9 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
 // needs the walks' sums and before it writes anything (every thread waits: the grid must not
 // end before the walks).  Both together against one after the other: 17.0 against 24.1 us on
 // a 65,536-particle cavity (54 -> 47 us a step), 216 against 228 on a million particles,
-// 315 against 330 on a 432,000-particle 3D dam break.
+// 315 against 330 on a 432,000-particle 3D dam break (before the eight sums: 25.7, 254, 488).
+// The Shepard sums are a second pass over the list: 385 us with them at a million particles
+// (684 in lanes, 330 before, when the walk of the cells formed them).
 template <int DIM, int KK, int MODE, bool SHEP>
 __global__ void __launch_bounds__(128, 4)
     k_momentum_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl, SortScratch sc,
@@ -859,7 +876,9 @@ __global__ void __launch_bounds__(128, 4)
 // Small scenes: eight lanes a particle, lane t the
 // entries t, t + 8, ... of its list, or a neighbour row of the walls (and of the fluid, for a
 // particle whose list did not fit).  A block of 256 threads takes 32 particles; its first
-// warp merges the lanes' sums and updates the particles.  Continuity starts it early: the
+// warp merges the lanes' sums and updates the particles (30.6 -> 9.1 us on a 5,000-particle dam
+// break, 23.9 -> 11.3 on a 15,000-particle channel; a million particles would take 473 us, a
+// thread each 216).  Continuity starts it early: the
 // chain of loads to a particle's scene and own values is then over when the lists are there
 // (a step of a 5,000-particle dam break 23.5 -> 22.7 us).
 template <int DIM, int KK, int MODE, bool SHEP>
@@ -974,14 +993,29 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
 }
 
 // -------------------------------------------------------------------- launchers
-// A lane a row (continuity) and eight lanes a particle (momentum) below this many particles,
-// a thread a particle from there on.
-constexpr int64_t kLanesBelow = 40000;
+// Continuity takes a lane a row up to two waves of its blocks of 32 particles (four resident an
+// SM) and a thread a particle beyond.  The chain of a thread takes the same time however few
+// particles there are, the rows the longer the more waves they come in: 2D cavities of 10,000,
+// 29,900, 39,600 and 50,200 particles take 9, 17, 22 and 26 us in rows and 18, 20, 20 and 22 us
+// in threads, 3D dam breaks of 9,700, 38,700 and 53,200 particles 24, 67 and 113 us against 73,
+// 77 and 77.
+constexpr int64_t kRowsUpTo = 2 * 152 * 4 * 32;
+// Momentum takes eight lanes a particle while their blocks of 32 particles are all resident at
+// once (four an SM in 2D, three in 3D), a thread a particle beyond: cavities of 10,000, 15,100
+// and 19,900 particles 12.2, 13.5 and 18.9 us in lanes and 13.1, 12.9 and 13.4 us in threads (with
+// the Shepard sums 13.9, 15.6 and 24.6 against 21.7, 21.1 and 22.8), 3D dam breaks of 9,700,
+// 15,000 and 21,900 particles 31, 43 and 53 us against 33, 35 and 36.
+template <int DIM>
+constexpr int64_t kMomentumLanesUpTo = 152 * 32 * (DIM == 3 ? 3 : 4);
+template <int DIM>
+bool momentum_lanes(const LaunchCtx& L) {
+    return L.lanes[1] < 0 ? L.cap <= kMomentumLanesUpTo<DIM> : L.lanes[1] != 0;
+}
 
 template <int DIM, int KK, int MODE>
 void launch_momentum(const LaunchCtx& L) {
     const int sel = L.shepard ? L.force_reinit : L.skip_reinit;
-    if (L.lanes) {
+    if (momentum_lanes<DIM>(L)) {
         auto kernel = L.shepard ? k_momentum_lanes_f32<DIM, KK, MODE, true> : k_momentum_lanes_f32<DIM, KK, MODE, false>;
         launch_dep(kernel, (L.cap + 31) / 32, 256, L.stream, L.scenes, L.st, L.nx, L.wl, L.sc, L.cap, L.bf, L.bs, L.br,
                    L.nl, sel);
@@ -995,13 +1029,11 @@ void launch_momentum(const LaunchCtx& L) {
 }
 
 template <int DIM, int KK>
-void launch_kk(int stage, const LaunchCtx& C) {
-    LaunchCtx L = C;
-    if (L.lanes < 0) L.lanes = L.cap < kLanesBelow;
+void launch_kk(int stage, const LaunchCtx& L) {
     if (stage == 0) {
-        if (L.lanes)
+        if (L.lanes[0] < 0 ? L.cap <= kRowsUpTo : L.lanes[0])
             launch_dep(k_continuity_rows_f32<DIM, KK>, (L.cap + 31) / 32, 256, L.stream, L.scenes, L.st, L.sc, L.cap,
-                       L.bf, L.nl);
+                       L.bf, L.nl, L.wl, !momentum_lanes<DIM>(L));
         else
             launch_dep(k_continuity_f32<DIM, KK>, (L.cap + 127) / 128, 128, L.stream, L.scenes, L.st, L.sc, L.cap, L.bf,
                        L.nl, L.wl);

@@ -34,7 +34,8 @@ struct LaunchCtx {
     int shepard;
     int force_reinit;
     int skip_reinit;
-    int lanes;   // FP32 gathers: 1 lanes share a particle, 0 a thread each, -1 by the particle count
+    // FP32 continuity, momentum: 1 lanes share a particle, 0 a thread each, -1 by the particle count
+    int lanes[2];
     NbrList nl;  // neighbour list of the FP32 form (e null: momentum walks the cells)
     // inlet/outlet buffers (bf.n == nullptr: none): current and next sorted buffers
     BufferState bf, bf2;

@@ -62,3 +62,37 @@ def test_lanes_and_threads_give_the_same_bits(pkg, name):
         beside = bt.download(k)
     for f in alone:
         assert np.array_equal(alone[f], beside[f]), f
+
+
+def beside_medium(name):
+    sc = scenes_mod()
+    d3 = lambda dx: sc.dam_break_3d(dx=dx, tank=(0.6, 0.3, 0.4), column=(0.25, 0.2, 0.3))
+    big = {"dam": lambda: sc.dam_break_2d(dx=0.0085), "squeezed": lambda: sc.dam_break_2d(dx=0.0085),
+           "heat": lambda: sc.natural_convection_2d(n=160), "lid": lambda: sc.lid_driven_cavity_2d(n=160),
+           "periodic": lambda: sc.poiseuille_periodic_2d(n_across=80), "dam_3d": lambda: d3(0.0088),
+           "squeezed_3d": lambda: d3(0.0088)}[name]()
+    return pair(name)[0], developed(big)
+
+
+@pytest.mark.parametrize("name", ["dam", "squeezed", "heat", "lid", "periodic", "dam_3d", "squeezed_3d"])
+def test_rows_with_momentum_threads_give_the_same_bits(pkg, name):
+    # launches of 19,457 (3D: 14,593) to 39,999 particles: continuity in lanes, which lists the
+    # particles near walls and without a list for momentum's threads
+    from ethersph_gb300 import batch
+    a, big = beside_medium(name)
+    assert 20_000 < big.n_fluid and a.n_fluid + big.n_fluid < 40_000
+    with pkg.Simulation(a.params(precision=1), a.n_fluid, a.n_wall) as sim:
+        for w in a.walls:
+            sim.upload_walls(w)
+        sim.upload_fluid(a.fluid)
+        sim.step(1, 5)
+        alone = sim.download()
+    need = [batch.footprint(s, 1) for s in (a, big)]
+    with batch.Batch(a.params(precision=1), *[sum(n[k] for n in need) + 8 for k in range(3)], 4) as bt:
+        bt.add_scene(big, 1, 5)
+        k = bt.add_scene(a, 1, 5)
+        bt.step(5)
+        bt.synchronize()
+        beside = bt.download(k)
+    for f in alone:
+        assert np.array_equal(alone[f], beside[f]), f
