@@ -788,8 +788,9 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
 // end before the walks).  Both together against one after the other: 17.0 against 24.1 us on
 // a 65,536-particle cavity (54 -> 47 us a step), 216 against 228 on a million particles,
 // 315 against 330 on a 432,000-particle 3D dam break (before the eight sums: 25.7, 254, 488).
-// The Shepard sums are a second pass over the list: 385 us with them at a million particles
-// (684 in lanes, 330 before, when the walk of the cells formed them).
+// The Shepard sums are one FP64 sum each, in the list's order: 320 us with them at a million
+// particles, 457 on the 3D dam break (eight sums each, in a second pass over the list: 385 and
+// 633; before: 330 and 533).
 template <int DIM, int KK, int MODE, bool SHEP>
 __global__ void __launch_bounds__(128, 4)
     k_momentum_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl, SortScratch sc,
@@ -811,6 +812,7 @@ __global__ void __launch_bounds__(128, 4)
     const SelfF a = self_f<DIM, KK, HEAT>(S, st, i);
     const int count = nl.e ? nl.n[i] : kListWalk;
     SumsF<DIM, HEAT> acc[kCoopLanes];
+    double sw = 0.0, sws = 0.0;  // Shepard sums, in the list's order
     if (count != kListWalk) {
         // the next eight entries are loaded before the current eight are processed
         const int32_t* entry = nl.e + i;
@@ -831,31 +833,16 @@ __global__ void __launch_bounds__(128, 4)
                 const int j = i + (code[u] >> 9);
                 const float4 r = listed<DIM>(code[u], a.x, __ldg(st.fa + j), j, S);
                 float t[DIM + 1];
-                pair_terms<DIM, KK, HEAT>(S, st, a, r, __ldg(st.fb + j), __ldg(st.fc + j), t);
-                if (k + u < count) acc[u].add(t);
+                const float w = pair_terms<DIM, KK, HEAT>(S, st, a, r, __ldg(st.fb + j), __ldg(st.fc + j), t);
+                if (k + u < count) {
+                    acc[u].add(t);
+                    if constexpr (SHEP) shepard_terms(S, st, w, j, sw, sws);
+                }
             }
         }
     }
 #pragma unroll
     for (int u = 1; u < kCoopLanes; ++u) acc[0].merge_in(acc[u]);
-    double sw = 0.0, sws = 0.0;
-    if constexpr (SHEP) {  // the Shepard sums, in a second pass over the list
-        double w8[kCoopLanes] = {}, ws8[kCoopLanes] = {};
-        const int32_t* entry = nl.e + i;
-        const int entries = count != kListWalk ? count : 0;
-#pragma unroll 1
-        for (int k = 0; k < entries; k += kCoopLanes)
-#pragma unroll
-            for (int u = 0; u < kCoopLanes; ++u) {
-                const int32_t code = k + u < entries ? __ldg(entry + (k + u) * nl.stride) : 0;
-                const int j = i + (code >> 9);
-                const PairF<DIM, KK> p(listed<DIM>(code, a.x, __ldg(st.fa + j), j, S), S);
-                if (k + u < entries) shepard_terms(S, st, p.w, j, w8[u], ws8[u]);
-            }
-        // (the order of coop_sum)
-        sw = ((w8[0] + w8[1]) + (w8[2] + w8[3])) + ((w8[4] + w8[5]) + (w8[6] + w8[7]));
-        sws = ((ws8[0] + ws8[1]) + (ws8[2] + ws8[3])) + ((ws8[4] + ws8[5]) + (ws8[6] + ws8[7]));
-    }
     pdl_wait();
     if (count == kListWalk || (wl.n > 0 && wl.near[st.cell[i]])) {  // the cell walks (k_walks_f32)
         const float2* in = sc.walk_sums + (int64_t)i * (2 * kSums + 2);
@@ -908,7 +895,7 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
         pdl_wait();
         a.f = st.fc[i];
         SumsF<DIM, HEAT> sum;
-        double sw = 0.0, sws = 0.0;  // Shepard sums (ReconstructValue.jl:28-50), FP64
+        double sw = 0.0, sws = 0.0;  // Shepard sums of a walked particle, by lane
         const int count = on ? (nl.e ? nl.n[i] : kListWalk) : 0;
         auto shepard = [&](float w, int j) { if constexpr (SHEP) shepard_terms(S, st, w, j, sw, sws); };
         if (count != kListWalk && lane < count) {
@@ -933,8 +920,7 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
                     if (k + 2 * kCoopLanes < count) next = __ldg(entry += ahead);
                 }
                 float t[DIM + 1];
-                const float w = pair_terms<DIM, KK, HEAT>(S, st, a, r, vj, fj, t);
-                shepard(w, __float_as_int(r.w));
+                pair_terms<DIM, KK, HEAT>(S, st, a, r, vj, fj, t);
                 sum.add(t);
                 if (!more) break;
                 k += kCoopLanes;
@@ -949,8 +935,31 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
             if (walk && lane == 0) sum = fluid;
         }
         if constexpr (SHEP) {
+            // in the list's order, as a thread of k_momentum_f32 adds them: the lanes form eight
+            // kernel values, lane 0 adds W vol and lane 1 W m
+            const int entries = walk ? 0 : count;
+            const int most = (int)__reduce_max_sync(full, (unsigned)entries);
+            double s = 0.0;
+            for (int k0 = 0; k0 < most; k0 += kCoopLanes) {
+                const int k = k0 + lane;
+                const int32_t code = k < entries ? __ldg(nl.e + i + k * nl.stride) : 0;
+                const int j = i + (code >> 9);
+                const PairF<DIM, KK> p(listed<DIM>(code, a.x, __ldg(st.fa + j), j, S), S);
+                const double W = (double)__fmul_rn(S.kw_a_f, p.w), vol = st.vol[j], m = st.m[j];
+#pragma unroll
+                for (int e = 0; e < kCoopLanes; ++e) {
+                    const double We = __shfl_sync(full, W, e, kCoopLanes), ve = __shfl_sync(full, vol, e, kCoopLanes),
+                                 me = __shfl_sync(full, m, e, kCoopLanes);
+                    if (k0 + e < entries) s = fma(We, lane == 1 ? me : ve, s);
+                }
+            }
+            const double lw = __shfl_sync(full, s, 0, kCoopLanes), lws = __shfl_sync(full, s, 1, kCoopLanes);
             sw = coop_sum(sw);
             sws = coop_sum(sws);
+            if (!walk) {
+                sw = lw;
+                sws = lws;
+            }
         }
 #pragma unroll
         for (int k = 0; k < DIM; ++k) sums[(k * kParts + lane) * kSumStride + g] = make_float2(sum.dv[k].s, sum.dv[k].c);
@@ -1002,9 +1011,8 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
 constexpr int64_t kRowsUpTo = 2 * 152 * 4 * 32;
 // Momentum takes eight lanes a particle while their blocks of 32 particles are all resident at
 // once (four an SM in 2D, three in 3D), a thread a particle beyond: cavities of 10,000, 15,100
-// and 19,900 particles 12.2, 13.5 and 18.9 us in lanes and 13.1, 12.9 and 13.4 us in threads (with
-// the Shepard sums 13.9, 15.6 and 24.6 against 21.7, 21.1 and 22.8), 3D dam breaks of 9,700,
-// 15,000 and 21,900 particles 31, 43 and 53 us against 33, 35 and 36.
+// and 19,900 particles 12.2, 13.5 and 18.9 us in lanes and 13.1, 12.9 and 13.4 us in threads, 3D
+// dam breaks of 9,700, 15,000 and 21,900 particles 31, 43 and 53 us against 33, 35 and 36.
 template <int DIM>
 constexpr int64_t kMomentumLanesUpTo = 152 * 32 * (DIM == 3 ? 3 : 4);
 template <int DIM>
