@@ -39,17 +39,14 @@ sys.path.insert(0, str(ROOT))
 METRIC = "particle-steps/s"
 MEASURED_PEAKS = ROOT / "MEASURED_PEAKS.json"
 FALLBACK_HBM_GBS = 6800.0
-LANES_LIST = 16  # SPH_LANES_LIST: momentum lanes codes >= 15 read the neighbour list
 # Counters of one launch of each gather on the default workload (n=256, FP32-compensated)
-# from ncu --set full --clock-control none (cold L2, as the bench's flushed steps), per
+# from ncu --clock-control none (cold L2, as the bench's flushed steps), per
 # launch shape captured (continuity lanes, momentum lanes, block; the third entry of a
 # shape is unused): DRAM bytes read + written, issue-active fraction and FP64-pipe
 # fraction.
 NCU_256 = {
-    ("-1,18,128", "continuity"): {"traffic": 3.99616e6, "issue_active": 0.400, "fp64_pipe": 0.145},
-    ("-1,18,128", "momentum"): {"traffic": 15.517184e6, "issue_active": 0.410, "fp64_pipe": 0.304},
-    ("-1,18,64", "continuity"): {"traffic": 3.996416e6, "issue_active": 0.411, "fp64_pipe": 0.142},
-    ("-1,18,64", "momentum"): {"traffic": 15.513856e6, "issue_active": 0.419, "fp64_pipe": 0.300},
+    ("1,1,128", "continuity"): {"traffic": 4.062464e6, "issue_active": 0.365, "fp64_pipe": 0.141},
+    ("1,1,128", "momentum"): {"traffic": 15.519488e6, "issue_active": 0.432, "fp64_pipe": 0.177},
 }
 
 
@@ -258,6 +255,16 @@ def scan_launches(cells):
     return 1 if cells <= 64 * 4096 else 3
 
 
+def gather_launches(scene, precision, launch_shape, autotuned):
+    """Kernels of a step's gathers: continuity and momentum, and on large FP32 scenes (a
+    thread a particle in momentum) the wall walks."""
+    if precision != 1:
+        return 2
+    one_wave = 152 * 32 * (3 if scene.params().dim == 3 else 4)
+    threads = launch_shape[1] == 1 if autotuned else scene.n_fluid > one_wave
+    return 3 if threads else 2
+
+
 def grid_cells(scene, precision):
     """Cells of the scene's grid, as the library builds it."""
     from ethersph_gb300 import batch
@@ -449,7 +456,7 @@ def run_ours(args, rank, world, local):
     hbm = hbm or FALLBACK_HBM_GBS
     pairs_ff, pairs_fw = sim.count_pairs()
     sim.close()
-    uses_list = args.precision == "fp32c" and launch_shape[1] >= LANES_LIST - 1
+    uses_list = args.precision == "fp32c"  # continuity records the neighbour list, momentum reads it
     entries = 2.0 * pairs_ff / scene.n_fluid if uses_list else 0.0
     shape_key = f"{launch_shape[0]},{launch_shape[1]},{launch_shape[3]}"
 
@@ -469,13 +476,13 @@ def run_ours(args, rank, world, local):
             "neighbour_list_bytes_per_launch": (4 + 4 * entries) * scene.n_fluid if uses_list else 0,
             "launch_ms": stages[stage],
             "traffic": ncu["traffic"] if ncu else None,
-            "traffic_source": (f"ncu --set full of this launch at n=256 and this launch shape ({shape_key}): "
+            "traffic_source": (f"ncu of this launch at n=256 and this launch shape ({shape_key}): "
                                "dram__bytes_read.sum + dram__bytes_write.sum" if ncu else
                                f"no capture at this launch shape ({shape_key})"),
             "issue_frac": ncu["issue_active"] if ncu else None,
             "fp64_pipe_frac": ncu["fp64_pipe"] if ncu else None,
             "limiter": ("FP64 ALU (FP64 at 1/64 of the FP32 rate on GB300)" if args.precision == "fp64" else
-                        "issue/latency: dependent neighbour loads and pair arithmetic on 13-23 warps per SM; "
+                        "issue/latency: dependent neighbour loads and pair arithmetic on 13 warps per SM; "
                         "DRAM reads at or below the algorithmic bytes"),
         }
 
@@ -528,9 +535,11 @@ def run_ours(args, rank, world, local):
         "configs": configs,
         "launch_shape": {"continuity_lanes": launch_shape[0], "momentum_lanes": launch_shape[1],
                          "block": launch_shape[3], "chosen_by": chosen_by},
-        # per step: continuity, momentum (with the Shepard sums on re-initialisation steps),
-        # scan (1 kernel up to 262,144 cells, else 3), fill, placement
-        "gpu_launches": args.steps * (4 + scan_launches(grid_cells(scene, prec))),
+        # per step: continuity, the wall walks of a large FP32 scene, momentum (with the Shepard
+        # sums on re-initialisation steps), scan (1 kernel up to 262,144 cells, else 3), fill,
+        # placement
+        "gpu_launches": args.steps * (2 + gather_launches(scene, prec, launch_shape, chosen_by == "sph_autotune") +
+                                      scan_launches(grid_cells(scene, prec))),
         "clocks": clocks,
     }
     return out

@@ -179,7 +179,7 @@ class Batch:
         self._check(self.lib.sph_set_launch_shape(self.h, shape))
 
     def set_stencil_pruning(self, on: bool) -> None:
-        """FP32 walks skip neighbour cells beyond r_cut (default: 3D on, 2D off); the
+        """FP32 walks skip neighbour cells beyond r_cut (default: on); the
         results are bitwise the same either way."""
         self._check(self.lib.sph_set_stencil_pruning(self.h, 1 if on else 0))
 

@@ -1890,6 +1890,7 @@ int32_t sph_set_launch_shape(SphHandle* h, const int32_t* shape) {
     if ((shape[1] == -1 || shape[1] == SPH_LANES_LIST - 1) && shape[3] > 256)
         return fail(h, SPH_ERR_ARG, "the pipelined momentum walk (-1) takes blocks of at most 256 threads");
     for (int k = 0; k < 4; ++k) h->tune[k] = shape[k];
+    h->lanes[0] = h->lanes[1] = -1;  // no longer the autotuner's pick
     for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second);
     h->graphs.clear();
     return SPH_OK;

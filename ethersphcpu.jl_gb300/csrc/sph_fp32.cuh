@@ -21,9 +21,9 @@
 // on the variant, the batch or the pruning.
 //
 // What bounds them: on small scenes the chain of loads and rounds of one particle, on large
-// ones the issue of instructions (continuity issues in 73 of 100 cycles, momentum in 43 to 54
-// with 16 warps an SM for its eight sums, waiting on neighbours from L2); the bytes would take
-// a fifth of the time.
+// ones the issue of instructions (continuity issues in 66 to 76 of 100 cycles, momentum in 43
+// to 57 with 15 warps an SM for its eight sums, waiting on neighbours from L2); the bytes would
+// take a sixth of the time.
 //
 // On a re-initialisation step the momentum gather also forms the Shepard sums over the
 // same neighbours and writes the re-initialised density: the update and the

@@ -78,12 +78,10 @@ def summarize_ranks(report: Report, world: int = 1) -> dict:
     }
 
 
-# Launch shape of the FP32-compensated form in a served batch: continuity on one pipelined
-# lane recording the neighbour list, momentum reading it on two lanes, 128-thread blocks.
-# Fixed (not re-tuned as the mix changes): a served result equals the same scene run alone
-# at this shape, and on GB300 the fixed list shape served the bench's 48-request stream
-# faster (500 M particle-steps/s, p50 6.0 s) than re-tuning whenever the live particles
-# doubled (458 M/s, p50 6.7 s: the tuning launches cost more than they won).
+# Launch shape of the FP32-compensated form in a served batch.  The library takes it and
+# chooses its kernels by the live particles (the results do not depend on the choice);
+# re-tuning whenever they doubled cost more than it won (458 against 500 M particle-steps/s
+# on the 48-request stream).
 DEFAULT_LAUNCH_SHAPE = (-1, _abi.LANES_LIST + 2, -1, 128)
 
 
@@ -96,8 +94,8 @@ class Server:
         self.precision = precision
         self.keep_results = keep_results
         # re-tune a batch's launch shape (sph_autotune) whenever its live particles have
-        # doubled since the last tuning; off by default, because the FP32 form's results
-        # depend on the shape and a served result should equal the same scene run alone
+        # doubled since the last tuning; off by default: the trial launches cost more than
+        # they win
         self.autotune = autotune and launch_shape is None and precision == _abi.PRECISION_FP32_COMPENSATED
         if launch_shape is None and not self.autotune and precision == _abi.PRECISION_FP32_COMPENSATED:
             launch_shape = DEFAULT_LAUNCH_SHAPE

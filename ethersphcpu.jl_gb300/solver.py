@@ -223,7 +223,7 @@ class Simulation:
         self._check(self.lib.sph_set_launch_shape(self.h, shape))
 
     def set_stencil_pruning(self, on: bool) -> None:
-        """FP32 walks skip neighbour cells beyond r_cut (default: 3D on, 2D off); the
+        """FP32 walks skip neighbour cells beyond r_cut (default: on); the
         results are bitwise the same either way."""
         self._check(self.lib.sph_set_stencil_pruning(self.h, 1 if on else 0))
 
@@ -371,8 +371,8 @@ def solve(fluid, *args, check=None, vtp_io=None, precision: int = _abi.PRECISION
     downloads the state and writes the file here.  `domain_lo/hi` bound the cell grid
     (default: the particles' bounding box grown by two cut-off radii; particles leaving
     it are clamped into the edge cells, which stays exact but slower).  `autotune` picks
-    the FP32-compensated form's launch shape on the uploaded scene (sph_autotune); the
-    form's results depend on the shape in the last bits, so it is off by default.
+    the FP32-compensated form's kernel variants by timing them on the uploaded scene
+    (sph_autotune) instead of by the number of particles; the results are the same.
     """
     *walls, kernel, model, td = args
     for w in walls:

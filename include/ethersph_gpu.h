@@ -326,47 +326,38 @@ int32_t sph_batch_free(SphHandle* h, int64_t* out);
 int32_t sph_count_pairs_noalloc(const SphParams* params, int64_t n, const double* x, int64_t n_wall,
                                 const double* wall_x, int64_t* counts, void* stream);
 
-/* Autotuner of the FP32-compensated form: times the continuity and momentum gathers on
- * the current state for every lanes-per-particle count {-1, 1, 2, 4, 8} and block size
- * {64, 128, 256}, and the neighbour-list pair (continuity recording the list with lanes
- * {-1, 1, 2}, momentum reading it with lanes {-1, 1, 2, 4}); keeps the faster of the
- * cell-walk and list pairs and rebuilds the step graphs.  out[4] (may be NULL) receives
- * the launch shape (see sph_set_launch_shape).  The fluid state is left unchanged.  No-op
- * for the FP64 form, which keeps one thread per particle so that its summation order is
- * fixed. */
+/* Autotuner of the FP32-compensated form: times the gathers on the current state with
+ * eight lanes sharing a particle in both, in continuity only, and with a thread a particle,
+ * keeps the fastest and rebuilds the step graphs.  Without it the choice follows the number
+ * of particles.  The results are bitwise the same whichever runs.  out[4] (may be NULL)
+ * receives (continuity lanes, momentum lanes, 1, block size): lanes 8 or 1, blocks of 256 or
+ * 128.  The fluid state is left unchanged.  No-op for the FP64 form. */
 int32_t sph_autotune(SphHandle* h, int32_t reps, int32_t* out);
 
 /* Momentum lanes code of the neighbour list: SPH_LANES_LIST + t, t in {1, 2, 4, -1}.
- * The continuity gather (one or two lanes per particle) records, in its walk order, every
- * neighbour within r_cut of each particle (two lanes: each lane its share of the
- * candidates, lane 0 from the list's first entry up, lane 1 from its last entry down),
- * and the momentum gather of the same step reads
- * that list with t lanes per particle instead of walking the cells a second time (same
- * pairs: positions do not change between the two gathers).  The list holds about
- * 1.25 x the lattice neighbour count of the finest uploaded spacing per particle
- * (4 bytes each, grown with the live particle count); a particle with more neighbours
- * walks the cells. */
+ * The FP32 form always runs with the list: the continuity gather records, in its walk
+ * order, every neighbour within r_cut of each particle, and the momentum gather of the same
+ * step reads that list instead of walking the cells a second time (same pairs: positions do
+ * not change between the two gathers).  The list holds about 1.25 x the lattice neighbour
+ * count of the finest uploaded spacing per particle (4 bytes each, grown with the live
+ * particle count); a particle with more neighbours, and every particle where there is no
+ * memory for the list, walks the cells. */
 #define SPH_LANES_LIST 16
 
 /* Set the FP32 launch shape by hand (a new handle starts at (1, 1, 1, 128)):
- * shape[4] = (continuity lanes, momentum lanes, unused, block size).  shape[2] is kept for
- * the layout and must be a lanes code: the Shepard sums of a re-initialisation step run
- * inside the momentum gather, at its lanes.  Lanes in {1, 2, 4, 8} or -1 (one lane whose candidate loop
- * is software-pipelined: loads of the next neighbour overlap the current one's
- * arithmetic; momentum lanes -1 take blocks of at most 256), block in {32, 64, ..., 1024}
- * and a multiple of 32.  Momentum lanes may instead be a neighbour-list code
- * (SPH_LANES_LIST + 1, 2, 4 or -1; continuity lanes 1, 2 or -1 then).  Results of the FP32
- * form depend on the lanes codes (the order of the compensated partial sums, and for -1
- * against 1 the compiler's contraction of a*b+c into fused multiply-adds), never on the
- * block size. */
+ * shape[4] = (continuity lanes, momentum lanes, unused, block size).  Kept for callers that
+ * set one: the codes are checked as ever (lanes 1, 2, 4, 8 or -1; momentum lanes also
+ * SPH_LANES_LIST + 1, 2, 4 or -1 with continuity lanes 1, 2 or -1; blocks of a multiple of 32
+ * up to 1024, up to 256 with momentum lanes -1) and reported by sph_autotune, but one set of
+ * kernels serves them all: the variant follows the number of particles again (an autotuned
+ * choice is dropped) and the results do not depend on the shape. */
 int32_t sph_set_launch_shape(SphHandle* h, const int32_t* shape);
 
-/* Stencil pruning of the FP32-compensated walks (the FP64 form's walks always prune, with
- * the same bitwise-neutral rule; default: on for 3D scenes, off for 2D,
- * where it does not pay on GB300): for each neighbour row
+/* Stencil pruning of the FP32-compensated walks (the FP64 form's always prune, with
+ * the same bitwise-neutral rule; default: on): for each neighbour row
  * the walk visits only the cells whose extent comes within r_cut of the particle (with a
  * margin of 1e-5 on r_cut^2), instead of all 2m+1 cells of the (2m+1)^dim stencil.  Only
- * candidates the distance test would reject are skipped, so with one lane per particle
+ * candidates the distance test would reject are skipped, so
  * the results are bitwise the same either way.  No counterpart in the reference. */
 int32_t sph_set_stencil_pruning(SphHandle* h, int32_t on);
 
