@@ -7,7 +7,7 @@
 // restatement: the key is the one the step's sort uses, and the neighbour test is the
 // one the gathers of the handle's form use (FP64: d^2 <= r_cut^2 in FP64 with the
 // products and sums rounded one by one, as k_momentum_fp64; FP32-compensated: the same
-// test in FP32 on cell-relative positions, as coop_select takes it; the stencil pruning
+// test in FP32 on cell-relative positions, as the gathers take it; the stencil pruning
 // leaves out only what that test rejects).
 #include "sph_coop.cuh"
 

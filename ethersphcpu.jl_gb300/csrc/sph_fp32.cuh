@@ -7,7 +7,7 @@
 // Kahan-compensated FP32 accumulators; the result (sum - compensation) goes to FP64 before
 // the forward-Euler update, which runs in FP64 on the FP64 master position / velocity /
 // density / temperature.  The Shepard sums accumulate in FP64 (FP32 kernel values times
-// FP64 volumes and masses).
+// FP64 volumes and masses), in the list's order.
 //
 // Continuity walks the cells, one thread a particle on large scenes and a lane a neighbour
 // row on small ones (the same sums, bit for bit), and records each particle's neighbours
@@ -147,7 +147,7 @@ constexpr int kRowEntries = 16;  // list entries of a row (more: momentum walks 
 __device__ __forceinline__ float code_offset(int32_t code, int shift) {  // the offset + 3 as a float
     return __int_as_float(0x4b000000 | (code >> shift & 7)) - (8388608.f + 3.f);
 }
-// r_vec of the listed pair as coop_select forms it, and the neighbour's index.
+// r_vec of the listed pair as run_walk forms it, and the neighbour's index.
 template <int DIM>
 __device__ __forceinline__ float4 listed(int32_t code, const float4& me, const float4& p, int j, const SceneDev& S) {
     const float rx = ((me.x - p.x) - code_offset(code, 0)) * S.cell_f[0];
@@ -158,8 +158,8 @@ __device__ __forceinline__ float4 listed(int32_t code, const float4& me, const f
 
 // -------------------------------------------------------------------- K4 (FP32)
 // The cells of neighbour row (dy, dz) of a particle, as one run [b, e) of the sorted arrays
-// or two where a periodic axis wraps, in x order; cells beyond r_cut are left out (prune)
-// with the margins and exceptions of coop_select.
+// or two where a periodic axis wraps, in x order; cells beyond r_cut are left out (prune) with
+// the margin rc2_prune and the exceptions of coop_select.
 template <int DIM>
 __device__ __forceinline__ void row_runs(const SceneDev& S, const int32_t* __restrict__ start, const int32_t c[3],
                                          const float4& me, bool prune, int dy, int dz, int& b, int& e, int& b2,
