@@ -300,10 +300,10 @@ __device__ __forceinline__ void continuity_update(const SceneDev& S, const Sorte
 // Large scenes: one thread a particle.  A row's terms are one compensated sum and the rows'
 // sums are merged in order; k_continuity_rows_f32 forms the same sums with a lane a row.  The
 // next row's cell starts and the next candidate's data are loaded ahead.  22.2 -> 19.7 us on a
-// 65,536-particle cavity, 170 -> 172 on a million particles (momentum reads the list it records
-// now), 418 -> 359 on a 432,000-particle 3D dam break.
-template <int DIM, int KK>
-__global__ void __launch_bounds__(128) k_continuity_f32(const SceneDev* __restrict__ scenes, SortedState st,
+// 65,536-particle cavity, 170 -> 148 on a million particles (and momentum reads the list it
+// records), 418 -> 349 on a 432,000-particle 3D dam break.
+template <int DIM, int KK, int BLOCKS>
+__global__ void __launch_bounds__(128, BLOCKS) k_continuity_f32(const SceneDev* __restrict__ scenes, SortedState st,
                                                         SortScratch sc, int32_t cap, BufferState bf, NbrList nl,
                                                         WallState wl) {
     pdl_wait();
@@ -1009,6 +1009,20 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
 // in threads, 3D dam breaks of 9,700, 38,700 and 53,200 particles 24, 67 and 113 us against 73,
 // 77 and 77.
 constexpr int64_t kRowsUpTo = 2 * 152 * 4 * 32;
+// Continuity's thread kernel takes 72 registers, seven blocks of 128 an SM; held to 56 (2D: nine
+// blocks) or 64 (3D: eight) it spills a little and is the faster one where that saves a wave:
+// cavities of 144,400 and 1,048,576 particles 36 -> 26 and 163 -> 147 us, 3D dam breaks of 432,000
+// particles 359 -> 348.  With as many waves either way it is not: a step of 202,500 particles
+// 101.2 us against 102.0, of 250,000 in 3D 466 against 469.  Ten (nine) blocks: 158 (352).
+// (Without the bound of seven the compiler takes more registers: 360,000 particles 72 us, not 62.)
+constexpr int kSpread = 7;
+template <int DIM>
+constexpr int kPacked = DIM == 3 ? 8 : 9;
+template <int DIM>
+bool continuity_packed(int64_t blocks) {
+    auto waves = [&](int64_t an_sm) { return (blocks + 152 * an_sm - 1) / (152 * an_sm); };
+    return waves(kPacked<DIM>) < waves(kSpread);
+}
 // Momentum takes eight lanes a particle while their blocks of 32 particles are all resident at
 // once (four an SM in 2D, three in 3D), a thread a particle beyond: cavities of 10,000, 15,100
 // and 19,900 particles 12.2, 13.5 and 18.9 us in lanes and 13.1, 12.9 and 13.4 us in threads, 3D
@@ -1043,8 +1057,9 @@ void launch_kk(int stage, const LaunchCtx& L) {
             launch_dep(k_continuity_rows_f32<DIM, KK>, (L.cap + 31) / 32, 256, L.stream, L.scenes, L.st, L.sc, L.cap,
                        L.bf, L.nl, L.wl, !momentum_lanes<DIM>(L));
         else
-            launch_dep(k_continuity_f32<DIM, KK>, (L.cap + 127) / 128, 128, L.stream, L.scenes, L.st, L.sc, L.cap, L.bf,
-                       L.nl, L.wl);
+            launch_dep(continuity_packed<DIM>((L.cap + 127) / 128) ? k_continuity_f32<DIM, KK, kPacked<DIM>>
+                                                                   : k_continuity_f32<DIM, KK, kSpread>,
+                       (L.cap + 127) / 128, 128, L.stream, L.scenes, L.st, L.sc, L.cap, L.bf, L.nl, L.wl);
         return;
     }
     switch (L.mode) {

@@ -96,3 +96,30 @@ def test_rows_with_momentum_threads_give_the_same_bits(pkg, name):
         beside = bt.download(k)
     for f in alone:
         assert np.array_equal(alone[f], beside[f]), f
+
+
+@pytest.mark.parametrize("name", ["heat", "dam_3d"])
+def test_packed_continuity_gives_the_same_bits(pkg, name):
+    # 136,193 particles or more: continuity's thread kernel with fewer registers, which saves a
+    # wave of blocks here (2D up to 175,104 particles, 3D up to 155,648)
+    from ethersph_gb300 import batch
+    a = pair(name)[0]
+    sc = scenes_mod()
+    big = developed(sc.natural_convection_2d(n=380) if name == "heat" else
+                    sc.dam_break_3d(dx=0.0047, tank=(0.6, 0.3, 0.4), column=(0.25, 0.2, 0.3)))
+    assert 136_193 <= big.n_fluid and a.n_fluid + big.n_fluid <= 155_648
+    with pkg.Simulation(a.params(precision=1), a.n_fluid, a.n_wall) as sim:
+        for w in a.walls:
+            sim.upload_walls(w)
+        sim.upload_fluid(a.fluid)
+        sim.step(1, 5)
+        alone = sim.download()
+    need = [batch.footprint(s, 1) for s in (a, big)]
+    with batch.Batch(a.params(precision=1), *[sum(n[k] for n in need) + 8 for k in range(3)], 4) as bt:
+        bt.add_scene(big, 1, 5)
+        k = bt.add_scene(a, 1, 5)
+        bt.step(5)
+        bt.synchronize()
+        beside = bt.download(k)
+    for f in alone:
+        assert np.array_equal(alone[f], beside[f]), f
