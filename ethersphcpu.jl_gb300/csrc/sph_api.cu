@@ -1092,7 +1092,7 @@ int32_t allocate_state(SphHandle* h, int64_t cells) {
                 {&h->sc.tmp, (size_t)h->cap},        {&h->sc.count, ncell},
                 {&h->sc.start, ncell + 1},           {&h->sc.block_sums, ncell / 1024 + 2},
                 {&h->sc.status, 1},                  {&h->nbuf, 2},
-                {&h->sc.queue, 4},                   {&h->sc.n_walked, 1},
+                {&h->sc.queue, kQueueWords},                   {&h->sc.n_walked, 1},
                 {&h->W.start, ncell + 1},            {&h->W.kind, wc}};
     for (auto& a : ints)
         if ((e = dalloc(h, a.p, a.n)) != cudaSuccess) return cuda_fail(nullptr, e, "scratch");
@@ -1763,6 +1763,9 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
     Lr.shepard = 1;
     Lr.force_reinit = 1;
     const int par = h->par;
+    auto clear_queue = [&] {  // what the placement does between the gathers of two steps
+        if (h->precision == SPH_PRECISION_FP64) cudaMemsetAsync(h->sc.queue, 0, 4 * kQueueWords, st);
+    };
     auto run = [&](int stage) {
         switch (stage) {
             case SPH_STAGE_CELL_COUNT:
@@ -1773,10 +1776,17 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
             case SPH_STAGE_SORT: launch_place(Lh); break;
             case SPH_STAGE_CONTINUITY:
                 cudaMemsetAsync(h->sc.n_walked, 0, 4, st);  // continuity appends to the walked particles
+                clear_queue();
                 launch_physics(0, L);
                 break;
-            case SPH_STAGE_MOMENTUM: launch_physics(1, L); break;
-            case SPH_STAGE_REINIT: launch_physics(1, Lr); break;
+            case SPH_STAGE_MOMENTUM:
+                clear_queue();
+                launch_physics(1, L);
+                break;
+            case SPH_STAGE_REINIT:
+                clear_queue();
+                launch_physics(1, Lr);
+                break;
         }
     };
     for (int stage = 0; stage < SPH_NUM_STAGES; ++stage) {
@@ -1794,6 +1804,7 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
         }
     }
     // the momentum stage left arrivals in count[]: the next step expects it zeroed
+    clear_queue();
     SPH_CUDA(h, cudaMemsetAsync(h->sc.n_walked, 0, 4, st));
     SPH_CUDA(h, cudaMemsetAsync(h->sc.count, 0, sizeof(int32_t) * (size_t)h->scan_cells, st));
     // restore p and c (output-only fields) from the copy the placement stage wrote

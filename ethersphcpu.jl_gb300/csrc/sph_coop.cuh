@@ -426,8 +426,8 @@ inline CoopShape coop_shape(int64_t n) {
 
 // A warp's part of n particles: body(i, p, on) for its group's particle i (clamped to a
 // valid one with on = false past the end), p its place among the warp's next 32; update(i)
-// one lane a particle after each 32 and at the end.  queue[0]: draws beyond every warp's
-// first, queue[1]: blocks that are done (the last one leaves both at 0 for the next launch).
+// one lane a particle after each 32 and at the end.  *queue counts the draws beyond every
+// warp's first: 0 before the launch, a word of the launch's own (SortScratch::queue).
 template <typename Body, typename Update>
 __device__ __forceinline__ void coop_turns(int n, int32_t* queue, Body&& body, Update&& update) {
     const unsigned full = 0xffffffffu;
@@ -451,14 +451,6 @@ __device__ __forceinline__ void coop_turns(int n, int32_t* queue, Body&& body, U
         const int i = __shfl_sync(full, mine, lane / kCoopGroups) * kCoopGroups + lane % kCoopGroups;
         if (i < n) update(i);
         __syncwarp();
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        if (atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
-            queue[0] = 0;
-            queue[1] = 0;
-        }
     }
 }
 

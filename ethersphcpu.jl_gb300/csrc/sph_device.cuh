@@ -177,6 +177,8 @@ struct NbrList {
 constexpr int32_t kListWalk = 0x7fffffff;
 constexpr int32_t kListDelta = 1 << 22;  // |j - i| < kListDelta
 
+enum { kQueueContinuity, kQueueMomentum, kQueueShepard, kQueueWords };  // words of SortScratch::queue
+
 struct SortScratch {
     int32_t* key;    // per particle (unsorted index): global cell key or kDeadKey
     int32_t* slot;   // per particle: arrival slot inside its cell
@@ -186,8 +188,10 @@ struct SortScratch {
     int32_t* block_sums;
     int32_t* n_live;    // device scalar: live particles after the last sort
     int32_t* status;    // device scalar: status bits
-    int32_t* queue;     // draws and finished blocks of a cooperative gather (coop_turns), 0 between launches;
-                        // a pair for continuity, a pair for momentum, which starts beside it
+    // draws of the cooperative gathers (coop_turns), a word for each gather of a step: momentum
+    // draws before its wait, when the gather in front of it may not have ended.  The placement
+    // zeroes them, and every gather of the next step starts after one that waited for it.
+    int32_t* queue;
     // FP32 form, large scenes: the particles whose cells the momentum gather walks, their
     // number (0 before continuity) and their sums of those walks (fluid, walls, Shepard)
     int32_t* walked;

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
             st.vol[i] = m_i / rho;
         }
     };
-    coop_turns(min(cap, *sc.n_live), sc.queue, gather, update);
+    coop_turns(min(cap, *sc.n_live), sc.queue + kQueueContinuity, gather, update);
 }
 
 // SHEP: the momentum gather of density re-initialisation steps, for the particles of the
@@ -563,7 +563,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
             cell_arrival(sc, i, moved_key<DIM>(st.cell[i], st.fa[i], xi, xo, S));
         }
     };
-    coop_turns(min(cap, *sc.n_live), sc.queue + 2, gather, update);
+    coop_turns(min(cap, *sc.n_live), sc.queue + (SHEP ? kQueueShepard : kQueueMomentum), gather, update);
     pdl_wait();
 }
 
