@@ -140,7 +140,7 @@ struct PairF {
     }
 };
 
-constexpr int kRowEntries = 16;  // list entries of a row (more: momentum walks the cells for the particle)
+constexpr int kRowEntries = 16;  // neighbours of a row that k_continuity_rows_f32 keeps in shared memory
 
 // List entry of neighbour j of i in the cell (dx, dy, dz) away: (j - i) << 9 | (dz + 3) << 6 |
 // (dy + 3) << 3 | (dx + 3).
@@ -320,7 +320,6 @@ __global__ void __launch_bounds__(128, BLOCKS) k_continuity_f32(const SceneDev* 
     const int room = fits ? nl.kmax : 0;
     int32_t* entry = nl.e + i;
     int cnt = 0;
-    bool listed_all = fits;
     Kahan total;
     auto emit = [&](int32_t code) {
         if (cnt < room) {
@@ -340,7 +339,6 @@ __global__ void __launch_bounds__(128, BLOCKS) k_continuity_f32(const SceneDev* 
             row_runs<DIM>(S, sc.start, c, me, prune, turn ? -S.reach : dy + 1, turn ? (DIM == 3 ? dz + 1 : 4) : dz, nb,
                           ne, nb2, ne2);
             Kahan row;
-            const int before = cnt;
             const int tag = (dz + 3) << 6 | (dy + 3) << 3;
 #pragma unroll 1
             while (b < e) {
@@ -350,14 +348,13 @@ __global__ void __launch_bounds__(128, BLOCKS) k_continuity_f32(const SceneDev* 
                 b2 = e2 = 0;
             }
             merge(total, row.s, row.c);
-            listed_all &= cnt - before <= kRowEntries;
             b = nb;
             e = ne;
             b2 = nb2;
             e2 = ne2;
         }
     }
-    const bool walk = !(listed_all && cnt <= room);
+    const bool walk = !(fits && cnt <= room);
     if (nl.e) nl.n[i] = walk ? kListWalk : cnt;
     if (walk || (wl.n > 0 && wl.near[st.cell[i]])) sc.walked[atomicAdd(sc.n_walked, 1)] = i;
     continuity_update<DIM, KK>(S, st, bf, i, make_float2(total.s, total.c));
@@ -399,6 +396,7 @@ __global__ void __launch_bounds__(256) k_continuity_rows_f32(const SceneDev* __r
             const int dy = lane - 3;
             int b = 0, e = 0, b2 = 0, e2 = 0, cnt = 0;
             if (on && lane < 7) row_runs<DIM>(S, sc.start, c, me, prune, dy, dz, b, e, b2, e2);
+            const int first = b, first_end = e, second = b2, second_end = e2;
             Kahan row;
             const int tag = (dz + 3) << 6 | lane << 3;
 #pragma unroll 1
@@ -424,10 +422,23 @@ __global__ void __launch_bounds__(256) k_continuity_rows_f32(const SceneDev* __r
                 if (lane >= o) end += v;
             }
             const int all = __shfl_sync(full, end, kCoopLanes - 1, kCoopLanes);
-            const bool small = __ballot_sync(full, cnt > kRowEntries) >> ((threadIdx.x & 31) - lane) << 24 == 0;
-            fits &= small && count + all <= nl.kmax;
-            if (fits)
-                for (int q = 0; q < cnt; ++q) nl.e[(int64_t)(count + end - cnt + q) * nl.stride + i] = mine[q * 256];
+            fits &= count + all <= nl.kmax;
+            if (fits) {
+                int32_t* entry = nl.e + (int64_t)(count + end - cnt) * nl.stride + i;
+                if (cnt <= kRowEntries) {
+                    for (int q = 0; q < cnt; ++q, entry += nl.stride) *entry = mine[q * 256];
+                } else {  // a long row (wide cells, or a spacing far below r_cut): walked again
+                    auto list_run = [&](int j, int e) {
+                        run_walk<DIM>(S, st.fa, i, me, j, e, (float)dy, (float)dz, [](int) { return 0; },
+                                      [&](int q, const float4&, int dx3, int) {
+                                          *entry = (int32_t)((uint32_t)(q - i) << 9) | tag | dx3;
+                                          entry += nl.stride;
+                                      });
+                    };
+                    list_run(first, first_end);
+                    list_run(second, second_end);
+                }
+            }
             count += all;
         }
         if (lane == 0) {
