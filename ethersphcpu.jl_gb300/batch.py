@@ -64,14 +64,18 @@ def footprint(scene, precision: int = _abi.PRECISION_FP64) -> tuple[int, int, in
 
 
 def bytes_per(dim: int, thermal: bool, precision: int) -> tuple[int, int, int]:
-    """Device bytes per particle, per cell and per wall particle of a batch handle."""
+    """Device bytes per particle, per cell and per wall particle of a batch handle, with the
+    neighbour list the FP32-compensated form allocates when it steps (its depth at r_cut = 3
+    spacings: 48 entries in 2D, 168 in 3D)."""
     vec = 16 if dim == 2 else 32
     scal = 7 + (3 if thermal else 0)
     per_sorted = 2 * vec + 8 * scal + 8 + 16 + 4 + 8
     if precision == _abi.PRECISION_FP32_COMPENSATED:
         per_sorted += 2 * 16
     sums = 2 * (dim + (1 if thermal else 0)) + 2 if precision == _abi.PRECISION_FP32_COMPENSATED else 0
-    particle = 2 * per_sorted + 2 * vec + 8 + (8 if thermal else 0) + 12 + 8 * sums + (4 if sums else 0)
+    particle = 2 * per_sorted + 2 * vec + 8 + (8 if thermal else 0) + 12
+    if sums:
+        particle += 8 * sums + 4 + 4 * (48 if dim == 2 else 168) + 4
     cell = 4 * 3 + 1
     wall = 3 * vec + 3 * 8 + 4 + (52 if precision == _abi.PRECISION_FP32_COMPENSATED else 16)
     return particle, cell, wall
