@@ -366,7 +366,7 @@ struct SphHandle {
     int tune[4] = {1, 1, 1, 128};
     int lanes[2] = {-1, -1};
     NbrList nl{};          // neighbour list of the FP32 form (ensure_list)
-    bool no_list = false;  // no room for it
+    bool list_short = false;  // no room for it, or not at its full depth (until the particles or scenes change)
     // stencil pruning of the FP32 gathers (sph_set_stencil_pruning), on by default: the rows
     // of a particle's stencil are bounded by its eight lanes together
     int prune = 1;
@@ -496,14 +496,18 @@ int32_t list_depth_for(int dim, double rc2, double gap) {
 }
 
 // Storage of the neighbour list of the FP32 form for the current per-particle grid and scene
-// depths; a larger one replaces it (and the captured graphs, which hold its address).  A
-// device without room for it leaves the momentum gather walking the cells.
+// depths; a larger one replaces it (and the captured graphs, which hold its address).  On a
+// device without room for that it is as deep as before (a particle with more neighbours
+// walks the cells), or there is none and momentum walks the cells for every particle;
+// sph_last_error then says so, and a larger one is tried again when the particles or scenes
+// change.
 int32_t ensure_list(SphHandle* h) {
-    if (h->precision != SPH_PRECISION_FP32_COMPENSATED || h->no_list) return SPH_OK;
+    if (h->precision != SPH_PRECISION_FP32_COMPENSATED) return SPH_OK;
+    const int64_t rows = grid_rows(h);
+    if (h->list_short && (!h->nl.e || rows <= h->nl.stride)) return SPH_OK;
     int32_t depth = 8;
     for (const SceneRec& R : h->scenes)
         if (R.used) depth = std::max(depth, R.list_depth);
-    const int64_t rows = grid_rows(h);
     if (h->nl.e && rows <= h->nl.stride && depth <= h->nl.kmax) return SPH_OK;
     // rows grow by half again at least: a serving batch raises its live bound scene by scene
     int64_t stride = std::max<int64_t>(std::max<int64_t>(rows, h->nl.stride), 1);
@@ -511,22 +515,33 @@ int32_t ensure_list(SphHandle* h) {
         stride = std::max<int64_t>(stride, std::min<int64_t>(h->cap, h->nl.stride + h->nl.stride / 2));
     depth = std::max(depth, h->nl.kmax);
     SPH_CUDA(h, cudaStreamSynchronize(h->stream));
+    const int32_t had = h->nl.kmax;
     if (h->nl.e) cudaFree(h->nl.e);
     if (h->nl.n) cudaFree(h->nl.n);
     h->nl = NbrList{};
     for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second);
     h->graphs.clear();
-    cudaError_t e = cudaMalloc((void**)&h->nl.e, (size_t)stride * (size_t)depth * 4);
-    if (e == cudaSuccess) e = cudaMalloc((void**)&h->nl.n, (size_t)stride * 4);
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        if (h->nl.e) cudaFree(h->nl.e);
-        h->nl = NbrList{};
-        h->no_list = true;
-        return SPH_OK;
-    }
-    h->nl.kmax = depth;
-    h->nl.stride = stride;
+    auto got = [&](int64_t rows_, int32_t depth_) {
+        NbrList nl{};
+        cudaError_t e = cudaMalloc((void**)&nl.e, (size_t)rows_ * (size_t)depth_ * 4);
+        if (e == cudaSuccess) e = cudaMalloc((void**)&nl.n, (size_t)rows_ * 4);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            if (nl.e) cudaFree(nl.e);
+            return false;
+        }
+        nl.kmax = depth_;
+        nl.stride = rows_;
+        h->nl = nl;
+        return true;
+    };
+    const int64_t least = std::max<int64_t>(rows, 1);
+    if (got(stride, depth) || (stride > least && got(least, depth))) return SPH_OK;
+    h->list_short = true;
+    const bool some = had > 0 && had < depth && got(least, had);
+    h->err = some ? "no device memory for the whole neighbour list: particles with more than " + std::to_string(had) +
+                        " neighbours walk the cells"
+                  : "no device memory for the neighbour list: momentum walks the cells";
     return SPH_OK;
 }
 
@@ -637,6 +652,7 @@ bool is_step_host(int64_t step, int64_t interval) { return interval > 0 && step 
 
 // New bound on the live particles; the captured step graphs bake the grid sizes.
 void set_n_upper(SphHandle* h, int64_t n) {
+    h->list_short = false;  // called whenever particles or scenes come or go
     if (n != h->n_upper) {
         for (auto& kv : h->graphs) cudaGraphExecDestroy(kv.second);
         h->graphs.clear();

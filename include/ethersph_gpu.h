@@ -340,8 +340,10 @@ int32_t sph_autotune(SphHandle* h, int32_t reps, int32_t* out);
  * step reads that list instead of walking the cells a second time (same pairs: positions do
  * not change between the two gathers).  The list holds about 1.25 x the lattice neighbour
  * count of the finest uploaded spacing per particle (4 bytes each, grown with the live
- * particle count); a particle with more neighbours, and every particle where there is no
- * memory for the list, walks the cells. */
+ * particle count); a particle with more neighbours walks the cells.  Without memory for it
+ * the list keeps its former depth or, if not even that fits, every particle walks the cells,
+ * which takes longer; sph_last_error then says so, and the allocation is tried again once
+ * fluid is uploaded or a scene added or retired. */
 #define SPH_LANES_LIST 16
 
 /* Set the FP32 launch shape by hand (a new handle starts at (1, 1, 1, 128)):
@@ -458,7 +460,9 @@ int32_t sph_output_write(SphHandle* h, int64_t file_step, double time);
 /* Wait until every queued file is on disk; returns the first write error (SPH_ERR_IO). */
 int32_t sph_output_flush(SphHandle* h);
 
-/* Text of the last error on this handle (or of the last failed sph_create when h is NULL). */
+/* Text of the last error on this handle (or of the last failed sph_create when h is NULL).  A
+ * step of the FP32 form that found no memory for its neighbour list (SPH_LANES_LIST) succeeds
+ * and leaves a note here. */
 const char* sph_last_error(const SphHandle* h);
 
 /* Free all device memory of the handle. */
