@@ -967,10 +967,19 @@ void ascending_id_order(const std::vector<int32_t>& ids, std::vector<int32_t>& o
     std::sort(order.begin(), order.end(), [&](int32_t a, int32_t b) { return ids[a] < ids[b]; });
 }
 
+// Host memory that is not page-locked, registered or managed.
+bool pageable(const void* p) {
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) == cudaSuccess) return a.type == cudaMemoryTypeUnregistered;
+    cudaGetLastError();
+    return false;
+}
+
 // Download the live particles of scene s in ascending id: the rows are put in that order
 // on the device (one gather launch into a staging buffer), then the requested arrays are
-// copied straight into the caller's memory, those that lie one behind the other there (as
-// Batch.download lays them out) as one: a pageable copy costs 10-15 us however small.
+// copied straight into the caller's memory, pageable ones that lie one behind the other there
+// (as Batch.download lays them out) as one: a pageable copy costs 10-15 us however small.
+// Page-locked arrays that touch may be allocations of their own, which one copy must not span.
 int32_t download_scene(SphHandle* h, int s, int64_t capacity, int64_t* n_out, double* x, double* v, double* rho,
                        double* p, double* c, double* mass, double* gap, double* t, double* kappa, double* cp,
                        int64_t* ids_out) {
@@ -1027,7 +1036,8 @@ int32_t download_scene(SphHandle* h, int s, int64_t capacity, int64_t* n_out, do
     } part[10] = {};
     int parts = 0;
     auto add = [&](double* to, size_t words) {
-        if (parts && (uintptr_t)(part[parts - 1].to) + part[parts - 1].words * 8 == (uintptr_t)to)
+        double* const end = parts ? part[parts - 1].to + part[parts - 1].words : nullptr;
+        if (end == to && pageable(end - 1) && pageable(to))
             part[parts - 1].words += words;
         else
             part[parts++] = {to, words};
