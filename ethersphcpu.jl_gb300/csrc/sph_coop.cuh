@@ -366,6 +366,33 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const SelectScale
     }
 }
 
+// d^2 <= r_cut^2 in FP64, for the selection of particles far outside the grid.
+template <int DIM, typename V>
+__device__ __forceinline__ bool within_cut(const V& xi, const V& xj, const SceneDev& S) {
+    double rv[DIM];
+    make_rvec<DIM>(xi, xj, S, rv);
+    return norm_sq<DIM>(rv) <= S.rc2;
+}
+
+// Selection into a list of indices with a relative margin of 1e-4 on r_cut^2 (cell-relative
+// differences within the stencil carry an FP32 error of some 1e-6 cells): only candidates
+// beyond r_cut are left out.  A particle far outside its cell (clamped from outside the
+// grid) or with a non-finite position is tested by within(j), in FP64.
+template <int DIM, typename Within, typename Pairs>
+__device__ __forceinline__ void select_64(const SceneDev& S, const int32_t* __restrict__ start,
+                                          const float4* __restrict__ pos, const int32_t c[3], const float4& me,
+                                          int self, bool on, int32_t* list, Within&& within, Pairs&& pairs) {
+    const SelectScale scale{S.sel_e[0], S.sel_e[1], S.sel_e[2], S.sel_inv_ex, 1.0001f, true};
+    const bool far = select_far(me);
+    coop_select<DIM, kCoopList<DIM>>(
+        S, scale, start, pos, c, me, self, on, [&](int j, float d2) { return far ? within(j) : d2 <= 1.0001f; },
+        [&](int slot, int j, float, float, float) { list[slot] = j; },
+        [&](int first, int cnt, bool) {
+            pairs(first, cnt);
+            return 0;
+        });
+}
+
 // The next step's cell key of a particle that moved from x0 to x1: its FP32 cell position
 // decides it where the particle is clear of the cell boundaries (by 1e-4 cells, far above
 // the FP32 error) and of the grid's edge cells, the FP64 hash otherwise; the key is the

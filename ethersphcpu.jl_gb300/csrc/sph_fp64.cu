@@ -61,33 +61,6 @@ __device__ __forceinline__ double dot_fma(const double a[DIM], const double b[DI
     return s;
 }
 
-// d^2 <= r_cut^2 in FP64, for the selection of particles far outside the grid.
-template <int DIM, typename V>
-__device__ __forceinline__ bool within_cut(const V& xi, const V& xj, const SceneDev& S) {
-    double rv[DIM];
-    make_rvec<DIM>(xi, xj, S, rv);
-    return norm_sq<DIM>(rv) <= S.rc2;
-}
-
-// Selection into a list of indices with a relative margin of 1e-4 on r_cut^2 (cell-relative
-// differences within the stencil carry an FP32 error of some 1e-6 cells): only candidates
-// beyond r_cut are left out.  A particle far outside its cell (clamped from outside the
-// grid) or with a non-finite position is tested by within(j), in FP64.
-template <int DIM, typename Within, typename Pairs>
-__device__ __forceinline__ void select_64(const SceneDev& S, const int32_t* __restrict__ start,
-                                          const float4* __restrict__ pos, const int32_t c[3], const float4& me,
-                                          int self, bool on, int32_t* list, Within&& within, Pairs&& pairs) {
-    const SelectScale scale{S.sel_e[0], S.sel_e[1], S.sel_e[2], S.sel_inv_ex, 1.0001f, true};
-    const bool far = select_far(me);
-    coop_select<DIM, kCoopList<DIM>>(
-        S, scale, start, pos, c, me, self, on, [&](int j, float d2) { return far ? within(j) : d2 <= 1.0001f; },
-        [&](int slot, int j, float, float, float) { list[slot] = j; },
-        [&](int first, int cnt, bool) {
-            pairs(first, cnt);
-            return 0;
-        });
-}
-
 template <int DIM, int KK>
 __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
     k_continuity_fp64(const SceneDev* __restrict__ scenes, SortedState st, SortScratch sc, int32_t cap, BufferState bf) {
