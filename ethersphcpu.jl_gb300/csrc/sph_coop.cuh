@@ -71,6 +71,14 @@ __device__ __forceinline__ double sqrt3(double a, double& inv) {
     return fma(s * e, p, s);
 }
 
+// y = 1 / a from a residual correction, right but for a mantissa of all ones: there 1 / a lies
+// just above the middle between a power of two and its successor, which is the value to return,
+// and the correction stays at the power.
+__device__ __forceinline__ double rcp_of_ones(double a, double y) {
+    const bool ones = (__double2loint(a) & (__double2hiint(a) | 0xfff00000)) == -1;
+    return __hiloint2double(__double2hiint(y), ones ? 1 : __double2loint(y));
+}
+
 // sqrt(a) and 1 / sqrt(a), both rounded to nearest as the IEEE operations round them
 // (the second is 1 / (the rounded root)), for a in [2^-900, 2^900]: the values above,
 // corrected by their residuals (Markstein, Computation of elementary functions on the IBM
@@ -83,7 +91,7 @@ __device__ __forceinline__ double sqrt_rn(double a, double& inv) {
     const double y1 = fma(y * e, p, y);
     const double s1 = fma(s * e, p, s);
     const double r = fma(fma(-s1, s1, a), 0.5 * y1, s1);
-    inv = fma(fma(-r, y1, 1.0), y1, y1);
+    inv = rcp_of_ones(r, fma(fma(-r, y1, 1.0), y1, y1));
     return r;
 }
 __device__ __forceinline__ bool sqrt_rn_range(double a) {
@@ -97,7 +105,7 @@ __device__ __forceinline__ bool rcp_rn_range(double a) {
 // 1 / a rounded to nearest, for |a| in [2^-900, 2^900].
 __device__ __forceinline__ double rcp_rn(double a) {
     const double y = rcp3(a);
-    return fma(fma(-a, y, 1.0), y, y);
+    return rcp_of_ones(a, fma(fma(-a, y, 1.0), y, y));
 }
 
 // a / b rounded to nearest, y = 1 / b rounded to nearest (the same residual correction).
