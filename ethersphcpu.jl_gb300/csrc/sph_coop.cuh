@@ -231,31 +231,25 @@ __device__ __forceinline__ float dist2(float rx, float ry, float rz) {
     return __fmaf_rn(rx, rx, __fmaf_rn(ry, ry, __fmul_rn(rz, rz)));
 }
 
-// Lengths of a selection: the cell edges, 1 / ex, and the bound on d^2 beyond which rows and
-// cells are left out (prune).
-struct SelectScale {
-    float ex, ey, ez, inv_ex, r2;
-    bool prune;
-};
-
-// The candidates of one particle in the cell list (start, pos), tested in FP32 and packed
-// into a list in walk order (cells z, y, x): accept(j, d2) says whether candidate j is taken,
-// emit(slot, j, rx, ry, rz) lists it (r = x_i - x_j), CAP slots; the pair work
-// pairs(first, cnt, last) runs at the end (last) and before when a list of the warp is full:
-// the list then holds entries first .. first + cnt - 1 of the whole, and pairs returns how
-// many of them it left at its front.  me: the particle's select_pos, c its cell, self its
-// index in `pos` (-1: none).  Every lane of the warp calls this together; a group without a
-// particle passes on = false.
+// The neighbours of one particle in the cell list (start, pos), selected in FP32 and packed
+// into a list in walk order (cells z, y, x) with a relative margin of 1e-4 on r_cut^2
+// (cell-relative differences within the stencil carry an FP32 error of some 1e-6 cells): only
+// candidates beyond r_cut are left out.  A particle far outside its cell (clamped from
+// outside the grid) or with a non-finite position is tested by within(j), in FP64.  The pair
+// work pairs(first, cnt) runs at the end, and before when a list of the warp is full: the list
+// (kCoopList entries) then holds entries first .. first + cnt - 1 of the whole.  me: the
+// particle's select_pos, c its cell, self its index in `pos` (-1: none).  Every lane of the
+// warp calls this together; a group without a particle passes on = false.
 //
-// Pruning keeps a margin on r_cut^2 far above the FP32 rounding of positions within a few
-// cells.  Rows on the y/z grid boundary and the first and last x cells may hold particles
-// clamped from outside the grid and stay whole, as does the stencil of a particle itself far
-// outside its cell.
-template <int DIM, int CAP, typename Accept, typename Emit, typename Pairs>
-__device__ __forceinline__ void coop_select(const SceneDev& S, const SelectScale& sc,
-                                            const int32_t* __restrict__ start, const float4* __restrict__ pos,
-                                            const int32_t c[3], const float4 me, int self, bool on, Accept&& accept,
-                                            Emit&& emit, Pairs&& pairs) {
+// Rows and cells beyond r_cut are left out with the same margin.  Rows on the y/z grid
+// boundary and the first and last x cells may hold particles clamped from outside the grid
+// and stay whole, as does the stencil of a particle itself far outside its cell.
+template <int DIM, typename Within, typename Pairs>
+__device__ __forceinline__ void coop_select(const SceneDev& S, const int32_t* __restrict__ start,
+                                            const float4* __restrict__ pos, const int32_t c[3], const float4& me,
+                                            int self, bool on, int32_t* list, Within&& within, Pairs&& pairs) {
+    const float ex = S.sel_e[0], ey = S.sel_e[1], ez = S.sel_e[2], inv_ex = S.sel_inv_ex;  // cell edges / r_cut
+    constexpr float kR2 = 1.0001f;
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & (kCoopLanes - 1);
     const int shift = (threadIdx.x & 31) & ~(kCoopLanes - 1);
@@ -263,7 +257,7 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const SelectScale
     const int m = S.reach;
     const int zr = DIM == 3 ? m : 0;
     const float nx = (float)S.n[0];
-    const bool prune = sc.prune && !select_far(me);
+    const bool far = select_far(me);
     const int planes = DIM == 3 ? (int)__reduce_max_sync(full, (unsigned)zr) : 0;
     int first_entry = 0, cnt = 0;
     for (int dz = -planes; dz <= planes; ++dz) {
@@ -277,16 +271,16 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const SelectScale
             int x0 = c[0] - m, x1 = c[0] + m;
             bool keep = true;
             const bool edge = y == 0 || y == S.n[1] - 1 || (DIM == 3 && (z == 0 || z == S.n[2] - 1));
-            if (!edge && prune) {
-                const float gy = fmaxf(fmaxf((float)dy - me.y, me.y - (float)(dy + 1)), 0.f) * sc.ey;
-                float rem = sc.r2 - gy * gy;
+            if (!edge && !far) {
+                const float gy = fmaxf(fmaxf((float)dy - me.y, me.y - (float)(dy + 1)), 0.f) * ey;
+                float rem = kR2 - gy * gy;
                 if (DIM == 3) {
-                    const float gz = fmaxf(fmaxf((float)dz - me.z, me.z - (float)(dz + 1)), 0.f) * sc.ez;
+                    const float gz = fmaxf(fmaxf((float)dz - me.z, me.z - (float)(dz + 1)), 0.f) * ez;
                     rem -= gz * gz;
                 }
                 keep = !(rem < 0.f);
                 if (keep && !S.periodic_x) {
-                    const float w = sqrtf(rem) * sc.inv_ex;
+                    const float w = sqrtf(rem) * inv_ex;
                     const int a = c[0] + (int)floorf(me.x - w), e = c[0] + (int)floorf(me.x + w);
                     if (x0 > 0 && a > x0) x0 = min(a, S.n[0] - 1);
                     if (x1 < S.n[0] - 1 && e < x1) x1 = max(e, 0);
@@ -353,22 +347,22 @@ __device__ __forceinline__ void coop_select(const SceneDev& S, const SelectScale
             for (int h = 0; h < 2; ++h) {
                 float cx = me.w - p[h].w;
                 if (S.periodic_x) cx = cx > 0.5f * nx ? cx - nx : (cx < -0.5f * nx ? cx + nx : cx);
-                const float rx = (cx + (me.x - p[h].x)) * sc.ex;
-                const float ry = ((me.y - p[h].y) - dyf[h]) * sc.ey;
-                const float rz = DIM == 3 ? ((me.z - p[h].z) - (float)dz) * sc.ez : 0.f;
+                const float rx = (cx + (me.x - p[h].x)) * ex;
+                const float ry = ((me.y - p[h].y) - dyf[h]) * ey;
+                const float rz = DIM == 3 ? ((me.z - p[h].z) - (float)dz) * ez : 0.f;
                 bool take = j[h] >= 0 && j[h] != self;
-                if (take) take = accept(j[h], dist2(rx, ry, rz));
+                if (take) take = far ? within(j[h]) : dist2(rx, ry, rz) <= kR2;
                 const unsigned hit = (__ballot_sync(full, take) >> shift) & 0xffu;
-                if (take) emit(cnt + __popc(hit & below), j[h], rx, ry, rz);
+                if (take) list[cnt + __popc(hit & below)] = j[h];
                 cnt += __popc(hit);
             }
             const bool last = dz == planes && t0 + 2 * kCoopLanes >= rounds;
-            if (last || __any_sync(full, cnt > CAP - 2 * kCoopLanes)) {
+            if (last || __any_sync(full, cnt > kCoopList<DIM> - 2 * kCoopLanes)) {
                 __syncwarp(full);
-                const int kept = pairs(first_entry, cnt, last);
+                pairs(first_entry, cnt);
                 __syncwarp(full);
-                first_entry += cnt - kept;
-                cnt = kept;
+                first_entry += cnt;
+                cnt = 0;
             }
         }
     }
@@ -380,25 +374,6 @@ __device__ __forceinline__ bool within_cut(const V& xi, const V& xj, const Scene
     double rv[DIM];
     make_rvec<DIM>(xi, xj, S, rv);
     return norm_sq<DIM>(rv) <= S.rc2;
-}
-
-// Selection into a list of indices with a relative margin of 1e-4 on r_cut^2 (cell-relative
-// differences within the stencil carry an FP32 error of some 1e-6 cells): only candidates
-// beyond r_cut are left out.  A particle far outside its cell (clamped from outside the
-// grid) or with a non-finite position is tested by within(j), in FP64.
-template <int DIM, typename Within, typename Pairs>
-__device__ __forceinline__ void select_64(const SceneDev& S, const int32_t* __restrict__ start,
-                                          const float4* __restrict__ pos, const int32_t c[3], const float4& me,
-                                          int self, bool on, int32_t* list, Within&& within, Pairs&& pairs) {
-    const SelectScale scale{S.sel_e[0], S.sel_e[1], S.sel_e[2], S.sel_inv_ex, 1.0001f, true};
-    const bool far = select_far(me);
-    coop_select<DIM, kCoopList<DIM>>(
-        S, scale, start, pos, c, me, self, on, [&](int j, float d2) { return far ? within(j) : d2 <= 1.0001f; },
-        [&](int slot, int j, float, float, float) { list[slot] = j; },
-        [&](int first, int cnt, bool) {
-            pairs(first, cnt);
-            return 0;
-        });
 }
 
 // The next step's cell key of a particle that moved from x0 to x1: its FP32 cell position

@@ -5,7 +5,7 @@
 // (CellListMap.update!/neighborlist! + findNeighbours!, FluidWallSolve.jl:21-35,
 // Neighbour.jl:88-128) so that it can be compared particle by particle with a CPU
 // restatement: the key is the one the step's sort uses, and the neighbours are found by the
-// functions with which the gathers of the handle's form find them (FP64: select_64 and
+// functions with which the gathers of the handle's form find them (FP64: coop_select and
 // inside_cut, as k_momentum_fp64; FP32-compensated: row_runs and run_walk, as
 // k_continuity_f32 records its list).
 #include "sph_fp32.cuh"
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kCoopThreads)
     int32_t* list = lists + group * kCoopList<DIM>;
     int32_t* out = ids ? ids + rows[i - b] : nullptr;
     int32_t n = 0;
-    select_64<DIM>(
+    coop_select<DIM>(
         S, start, st.fa, c, st.fa[i], i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
         [&](int, int cnt) {
             const int most = (int)__reduce_max_sync(0xffffffffu, (unsigned)cnt);

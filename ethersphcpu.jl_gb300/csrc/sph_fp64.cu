@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
         int32_t c[3];
         decode_cell(st.cell[i], S, c);
         double drho = 0.0;
-        select_64<DIM>(
+        coop_select<DIM>(
             S, sc.start, st.fa, c, st.fa[i], i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
             [&](int first, int cnt) {
                 int k = (lane - first) & (kCoopLanes - 1);
@@ -232,7 +232,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
         // PressureForce.jl:14-19, ViscosityForce.jl:15-23, ThermalConduction.jl:15-21.  With
         // mu = nu0 rho the viscosity factor is 4 nu0 m_j r dW / ((rho_i + rho_j) (r^2 + 0.01 h^2));
         // heat is taken as aT = sum m_j/rho_j kappa_j r dW / ((kappa_i + kappa_j) (r^2 + 0.01 h^2)) T_ij
-        select_64<DIM>(
+        coop_select<DIM>(
             S, sc.start, st.fa, c, me, i, on, list, [&](int j) { return within_cut<DIM>(xi, x[j], S); },
             [&](int first, int cnt) {
                 if (!ready) {
@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
             const double Pw = P_i + S.P_bg;
             const double Wg_i = uniform ? S.wg : kernel_w<KK>(gap_i, S);
             const double nu_rho = 2.0 * S.nu0 / rho_i;  // 8 mu_i / (2 rho_i)^2
-            select_64<DIM>(
+            coop_select<DIM>(
                 S, wl.start, wl.fa, c, me, -1, walls, list, [&](int j) { return within_cut<DIM>(xi, wx[j], S); },
                 [&](int first, int cnt) {
                     rounds(first, cnt, [&](int k, int e0, int e1) {
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(kCoopThreads, kCoopBlocks)
             T_i = st.T[i];
             const double fluid = sums[threadIdx.x & 31], wall = sums[32 + (threadIdx.x & 31)];
             const double cp_i = st.cp[i];
-        dT = (4.0 * st.kappa[i] * fluid + S.inv_cp_d * S.inv_rho0 * m_i * cp_i * wall) / (cp_i * rho_i);
+            dT = (4.0 * st.kappa[i] * fluid + S.inv_cp_d * S.inv_rho0 * m_i * cp_i * wall) / (cp_i * rho_i);
         }
 
         // ---- updateTemperature!, updateVelocity!, updatePosition!
