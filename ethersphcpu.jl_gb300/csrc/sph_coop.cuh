@@ -117,6 +117,16 @@ __device__ __forceinline__ double div_rn(double a, double b, double y) {
 // max(a, 0) on the sign bit (integer work)
 __device__ __forceinline__ double relu(double a) { return __double2hiint(a) < 0 ? 0.0 : a; }
 
+// (double)x by integer work: the conversion takes the FP64 unit as long as an addition.  A
+// subnormal is scaled into the normal numbers (exactly) and its exponent set right after.
+__device__ __forceinline__ double widen(float x) {
+    const int32_t e = __float_as_int(x) & 0x7f800000;
+    const int32_t b = __float_as_int(e ? x : __fmul_rn(x, 16777216.f));
+    const int32_t bias = e == 0x7f800000 ? 0x70000000 : (e ? 0x38000000 : 0x38000000 - (24 << 20));
+    const int32_t top = (b & 0x7fffffff) ? ((b & 0x7fffffff) >> 3) + bias : 0;
+    return __hiloint2double((b & (int32_t)0x80000000) | top, b << 29);
+}
+
 // x^4 .. x^7 as jl_powi rounds them (finite x).
 template <int N>
 __device__ __forceinline__ double powi_fixed(double x) {

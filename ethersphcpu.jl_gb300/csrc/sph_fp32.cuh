@@ -524,11 +524,10 @@ __device__ __forceinline__ float pair_terms(const SceneDev& S, const SortedState
 }
 
 // A neighbour's terms of the Shepard sums (ReconstructValue.jl:28-50), FP64; w = W / kw_a.
-__device__ __forceinline__ void shepard_terms(const SceneDev& S, const SortedState& st, float w, int j, double& sw,
-                                              double& sws) {
-    const double W = (double)__fmul_rn(S.kw_a_f, w);
-    sw = fma(W, st.vol[j], sw);
-    sws = fma(W, st.m[j], sws);
+__device__ __forceinline__ void shepard_terms(const SceneDev& S, float w, double vol, double m, double& sw, double& sws) {
+    const double W = widen(__fmul_rn(S.kw_a_f, w));
+    sw = fma(W, vol, sw);
+    sws = fma(W, m, sws);
 }
 
 // Terms of a wall pair: the compulsive force (WallForce.jl:15-28), background pressure
@@ -767,7 +766,7 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
         SumsF<DIM, HEAT> fluid, wall;
         double sw = 0.0, sws = 0.0;
         coop_rows<DIM, KK, MODE>(S, st, wl, sc.start, i, self_f<DIM, KK, HEAT>(S, st, i), walk, walls, fluid, wall,
-                                 [&](float wk, int j) { if constexpr (SHEP) shepard_terms(S, st, wk, j, sw, sws); });
+                                 [&](float wk, int j) { if constexpr (SHEP) shepard_terms(S, wk, st.vol[j], st.m[j], sw, sws); });
         if constexpr (SHEP) {
             sw = coop_sum(sw);
             sws = coop_sum(sws);
@@ -799,9 +798,11 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
 // end before the walks).  Both together against one after the other: 17.0 against 24.1 us on
 // a 65,536-particle cavity (54 -> 47 us a step), 216 against 228 on a million particles,
 // 315 against 330 on a 432,000-particle 3D dam break (before the eight sums: 25.7, 254, 488).
-// The Shepard sums are one FP64 sum each, in the list's order: 320 us with them at a million
-// particles, 457 on the 3D dam break (eight sums each, in a second pass over the list: 385 and
-// 633; before: 330 and 533).
+// The Shepard sums are one FP64 sum each, in the list's order: 285 us with them at a million
+// particles, 409 on the 3D dam break (eight sums each, in a second pass over the list: 385 and
+// 633; before: 330 and 533).  A neighbour's volume and mass are loaded with its other values
+// (415 us in 3D against 457), and its kernel value is widened without the FP64 unit, which the
+// sums keep busy (285 against 315 us).
 template <int DIM, int KK, int MODE, bool SHEP>
 __global__ void __launch_bounds__(128, 4)
     k_momentum_f32(const SceneDev* __restrict__ scenes, SortedState st, NextState nx, WallState wl, SortScratch sc,
@@ -843,11 +844,16 @@ __global__ void __launch_bounds__(128, 4)
             for (int u = 0; u < kCoopLanes; ++u) {
                 const int j = i + (code[u] >> 9);
                 const float4 r = listed<DIM>(code[u], a.x, __ldg(st.fa + j), j, S);
+                double vol = 0.0, m = 0.0;
+                if constexpr (SHEP) {
+                    vol = __ldg(st.vol + j);
+                    m = __ldg(st.m + j);
+                }
                 float t[DIM + 1];
                 const float w = pair_terms<DIM, KK, HEAT>(S, st, a, r, __ldg(st.fb + j), __ldg(st.fc + j), t);
                 if (k + u < count) {
                     acc[u].add(t);
-                    if constexpr (SHEP) shepard_terms(S, st, w, j, sw, sws);
+                    if constexpr (SHEP) shepard_terms(S, w, vol, m, sw, sws);
                 }
             }
         }
@@ -908,7 +914,7 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
         SumsF<DIM, HEAT> sum;
         double sw = 0.0, sws = 0.0;  // Shepard sums of a walked particle, by lane
         const int count = on ? (nl.e ? nl.n[i] : kListWalk) : 0;
-        auto shepard = [&](float w, int j) { if constexpr (SHEP) shepard_terms(S, st, w, j, sw, sws); };
+        auto shepard = [&](float w, int j) { if constexpr (SHEP) shepard_terms(S, w, st.vol[j], st.m[j], sw, sws); };
         if (count != kListWalk && lane < count) {
             // the entry two rounds ahead and the neighbour one round ahead are loaded before the
             // current pair is processed
@@ -956,7 +962,7 @@ __global__ void __launch_bounds__(256, DIM == 3 ? 3 : 4)
                 const int32_t code = k < entries ? __ldg(nl.e + i + k * nl.stride) : 0;
                 const int j = i + (code >> 9);
                 const PairF<DIM, KK> p(listed<DIM>(code, a.x, __ldg(st.fa + j), j, S), S);
-                const double W = (double)__fmul_rn(S.kw_a_f, p.w), vol = st.vol[j], m = st.m[j];
+                const double W = widen(__fmul_rn(S.kw_a_f, p.w)), vol = st.vol[j], m = st.m[j];
 #pragma unroll
                 for (int e = 0; e < kCoopLanes; ++e) {
                     const double We = __shfl_sync(full, W, e, kCoopLanes), ve = __shfl_sync(full, vol, e, kCoopLanes),

@@ -61,6 +61,10 @@ __global__ void k_pairs(int n, const double* a, SceneDev S, double* out) {
         out[(6 + k) * n + i] = want[k];
     }
 }
+__global__ void k_widen(int n, const float* a, double* out) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = widen(a[i]);
+}
 static int run(int n, const double* a, const double* b, void* out, size_t bytes, int which) {
     double *da = nullptr, *db = nullptr;
     void* dout = nullptr;
@@ -75,7 +79,10 @@ static int run(int n, const double* a, const double* b, void* out, size_t bytes,
     if (which == 1) k_powers<<<grid, 256>>>(n, da, (double*)dout);
     if (which == 2) k_ranges<<<grid, 256>>>(n, da, (int*)dout);
     cudaMemcpy(out, dout, bytes, cudaMemcpyDeviceToHost);
-    if (which >= 3) {
+    if (which == 7) {  // a holds 2 n floats
+        k_widen<<<(2 * n + 255) / 256, 256>>>(2 * n, (const float*)da, (double*)dout);
+        cudaMemcpy(out, dout, bytes, cudaMemcpyDeviceToHost);
+    } else if (which >= 3) {
         SceneDev S{};
         S.h = 0.037;
         S.inv_h = 1.0 / S.h;
@@ -99,6 +106,9 @@ extern "C" int ranges(int n, const double* a, int* out) { return run(n, a, nullp
 
 extern "C" int pairs(int n, const double* a, double* out, int kernel) {
     return run(3 * n, a, nullptr, out, 96ull * n, 3 + kernel);
+}
+extern "C" int widened(int n, const float* a, double* out) {  // n even
+    return run(n / 2, (const double*)a, nullptr, out, 8ull * n, 7);
 }
 """
 
@@ -196,6 +206,20 @@ def test_pairs(unit, kernel):
     assert unit.pairs(len(v), ptr(v), ptr(out), kernel) == 0
     for k in range(6):
         same(out[0, k] + 0.0, out[1, k] + 0.0, v[:, 0], v[:, 1], v[:, 2])  # a zero of either sign
+
+
+def test_widened_floats(unit):
+    # every exponent with mantissas at both ends and in the middle, both signs, subnormals,
+    # zeros, infinities, and random bits
+    mantissa = np.concatenate([np.arange(256), 2**23 - 1 - np.arange(256), 2**22 - 128 + np.arange(256)])
+    bits = (np.arange(512, dtype=np.int64)[:, None] << 23 | mantissa).ravel().astype(np.uint32)
+    bits = np.concatenate([bits, np.random.default_rng(6).integers(0, 2**32, N, dtype=np.uint32)])
+    x = bits.view(np.float32)
+    out = np.empty(len(x))
+    assert len(x) % 2 == 0 and unit.widened(len(x), ptr(x), ptr(out)) == 0
+    nan = np.isnan(x)
+    assert np.all(np.isnan(out[nan]))
+    same(out[~nan], x[~nan].astype(np.float64), x[~nan].astype(np.float64))
 
 
 def test_ranges_take_only_what_the_helpers_are_exact_on(unit):
