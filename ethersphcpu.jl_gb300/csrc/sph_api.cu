@@ -367,9 +367,7 @@ struct SphHandle {
     int lanes[2] = {-1, -1};
     NbrList nl{};          // neighbour list of the FP32 form (ensure_list)
     bool list_short = false;  // no room for it, or not at its full depth (until the particles or scenes change)
-    // stencil pruning of the FP32 gathers (sph_set_stencil_pruning), on by default: the rows
-    // of a particle's stencil are bounded by its eight lanes together
-    int prune = 1;
+    int prune = 1;  // stencil pruning of the FP32 gathers (sph_set_stencil_pruning)
     std::string err;
     std::vector<SceneRec> scenes;
     RangeAlloc cells, walls;

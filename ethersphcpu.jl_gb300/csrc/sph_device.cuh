@@ -25,13 +25,17 @@ constexpr int32_t kDeadKey = 0x7fffffff;
 // Programmatic dependent launch between the kernels of a step (launch_dep): the next
 // kernel's launch is prepared while its predecessor in the stream finishes; pdl_wait()
 // blocks until the predecessor grid has completed and its writes are visible (a no-op
-// when the kernel was launched without the attribute).  A step kernel calls it first, before
-// it touches device memory.  A kernel whose successor has nothing to do before its wait does
-// not trigger it early: blocks of the next kernel parked on the wait took SM slots from the tail of the current one (a
-// 65k-particle step on GB300: 0.0652 ms with an early trigger, 0.0642 ms without
-// programmatic launches, 0.0622 ms with the trigger at block exit, as here).
-// A predecessor may let its successor start early where that has work of its own to do before
-// it waits (pdl_trigger, after its own pdl_wait: what came before it is then visible to both).
+// when the kernel was launched without the attribute).  A step kernel whose predecessor does
+// not trigger it calls it first, before it touches device memory; no predecessor does so
+// where the successor would only wait: blocks of the next kernel parked on the wait took SM
+// slots from the tail of the current one (a 65k-particle step on GB300: 0.0652 ms with an
+// early trigger, 0.0642 ms without programmatic launches, 0.0622 ms with the trigger at block
+// exit).  Where the successor has work of its own, the predecessor triggers it after its own
+// wait (pdl_trigger: what came before the predecessor is then visible to both).  Such a
+// successor reads nothing that its predecessor writes, and writes nothing that it reads,
+// before its wait, and every one of its threads waits before it ends: k_fill (started by the
+// scan), k_place (by k_fill), k_momentum_fp64 (by continuity; it draws from a queue word of
+// its own), k_momentum_lanes_f32 (by continuity) and k_momentum_f32 (by k_walks_f32).
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
