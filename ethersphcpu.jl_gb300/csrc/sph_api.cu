@@ -1116,10 +1116,11 @@ int32_t allocate_state(SphHandle* h, int64_t cells) {
                 {&h->sc.tmp, (size_t)h->cap},        {&h->sc.count, ncell},
                 {&h->sc.start, ncell + 1},           {&h->sc.block_sums, ncell / 1024 + 2},
                 {&h->sc.status, 1},                  {&h->nbuf, 2},
-                {&h->sc.queue, kQueueWords},                   {&h->sc.n_walked, 1},
-                {&h->W.start, ncell + 1},            {&h->W.kind, wc}};
+                {&h->sc.queue, kQueueWords + 1},     {&h->W.start, ncell + 1},
+                {&h->W.kind, wc}};
     for (auto& a : ints)
         if ((e = dalloc(h, a.p, a.n)) != cudaSuccess) return cuda_fail(nullptr, e, "scratch");
+    h->sc.n_walked = h->sc.queue ? h->sc.queue + kQueueWords : nullptr;
     if (h->precision == SPH_PRECISION_FP32_COMPENSATED) {
         const size_t sums = 2 * (size_t)(h->dim + (h->mode == 2 ? 1 : 0)) + 2;
         if ((e = dalloc(h, &h->sc.walked, (size_t)h->cap)) != cudaSuccess) return cuda_fail(nullptr, e, "scratch");
@@ -1787,8 +1788,11 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
     Lr.shepard = 1;
     Lr.force_reinit = 1;
     const int par = h->par;
-    auto clear_queue = [&] {  // what the placement does between the gathers of two steps
-        if (h->precision == SPH_PRECISION_FP64) cudaMemsetAsync(h->sc.queue, 0, 4 * kQueueWords, st);
+    // what the placement does between the gathers of two steps: the draws of the FP64 form, and
+    // before continuity the number of walked particles, which it appends to
+    auto clear_counters = [&](bool walked) {
+        if (walked || h->precision == SPH_PRECISION_FP64)
+            cudaMemsetAsync(h->sc.queue, 0, 4 * (kQueueWords + (walked ? 1 : 0)), st);
     };
     auto run = [&](int stage) {
         switch (stage) {
@@ -1799,16 +1803,15 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
             case SPH_STAGE_SCAN: launch_scan(Lh, 0); break;
             case SPH_STAGE_SORT: launch_place(Lh); break;
             case SPH_STAGE_CONTINUITY:
-                cudaMemsetAsync(h->sc.n_walked, 0, 4, st);  // continuity appends to the walked particles
-                clear_queue();
+                clear_counters(true);
                 launch_physics(0, L);
                 break;
             case SPH_STAGE_MOMENTUM:
-                clear_queue();
+                clear_counters(false);
                 launch_physics(1, L);
                 break;
             case SPH_STAGE_REINIT:
-                clear_queue();
+                clear_counters(false);
                 launch_physics(1, Lr);
                 break;
         }
@@ -1828,8 +1831,7 @@ int32_t sph_time_stages(SphHandle* h, int32_t reps, double* ms_out) {
         }
     }
     // the momentum stage left arrivals in count[]: the next step expects it zeroed
-    clear_queue();
-    SPH_CUDA(h, cudaMemsetAsync(h->sc.n_walked, 0, 4, st));
+    clear_counters(true);
     SPH_CUDA(h, cudaMemsetAsync(h->sc.count, 0, sizeof(int32_t) * (size_t)h->scan_cells, st));
     // restore p and c (output-only fields) from the copy the placement stage wrote
     const size_t n = (size_t)h->cap;

@@ -197,7 +197,8 @@ struct SortScratch {
     // zeroes them, and every gather of the next step starts after one that waited for it.
     int32_t* queue;
     // FP32 form, large scenes: the particles whose cells the momentum gather walks, their
-    // number (0 before continuity) and their sums of those walks (fluid, walls, Shepard)
+    // number (0 before continuity; the word behind queue[]) and their sums of those walks
+    // (fluid, walls, Shepard)
     int32_t* walked;
     int32_t* n_walked;
     float2* walk_sums;
