@@ -253,8 +253,7 @@ __global__ void k_place(const SceneDev* __restrict__ scenes, SortedState src, Ne
     using V = typename VecT<DIM>::T;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     // count[] and the tile sums have been scanned: clear them for the next step's arrivals
-    if (i == 0) *sc.n_walked = 0;
-    if (i < kQueueWords) sc.queue[i] = 0;
+    if (i <= kQueueWords) sc.queue[i] = 0;  // and *n_walked, which lies behind
     for (int k = i; k < ncells; k += gridDim.x * blockDim.x) sc.count[k] = 0;
     for (int k = i; k < ncells / kScanTileCells + 1; k += gridDim.x * blockDim.x) sc.block_sums[k] = 0;
     const int32_t key = i < cap && i < *sc.n_live ? sc.key[i] : kDeadKey;
