@@ -21,7 +21,7 @@
 // on the variant, the batch or the pruning.
 //
 // What bounds them: on small scenes the chain of loads and rounds of one particle, on large
-// ones the issue of instructions (continuity issues in 66 to 76 of 100 cycles, momentum in 43
+// ones the issue of instructions (continuity issues in 71 to 80 of 100 cycles, momentum in 43
 // to 57 with 15 warps an SM for its eight sums, waiting on neighbours from L2); the bytes would
 // take a sixth of the time.
 //
